@@ -163,17 +163,18 @@ struct GeomBuf {
 struct Gmres {
     int dim = 0;
     double *U = nullptr;      // [5][C] Newton iterate (conserved)
-    double *Ustart = nullptr; // [5][C] conserved state at the start of the step
     double *r = nullptr;      // [5][C] Newton residual
-    double *delta = nullptr;  // [5][C] increment
     double *V = nullptr;      // [dim + 1][5][C] Krylov basis
     double *w = nullptr;      // [5][C]
     double *q1 = nullptr;     // [5][N] perturbed primitive state
     double *R1 = nullptr;     // [5][C] derivative of the perturbed state
-    double *part = nullptr;   // per-piece partial sums
+    int nchunks = 0;          // cell chunks of the Krylov vectors
+    int *chunk_beg = nullptr;       // [nchunks + 1]
+    int *inst_chunk_off = nullptr;  // [ninst + 1]
+    double *part = nullptr;   // [2 dim + 1][nchunks] partial sums
+    int *ticket = nullptr;    // [ninst] chunks that have finished the current pass
     double *sc = nullptr;     // per-instance device scalars (GmresScalar)
     int *flag = nullptr;      // per-instance progress (GmresFlag)
-    int *count = nullptr;     // [2] instances still iterating (Newton, Arnoldi)
     int *ctl = nullptr;       // [GC_COUNT] loop counters of the graph-driven loops
     double *Rm = nullptr;     // [5][C] FP32-flux form: the matvec's base residual, in FP32 fluxes
 };
@@ -309,7 +310,7 @@ struct tg_ctx {
     long igraph_kernels = 0;
     double ig_courant = 0, ig_newton_tol = 0, ig_krylov_tol = 0;
     int ig_dim = 0, ig_use_max_time = -1;
-    cudaStream_t cap_stream[3] = {nullptr, nullptr, nullptr};  // body captures of nested loops
+    cudaStream_t cap_stream[2] = {nullptr, nullptr};  // body captures of nested loops
 };
 
 static double &hd_at(tg_ctx *c, int field, int i) { return c->hd[(size_t)field * c->ninst + i]; }
@@ -345,6 +346,16 @@ static const double LSERK_ALPHA[3][6][7] = {
     },
 };
 
+static void free_gmres(Gmres &g)
+{
+    void *p[] = {g.U,    g.r,      g.V,  g.w,    g.q1,  g.R1, g.chunk_beg, g.inst_chunk_off,
+                 g.part, g.ticket, g.sc, g.flag, g.ctl, g.Rm};
+    for (void *x : p) {
+        if (x) cudaFree(x);
+    }
+    g = Gmres{};
+}
+
 static void free_ctx(tg_ctx *c)
 {
     if (!c) return;
@@ -369,11 +380,7 @@ static void free_ctx(tg_ctx *c)
     for (void *p : ptrs) {
         if (p) cudaFree(p);
     }
-    void *gp[] = {c->gm.U, c->gm.Ustart, c->gm.r, c->gm.delta, c->gm.V, c->gm.w, c->gm.q1, c->gm.R1,
-                  c->gm.part, c->gm.sc, c->gm.flag, c->gm.count, c->gm.ctl, c->gm.Rm};
-    for (void *p : gp) {
-        if (p) cudaFree(p);
-    }
+    free_gmres(c->gm);
     if (c->hd) cudaFreeHost(c->hd);
     if (c->hi) cudaFreeHost(c->hi);
     if (c->pinned) cudaFreeHost(c->pinned);
@@ -2271,59 +2278,52 @@ extern "C" int tg_batch_run(tg_ctx *c, int method, const void *context, double c
 //
 // Every instance of the arena takes its own implicit step at once: its own CFL step, Newton and
 // Arnoldi iterations that stop on their own tests, masked out of the vector updates once done.
-// The host loops over Newton and Arnoldi iterations and reads, once per iteration, how many
-// instances go on.
+// The Newton and Arnoldi loops run on the device (conditional nodes of the step's graph).
 
 static int gm_alloc(tg_ctx *c, int dim)
 {
     Gmres &g = c->gm;
     if (g.V && g.dim >= dim) return TG_OK;
-    void *old[] = {g.U, g.Ustart, g.r, g.delta, g.V, g.w, g.q1, g.R1, g.part, g.sc, g.flag, g.count, g.ctl, g.Rm};
-    for (void *p : old) {
-        if (p) cudaFree(p);
-    }
-    g = Gmres{};
+    free_gmres(g);
+    drop_graph(c);  // a captured implicit step refers to the old workspace
     size_t n = 5 * (size_t)c->s.C;
     TRY(dalloc(&g.U, n));
-    TRY(dalloc(&g.Ustart, n));
     TRY(dalloc(&g.r, n));
-    TRY(dalloc(&g.delta, n));
-    TRY(dalloc(&g.V, (size_t)(dim + 1) * n));
+    TRY(dalloc(&g.V, (size_t)dim * n));
     TRY(dalloc(&g.w, n));
     TRY(dalloc(&g.q1, 5 * (size_t)c->s.N));
     CU(cudaMemset(g.q1, 0, 5 * sizeof(double) * c->s.N));
     TRY(dalloc(&g.R1, n));
-    TRY(dalloc(&g.part, (size_t)c->npieces));
+    std::vector<int> beg, off(1, 0);
+    for (int i = 0; i < c->ninst; i++) {
+        const int lo = c->h_inst_cell_off[i], hi = c->h_inst_cell_off[i + 1];
+        const int per = krylov_chunk(hi - lo);
+        for (int x = lo; x < hi; x += per) beg.push_back(x);
+        off.push_back((int)beg.size());
+    }
+    g.nchunks = (int)beg.size();
+    beg.push_back(c->s.C);
+    TRY(dalloc(&g.chunk_beg, beg.size()));
+    TRY(dalloc(&g.inst_chunk_off, off.size()));
+    CU(cudaMemcpy(g.chunk_beg, beg.data(), sizeof(int) * beg.size(), cudaMemcpyHostToDevice));
+    CU(cudaMemcpy(g.inst_chunk_off, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice));
+    TRY(dalloc(&g.part, (size_t)(2 * dim + 1) * g.nchunks));
+    TRY(dalloc(&g.ticket, (size_t)c->ninst));
     TRY(dalloc(&g.sc, (size_t)c->ninst * gmres_scn(dim)));
     TRY(dalloc(&g.flag, (size_t)GF_COUNT * c->ninst));
     CU(cudaMemset(g.flag, 0, sizeof(int) * GF_COUNT * c->ninst));
-    TRY(dalloc(&g.count, 2));
     TRY(dalloc(&g.ctl, GC_COUNT));
     CU(cudaMemset(g.ctl, 0, sizeof(int) * GC_COUNT));
     if (c->precision == TG_PRECISION_FP32_FLUX) TRY(dalloc(&g.Rm, n));
     g.dim = dim;
-    drop_graph(c);  // a captured implicit step refers to the old workspace
     return TG_OK;
 }
 
 static GmresBatch gm_batch(tg_ctx *c, int dim)
 {
-    return GmresBatch{dim, gmres_scn(dim), c->ninst, c->cell_inst, c->gm.sc, c->gm.flag, c->gm.count, c->gm.ctl};
-}
-
-// sc[instance][slot] = x . y (or its square root) for the instances whose flag `which` is set
-static int gm_dot(tg_ctx *c, const GmresBatch &gb, const double *x, const double *y, int which, int slot,
-                  int take_sqrt)
-{
-    k_piece_dot<<<c->npieces, BLOCK, 0, c->stream>>>(c->seg, c->s.C, x, y, gb, which, c->gm.part);
-    k_inst_dot<<<c->ninst, GM_INST_BLOCK, 0, c->stream>>>(c->seg, c->gm.part, gb, which, slot, take_sqrt);
-    CU(cudaGetLastError());
-    return TG_OK;
-}
-
-static int inst_grid(const tg_ctx *c)
-{
-    return (c->ninst + 127) / 128;
+    const Gmres &g = c->gm;
+    return GmresBatch{dim,    gmres_scn(dim), c->ninst, g.nchunks, c->cell_inst, g.chunk_beg, g.inst_chunk_off,
+                      g.part, g.ticket,       g.sc,     g.flag,    g.ctl};
 }
 
 // ---- device-driven loops of a captured graph ---------------------------------------------------
@@ -2349,7 +2349,7 @@ static int while_begin(tg_ctx *c, WhileLoop &w, int depth, Init init)
     CU(cudaStreamGetCaptureInfo(c->stream, &status, nullptr, &graph, &deps, &ndeps));
     if (status != cudaStreamCaptureStatusActive) return fail(TG_ERR_INVALID, "device loops need a stream capture");
     CU(cudaGraphConditionalHandleCreate(&w.h, graph, 0, 0));
-    init(w.h);
+    TRY(init(w.h));
     CU(cudaGetLastError());
     CU(cudaStreamGetCaptureInfo(c->stream, &status, nullptr, &graph, &deps, &ndeps));
     cudaGraphNodeParams params = {};
@@ -2403,60 +2403,26 @@ static int newton_precision(const tg_ctx *c)
 }
 
 // one GMRES cycle for the increment of every Newton instance (gmres.c:52-149): the Arnoldi
-// iterations and each column's Gram-Schmidt rows are device loops (a finished instance is masked
-// out of every vector update); each Gram-Schmidt dot is fused with the update of the row before it
-static int gm_solve(tg_ctx *c, const GmresBatch &gb, double krylov_tol)
+// iterations are a device loop (a finished instance is masked out of every vector pass)
+static int gm_solve(tg_ctx *c, const GmresBatch &gb)
 {
     Gmres &g = c->gm;
-    const int C = c->s.C, cb = grid_of(C), ib = inst_grid(c);
-    k_gmres_begin<<<ib, 128, 0, c->stream>>>(gb, krylov_tol);
-    k_gmres_start<<<cb, BLOCK, 0, c->stream>>>(C, g.r, gb, g.V, g.delta);
-    CU(cudaGetLastError());
-    c->launches += 2;
+    const int C = c->s.C, cb = grid_of(C);
     WhileLoop arnoldi;
-    TRY(while_begin(c, arnoldi, 1, [&](cudaGraphConditionalHandle h) {
-        k_arnoldi_enter<<<1, 256, 0, c->stream>>>(gb, h);
+    TRY(while_begin(c, arnoldi, 1, [&](cudaGraphConditionalHandle h) -> int {
+        k_arnoldi_enter<<<1, 1, 0, c->stream>>>(gb, h);
         c->launches += 1;
+        return TG_OK;
     }));
-    {
-        // matvec (gmres.c:12-50)
-        k_piece_vnorm<<<c->npieces, BLOCK, 0, c->stream>>>(c->seg, C, g.V, gb, g.part);
-        k_inst_dot_at<<<c->ninst, GM_INST_BLOCK, 0, c->stream>>>(c->seg, g.part, gb, 2);
-        k_perturb_at<<<cb, BLOCK, 0, c->stream>>>(C, c->s.N, g.U, g.V, gb, c->prop[0], g.q1);
-        CU(cudaGetLastError());
-        c->launches += 3;
-        TRY(gm_derivative(c, g.q1, g.R1, c->precision));
-        // the matvec differences two residuals of the same precision (gmres.c:41-46)
-        k_matvec_finish_at<<<cb, BLOCK, 0, c->stream>>>(C, g.V, g.R1, g.Rm ? g.Rm : c->R, gb, g.w);
-        CU(cudaGetLastError());
-        c->launches += 1;
-        // modified Gram-Schmidt rows 0..k
-        WhileLoop mgs;
-        TRY(while_begin(c, mgs, 2, [&](cudaGraphConditionalHandle h) {
-            k_mgs_enter<<<1, 1, 0, c->stream>>>(gb, h);
-            c->launches += 1;
-        }));
-        k_mgs_piece<<<c->npieces, BLOCK, 0, c->stream>>>(c->seg, C, g.V, gb, 0, g.w, g.part);
-        k_inst_dot_at<<<c->ninst, GM_INST_BLOCK, 0, c->stream>>>(c->seg, g.part, gb, 0);
-        k_mgs_next<<<1, 1, 0, c->stream>>>(gb, mgs.h);
-        CU(cudaGetLastError());
-        c->launches += 3;
-        TRY(while_end(c, mgs));
-        // the last row's update and the norm of w
-        k_mgs_piece<<<c->npieces, BLOCK, 0, c->stream>>>(c->seg, C, g.V, gb, 1, g.w, g.part);
-        k_inst_dot_at<<<c->ninst, GM_INST_BLOCK, 0, c->stream>>>(c->seg, g.part, gb, 1);
-        CU(cudaMemsetAsync(g.count + 1, 0, sizeof(int), c->stream));
-        k_givens_at<<<ib, 128, 0, c->stream>>>(gb);
-        k_normalize_at<<<cb, BLOCK, 0, c->stream>>>(C, g.w, gb, g.V);
-        k_arnoldi_next<<<1, 1, 0, c->stream>>>(gb, arnoldi.h);
-        CU(cudaGetLastError());
-        c->launches += 5;
-    }
-    TRY(while_end(c, arnoldi));
-    k_backsolve<<<ib, 128, 0, c->stream>>>(gb);
-    k_accumulate<<<cb, BLOCK, 0, c->stream>>>(C, g.V, gb, g.delta);
+    // matvec (gmres.c:12-50); it differences two residuals of the same precision (gmres.c:41-46)
+    k_krylov_vector<<<cb, BLOCK, 0, c->stream>>>(C, c->s.N, g.U, g.r, g.w, gb, c->prop[0], g.V, g.q1);
     CU(cudaGetLastError());
-    c->launches += 2;
+    TRY(gm_derivative(c, g.q1, g.R1, c->precision));
+    k_arnoldi_dots<<<g.nchunks, KRYLOV_BLOCK, 0, c->stream>>>(C, g.V, g.R1, g.Rm ? g.Rm : c->R, gb, g.w);
+    k_arnoldi_update<<<g.nchunks, KRYLOV_BLOCK, 0, c->stream>>>(C, g.V, gb, g.w, arnoldi.h);
+    CU(cudaGetLastError());
+    c->launches += 3;
+    TRY(while_end(c, arnoldi));
     return TG_OK;
 }
 
@@ -2483,7 +2449,7 @@ static int enqueue_implicit_step(tg_ctx *c, double courant, double newton_tol, d
 {
     Gmres &g = c->gm;
     const GmresBatch gb = gm_batch(c, dim);
-    const int C = c->s.C, cb = grid_of(C), ib = inst_grid(c);
+    const int C = c->s.C, cb = grid_of(C);
     const size_t n = 5 * (size_t)C;
     // finite-difference perturbation relative to the state: teal's 1e-6 (advance.c:157) in FP64;
     // the FP32-flux form's residual carries ~1e-7 relative rounding, so it perturbs by 3e-4
@@ -2495,44 +2461,33 @@ static int enqueue_implicit_step(tg_ctx *c, double courant, double newton_tol, d
         Launch l(c, TG_PROF_REDUCE);
         k_inst_begin<<<c->ninst, INST_BLOCK, 0, c->stream>>>(c->seg, c->part_min, courant, c->st);
     }
-    k_newton_begin<<<ib, 128, 0, c->stream>>>(gb, c->st);
     CU(cudaGetLastError());
     CU(cudaMemcpyAsync(g.U, c->U0, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-    CU(cudaMemcpyAsync(g.Ustart, c->U0, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
     c->prepared = false;
 
-    TRY(gm_derivative(c, c->q, c->R, newton_precision(c)));
-    if (g.Rm) TRY(gm_derivative(c, c->q, g.Rm, c->precision));
-    k_newton_init<<<cb, BLOCK, 0, c->stream>>>(C, c->R, gb, g.r);
-    CU(cudaGetLastError());
-    TRY(gm_dot(c, gb, g.r, g.r, GF_NEWTON, GS_NORM, 1));
-    TRY(gm_dot(c, gb, g.U, g.U, GF_NEWTON, GS_CONS_NORM, 1));
-    k_fd_scale<<<ib, 128, 0, c->stream>>>(gb, fd_rel, newton_tol, 1);
-    CU(cudaGetLastError());
-    c->launches += 4;
-    auto newton_check = [&](cudaGraphConditionalHandle h, int enter) {
-        cudaMemsetAsync(g.count, 0, sizeof(int), c->stream);
-        k_newton_check<<<ib, 128, 0, c->stream>>>(gb, c->seg, c->st);
-        k_newton_next<<<1, 1, 0, c->stream>>>(gb, h, enter, c->st.error);
-        c->launches += 2;
-    };
-    WhileLoop newton;
-    TRY(while_begin(c, newton, 0, [&](cudaGraphConditionalHandle h) { newton_check(h, 1); }));
-    {
-        TRY(gm_solve(c, gb, krylov_tol));
-        k_newton_update<<<cb, BLOCK, 0, c->stream>>>(C, c->s.N, g.U, g.delta, gb, c->prop[0], c->q);
-        CU(cudaGetLastError());
+    // derivative of the iterate, Newton residual, its norms, the loop test
+    auto newton_residual = [&](cudaGraphConditionalHandle h, int first) -> int {
         TRY(gm_derivative(c, c->q, c->R, newton_precision(c)));
         if (g.Rm) TRY(gm_derivative(c, c->q, g.Rm, c->precision));
-        k_newton_residual<<<cb, BLOCK, 0, c->stream>>>(C, g.U, g.Ustart, c->R, gb, g.r);
+        k_newton_residual<<<g.nchunks, KRYLOV_BLOCK, 0, c->stream>>>(C, g.U, c->U0, c->R, gb, c->seg, c->st, fd_rel,
+                                                                     newton_tol, krylov_tol, first, g.r, h);
         CU(cudaGetLastError());
-        TRY(gm_dot(c, gb, g.r, g.r, GF_NEWTON, GS_NORM, 1));
-        TRY(gm_dot(c, gb, g.U, g.U, GF_NEWTON, GS_CONS_NORM, 1));
-        k_fd_scale<<<ib, 128, 0, c->stream>>>(gb, fd_rel, newton_tol, 0);
+        c->launches += 1;
+        return TG_OK;
+    };
+    WhileLoop newton;
+    TRY(while_begin(c, newton, 0, [&](cudaGraphConditionalHandle h) -> int {
+        k_newton_begin<<<1, KRYLOV_BLOCK, 0, c->stream>>>(gb, c->st, h);
         CU(cudaGetLastError());
-        c->launches += 3;
-        newton_check(newton.h, 0);
+        c->launches += 1;
+        return newton_residual(h, 1);
+    }));
+    {
+        TRY(gm_solve(c, gb));
+        k_newton_update<<<cb, BLOCK, 0, c->stream>>>(C, c->s.N, g.U, g.V, gb, c->prop[0], c->q);
         CU(cudaGetLastError());
+        c->launches += 1;
+        TRY(newton_residual(newton.h, 0));
     }
     TRY(while_end(c, newton));
     // residual of the last derivative (advance.c:188), time, iteration and the run loop's tests

@@ -15,36 +15,63 @@ namespace tg {
 // scalar slots of an instance's block in the device scalar array
 enum GmresScalar {
     GS_NORM = 0,       // Newton residual norm
-    GS_CONS_NORM = 1,  // norm of the conserved state
-    GS_FD_SCALE = 2,   // finite-difference scale
-    GS_VNORM = 3,      // norm of the Krylov vector being multiplied
-    GS_STEP = 4,       // time step
-    GS_KTOL = 5,       // Krylov tolerance * norm
-    GS_TOL_NORM = 6,   // Newton tolerance * first norm
-    GS_HEAD = 8        // H [(dim+1) x dim], cs [dim], sn [dim], rhs [dim+1], coef [dim]
+    GS_FD_SCALE = 1,   // finite-difference scale
+    GS_STEP = 2,       // time step
+    GS_KTOL = 3,       // Krylov tolerance * norm
+    GS_TOL_NORM = 4,   // Newton tolerance * first norm
+    GS_HEAD = 8        // H [(dim+1) x dim], cs [dim], sn [dim], rhs [dim+1], coef [dim], G [dim x dim]
 };
 
 // per-instance flags: Newton iterating, Arnoldi iterating, Krylov vectors used, Newton iterations
 enum GmresFlag { GF_NEWTON = 0, GF_ARNOLDI = 1, GF_M = 2, GF_ITER = 3, GF_COUNT = 4 };
 
-// device loop counters of the graph-driven solve: the Arnoldi column k, the Gram-Schmidt row i and
-// the Newton iterations of the current step
-enum GmresControl { GC_K = 0, GC_I = 1, GC_N = 2, GC_COUNT = 3 };
+// device loop counters of the graph-driven solve: the Arnoldi column k, the Newton iterations of the
+// current step, the instances that take part in the current Newton iteration and in the current
+// Arnoldi column, and of these the ones that have finished it and the ones that go on
+enum GmresControl {
+    GC_K = 0,
+    GC_N = 1,
+    GC_IN_NEWTON = 2,
+    GC_IN_ARNOLDI = 3,
+    GC_DONE = 4,
+    GC_GOING = 5,
+    GC_COUNT = 6
+};
 
 // Newton iterations one implicit step may take on the device before it stops with ERR_LOOP_LIMIT
 // (teal's own bound, 128 (cells + 1) per instance, advance.c:162, stays in force below it); the
 // bound keeps every device loop of the step graph finite
 constexpr int NEWTON_LOOP_LIMIT = 1000;
 
+// Cell chunks of the Krylov vectors: ranges of cells that never straddle two instances, one block
+// each. A chunk is KRYLOV_BLOCK cells (one per thread, so the vector being orthogonalised stays in
+// registers) up to KRYLOV_CHUNKS chunks an instance, two resident blocks on each of 148 SMs; larger
+// instances get larger chunks, so that one block can still sum an instance's partials.
+constexpr int KRYLOV_BLOCK = 256;
+constexpr int KRYLOV_CHUNKS = 296;
+// basis vectors per shared-memory accumulator tile, and loaded together
+constexpr int KRYLOV_TILE = 64;
+constexpr int KRYLOV_GROUP = 4;
+
+inline int krylov_chunk(long cells)
+{
+    const long per = (cells + KRYLOV_CHUNKS - 1) / KRYLOV_CHUNKS;
+    return (int)((per + KRYLOV_BLOCK - 1) / KRYLOV_BLOCK * KRYLOV_BLOCK);
+}
+
 struct GmresBatch {
     int dim;    // Krylov dimension
     int scn;    // doubles per instance block of `sc`
     int ninst;
+    int nchunks;
     const int *__restrict__ cell_inst;
-    double *sc;  // [ninst][scn]
-    int *flag;   // [GF_COUNT][ninst]
-    int *count;  // [2] instances still iterating (Newton, Arnoldi)
-    int *ctl;    // [GC_COUNT] loop counters read by the kernels of one Arnoldi iteration
+    const int *__restrict__ chunk_beg;       // [nchunks + 1]
+    const int *__restrict__ inst_chunk_off;  // [ninst + 1]
+    double *part;  // [2 dim + 1][nchunks] partial sums of the chunks
+    int *ticket;   // [ninst] chunks of the instance that have finished the current pass
+    double *sc;    // [ninst][scn]
+    int *flag;     // [GF_COUNT][ninst]
+    int *ctl;      // [GC_COUNT]
 
     __device__ __forceinline__ double *s(int i) const { return sc + (size_t)i * scn; }
     __device__ __forceinline__ double *H(int i, int r, int k) const { return s(i) + GS_HEAD + r * dim + k; }
@@ -52,6 +79,7 @@ struct GmresBatch {
     __device__ __forceinline__ double *sn(int i) const { return cs(i) + dim; }
     __device__ __forceinline__ double *rhs(int i) const { return sn(i) + dim; }
     __device__ __forceinline__ double *coef(int i) const { return rhs(i) + dim + 1; }
+    __device__ __forceinline__ double *G(int i, int r) const { return coef(i) + dim + r * dim; }
     __device__ __forceinline__ int &newton(int i) const { return flag[GF_NEWTON * ninst + i]; }
     __device__ __forceinline__ int &arnoldi(int i) const { return flag[GF_ARNOLDI * ninst + i]; }
     __device__ __forceinline__ int &m(int i) const { return flag[GF_M * ninst + i]; }
@@ -60,221 +88,192 @@ struct GmresBatch {
 
 __host__ __device__ inline int gmres_scn(int dim)
 {
-    return GS_HEAD + (dim + 1) * dim + 4 * dim + 2;
+    return GS_HEAD + (dim + 1) * dim + 4 * dim + 2 + dim * dim;
 }
 
-// per-piece partial sums of x . y over the 5 variables of the piece's cells; pieces of instances
-// whose flag `which` is off are skipped (their sums are not read)
-__global__ void __launch_bounds__(BLOCK) k_piece_dot(Segments seg, int C, const double *__restrict__ x,
-                                                     const double *__restrict__ y, GmresBatch gb, int which,
-                                                     double *__restrict__ part)
+// Whether this block is the last one of its instance to finish the current pass: its chunk's
+// partials are then visible to it with those of all other chunks. The same answer in every thread.
+__device__ __forceinline__ bool last_of_instance(const GmresBatch &gb, int inst)
 {
-    __shared__ double sh[BLOCK / 32];
-    const int beg = seg.piece_beg[blockIdx.x], end = seg.piece_beg[blockIdx.x + 1];
-    if (!gb.flag[which * gb.ninst + gb.cell_inst[beg]]) {
+    __shared__ int last;
+    __threadfence();  // this thread's partials before the ticket
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const int n = gb.inst_chunk_off[inst + 1] - gb.inst_chunk_off[inst];
+        last = atomicAdd(gb.ticket + inst, 1) == n - 1;
+        if (last) {
+            gb.ticket[inst] = 0;  // for the next pass
+        }
+    }
+    __syncthreads();
+    if (last) {
+        __threadfence();
+    }
+    return last != 0;
+}
+
+// One warp's sum of partial-sum row v over the instance's chunks, in every lane
+__device__ __forceinline__ double sum_chunks(const GmresBatch &gb, int inst, int v, int lane)
+{
+    const int beg = gb.inst_chunk_off[inst], end = gb.inst_chunk_off[inst + 1];
+    const double *p = gb.part + (size_t)v * gb.nchunks;
+    double t = 0;
+    for (int c = beg + lane; c < end; c += 32) {
+        t += __ldcg(p + c);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        t += __shfl_xor_sync(0xffffffffu, t, o);
+    }
+    return t;
+}
+
+// An instance has finished the current Newton iteration or Arnoldi column and goes on or not. True in
+// the thread that closes it for all instances (*going: the instances that go on). `in`: GC_IN_NEWTON or
+// GC_IN_ARNOLDI. Called by one thread of the instance's last block.
+__device__ __forceinline__ bool last_instance(const GmresBatch &gb, int in, bool goes_on, int *going)
+{
+    if (goes_on) {
+        atomicAdd(gb.ctl + GC_GOING, 1);
+    }
+    __threadfence();
+    if (atomicAdd(gb.ctl + GC_DONE, 1) != gb.ctl[in] - 1) {
+        return false;
+    }
+    __threadfence();
+    *going = atomicAdd(gb.ctl + GC_GOING, 0);
+    gb.ctl[GC_GOING] = 0;
+    gb.ctl[GC_DONE] = 0;
+    gb.ctl[in] = *going;
+    return true;
+}
+
+// start of a step, one block: Newton flag on for the active instances, steps copied; the Newton loop's
+// condition off (the residual kernel turns it on when an instance iterates)
+__global__ void __launch_bounds__(KRYLOV_BLOCK) k_newton_begin(GmresBatch gb, Steps st,
+                                                               cudaGraphConditionalHandle h)
+{
+    __shared__ int n;
+    if (threadIdx.x == 0) {
+        n = 0;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < gb.ninst; i += blockDim.x) {
+        const int on = st.active[i] != 0;
+        gb.newton(i) = on;
+        gb.arnoldi(i) = 0;
+        gb.m(i) = 0;
+        gb.iter(i) = 0;
+        gb.ticket[i] = 0;
+        if (on) {
+            gb.s(i)[GS_STEP] = st.step[i];
+            atomicAdd(&n, 1);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        gb.ctl[GC_N] = 0;
+        gb.ctl[GC_IN_NEWTON] = n;
+        gb.ctl[GC_DONE] = 0;
+        gb.ctl[GC_GOING] = 0;
+        cudaGraphSetConditional(h, 0u);
+    }
+}
+
+// Newton residual of every iterating instance, its norms and the loop test.
+//   first: r = -R step (advance.c:148-153), else r = U - U0 - R step (advance.c:176-181);
+//   fd_scale = fd_rel max(1, |U|) / max(1, |r|) (advance.c:155-159, fd_rel = 1e-6 there), on the first
+//   call of a step also the Newton target tol |r|;
+//   loop test (advance.c:162-165): iterate while |r| > tol |r0| and within 128 (cells + 1) iterations;
+//   a non-finite norm marks the instance failed;
+//   an instance that iterates starts its GMRES cycle (gmres.c:68-83): rhs = (norm, 0, ...), Arnoldi on.
+// 360 bytes a cell are read and written once; the rest is latency (a ticket and a sum over chunks).
+__global__ void __launch_bounds__(KRYLOV_BLOCK) k_newton_residual(int C, const double *__restrict__ U,
+                                                                  const double *__restrict__ U0,
+                                                                  const double *__restrict__ R, GmresBatch gb,
+                                                                  Segments seg, Steps st, double fd_rel,
+                                                                  double newton_tol, double krylov_tol, int first,
+                                                                  double *__restrict__ r,
+                                                                  cudaGraphConditionalHandle h)
+{
+    __shared__ double sh[KRYLOV_BLOCK / 32];
+    const int beg = gb.chunk_beg[blockIdx.x], end = gb.chunk_beg[blockIdx.x + 1];
+    const int inst = gb.cell_inst[beg];
+    if (!gb.newton(inst)) {
         return;
     }
-    double t = 0;
-    for (int c = beg + threadIdx.x; c < end; c += BLOCK) {
+    double *s = gb.s(inst);
+    const double step = s[GS_STEP];
+    double rr = 0, uu = 0;
+    for (int c = beg + threadIdx.x; c < end; c += KRYLOV_BLOCK) {
 #pragma unroll
         for (int v = 0; v < 5; v++) {
-            t += x[(size_t)v * C + c] * y[(size_t)v * C + c];
+            const size_t k = (size_t)v * C + c;
+            const double u = U[k];
+            const double x = first ? -R[k] * step : (u - U0[k]) - (R[k] * step);
+            r[k] = x;
+            rr += x * x;
+            uu += u * u;
         }
     }
-    double sum = block_sum<BLOCK>(t, sh);
+    rr = block_sum<KRYLOV_BLOCK>(rr, sh);
+    uu = block_sum<KRYLOV_BLOCK>(uu, sh);
     if (threadIdx.x == 0) {
-        part[blockIdx.x] = sum;
+        gb.part[blockIdx.x] = rr;
+        gb.part[gb.nchunks + blockIdx.x] = uu;
     }
-}
-
-constexpr int GM_INST_BLOCK = 128;
-
-// sc[inst][slot] = sum of the instance's piece partials (or its square root), for instances whose
-// flag `which` is set
-__global__ void __launch_bounds__(GM_INST_BLOCK) k_inst_dot(Segments seg, const double *__restrict__ part,
-                                                           GmresBatch gb, int which, int slot, int take_sqrt)
-{
-    __shared__ double sh[GM_INST_BLOCK / 32];
-    const int i = blockIdx.x;
-    if (!gb.flag[which * gb.ninst + i]) {
+    if (!last_of_instance(gb, inst) || threadIdx.x >= 32) {
         return;
     }
-    double t = 0;
-    for (int p = seg.inst_piece_off[i] + threadIdx.x; p < seg.inst_piece_off[i + 1]; p += GM_INST_BLOCK) {
-        t += part[p];
-    }
-    double sum = block_sum<GM_INST_BLOCK>(t, sh);
-    if (threadIdx.x == 0) {
-        gb.s(i)[slot] = take_sqrt ? sqrt(sum) : sum;
-    }
-}
-
-// start of a step for every instance: Newton flag on for the active ones, step copied
-__global__ void k_newton_begin(GmresBatch gb, Steps st)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= gb.ninst) {
+    const double norm = sqrt(sum_chunks(gb, inst, 0, threadIdx.x));
+    const double cons = sqrt(sum_chunks(gb, inst, 1, threadIdx.x));
+    if (threadIdx.x != 0) {
         return;
     }
-    const int on = st.active[i] != 0;
-    gb.newton(i) = on;
-    gb.arnoldi(i) = 0;
-    gb.m(i) = 0;
-    gb.iter(i) = 0;
-    if (on) {
-        gb.s(i)[GS_STEP] = st.step[i];
-    }
-}
-
-// r = -R * step (advance.c:148-153)
-__global__ void k_newton_init(int C, const double *__restrict__ R, GmresBatch gb, double *__restrict__ r)
-{
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C) {
-        return;
-    }
-    const int i = gb.cell_inst[c];
-    if (!gb.newton(i)) {
-        return;
-    }
-    const double step = gb.s(i)[GS_STEP];
-#pragma unroll
-    for (int v = 0; v < 5; v++) {
-        r[(size_t)v * C + c] = -R[(size_t)v * C + c] * step;
-    }
-}
-
-// r = U - U0 - R * step (advance.c:176-181)
-__global__ void k_newton_residual(int C, const double *__restrict__ U, const double *__restrict__ U0,
-                                  const double *__restrict__ R, GmresBatch gb, double *__restrict__ r)
-{
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C) {
-        return;
-    }
-    const int i = gb.cell_inst[c];
-    if (!gb.newton(i)) {
-        return;
-    }
-    const double step = gb.s(i)[GS_STEP];
-#pragma unroll
-    for (int v = 0; v < 5; v++) {
-        size_t k = (size_t)v * C + c;
-        r[k] = (U[k] - U0[k]) - (R[k] * step);
-    }
-}
-
-// fd_scale = fd_rel * max(1, |U|) / max(1, |r|) (advance.c:155-159, fd_rel = 1e-6 there); on the
-// first call of a step also the Newton target tol * |r|
-__global__ void k_fd_scale(GmresBatch gb, double fd_rel, double newton_tol, int first)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= gb.ninst || !gb.newton(i)) {
-        return;
-    }
-    double *s = gb.s(i);
-    s[GS_FD_SCALE] = fd_rel * fmax(1.0, s[GS_CONS_NORM]) / fmax(1.0, s[GS_NORM]);
+    s[GS_NORM] = norm;
+    s[GS_FD_SCALE] = fd_rel * fmax(1.0, cons) / fmax(1.0, norm);
     if (first) {
-        s[GS_TOL_NORM] = newton_tol * s[GS_NORM];
+        s[GS_TOL_NORM] = newton_tol * norm;
     }
-}
-
-// Newton loop test per instance (advance.c:162-165): keep iterating while |r| > tol * |r0| and
-// within 128 (cells + 1) iterations; a non-finite norm marks the instance failed. count[0] = instances
-// that go on.
-__global__ void k_newton_check(GmresBatch gb, Segments seg, Steps st)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= gb.ninst || !gb.newton(i)) {
-        return;
-    }
-    const double norm = gb.s(i)[GS_NORM];
+    bool on;
     if (!isfinite(norm)) {  // the instance stops (its residual follows as non-finite); the others go on
         atomicOr(st.error, ERR_NONFINITE);
-        st.fail[i] = 1;
-        gb.newton(i) = 0;
-        return;
+        st.fail[inst] = 1;
+        on = false;
     }
-    const long max_iter = 128L * (seg.inst_cell_off[i + 1] - seg.inst_cell_off[i] + 1);
-    const long it = gb.iter(i);
-    if (!(norm > gb.s(i)[GS_TOL_NORM]) || it >= max_iter) {
-        gb.newton(i) = 0;
-        return;
+    else {
+        const long max_iter = 128L * (seg.inst_cell_off[inst + 1] - seg.inst_cell_off[inst] + 1);
+        on = norm > s[GS_TOL_NORM] && gb.iter(inst) < max_iter;
     }
-    atomicAdd(&gb.count[0], 1);
-}
-
-// start of a GMRES cycle (gmres.c:68-83) per Newton instance: rhs = (norm, 0, ...), Arnoldi on
-// unless the residual is already zero
-__global__ void k_gmres_begin(GmresBatch gb, double krylov_tol)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= gb.ninst) {
-        return;
-    }
-    gb.arnoldi(i) = 0;
-    gb.m(i) = 0;
-    if (!gb.newton(i)) {
-        return;
-    }
-    double *s = gb.s(i);
-    const double norm = s[GS_NORM];
-    double *rhs = gb.rhs(i);
-    for (int k = 0; k <= gb.dim; k++) {
-        rhs[k] = 0.0;
-    }
-    rhs[0] = norm;
-    s[GS_KTOL] = krylov_tol * norm;
-    gb.arnoldi(i) = norm > 0;
-    gb.iter(i) += 1;
-}
-
-// V0 = -r / norm and delta = 0 for every Newton instance (delta stays 0 when the norm is 0)
-__global__ void k_gmres_start(int C, const double *__restrict__ r, GmresBatch gb, double *__restrict__ V0,
-                              double *__restrict__ delta)
-{
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C) {
-        return;
-    }
-    const int i = gb.cell_inst[c];
-    if (!gb.newton(i)) {
-        return;
-    }
-    const double norm = gb.s(i)[GS_NORM];
-    const bool on = gb.arnoldi(i) != 0;
-#pragma unroll
-    for (int v = 0; v < 5; v++) {
-        size_t k = (size_t)v * C + c;
-        if (on) {
-            V0[k] = -r[k] / norm;
+    gb.newton(inst) = on;
+    gb.arnoldi(inst) = on;  // |r| > tol |r0| >= 0
+    gb.m(inst) = 0;
+    if (on) {
+        double *rhs = gb.rhs(inst);
+        for (int k = 0; k <= gb.dim; k++) {
+            rhs[k] = 0.0;
         }
-        delta[k] = 0.0;
+        rhs[0] = norm;
+        s[GS_KTOL] = krylov_tol * norm;
+        gb.iter(inst) += 1;
     }
-}
-
-// back substitution coefficients for the instance's m Krylov vectors (gmres.c:128-136)
-__global__ void k_backsolve(GmresBatch gb)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= gb.ninst || !gb.newton(i)) {
-        return;
-    }
-    const int m = gb.m(i);
-    double *rhs = gb.rhs(i), *coef = gb.coef(i);
-    for (int r = m - 1; r >= 0; r--) {
-        double cr = rhs[r];
-        for (int j = r + 1; j < m; j++) {
-            cr -= *gb.H(i, r, j) * coef[j];
+    int going;
+    if (last_instance(gb, GC_IN_NEWTON, on, &going)) {
+        const int n = first ? 0 : gb.ctl[GC_N] + 1;
+        gb.ctl[GC_N] = n;
+        if (going > 0 && n >= NEWTON_LOOP_LIMIT) {
+            atomicOr(st.error, ERR_LOOP_LIMIT);
         }
-        coef[r] = cr / *gb.H(i, r, r);
+        cudaGraphSetConditional(h, (going > 0 && n < NEWTON_LOOP_LIMIT) ? 1u : 0u);
     }
 }
 
-// delta += coef[r] * V_r, r from m-1 down to 0 in one pass (gmres.c:137-141)
-__global__ void k_accumulate(int C, const double *__restrict__ V, GmresBatch gb, double *__restrict__ delta)
+// U += delta, delta = sum of coef[j] V_j with j from m - 1 down to 0 (gmres.c:137-141), q = prim(U)
+// (advance.c:168-173): the basis is read once, the increment is not stored
+__global__ void k_newton_update(int C, int N, double *__restrict__ U, const double *__restrict__ V, GmresBatch gb,
+                                double gamma, double *__restrict__ q)
 {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) {
         return;
     }
@@ -285,304 +284,294 @@ __global__ void k_accumulate(int C, const double *__restrict__ V, GmresBatch gb,
     const int m = gb.m(i);
     const double *coef = gb.coef(i);
     const size_t n = 5 * (size_t)C;
+    double d[5] = {0, 0, 0, 0, 0};
+#pragma unroll 2
+    for (int j = m - 1; j >= 0; j--) {
+        const double a = coef[j];
 #pragma unroll
-    for (int v = 0; v < 5; v++) {
-        size_t j = (size_t)v * C + c;
-        double d = delta[j];
-        for (int r = m - 1; r >= 0; r--) {
-            d += coef[r] * V[(size_t)r * n + j];
+        for (int v = 0; v < 5; v++) {
+            d[v] += a * V[(size_t)j * n + (size_t)v * C + c];
         }
-        delta[j] = d;
-    }
-}
-
-// U += delta, q = prim(U) (advance.c:168-173)
-__global__ void k_newton_update(int C, int N, double *__restrict__ U, const double *__restrict__ delta,
-                                GmresBatch gb, double gamma, double *__restrict__ q)
-{
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C) {
-        return;
-    }
-    if (!gb.newton(gb.cell_inst[c])) {
-        return;
     }
     Cons<double> u;
-    u.rho = U[c] += delta[c];
-    u.m.x = U[C + c] += delta[C + c];
-    u.m.y = U[2 * C + c] += delta[2 * C + c];
-    u.m.z = U[3 * C + c] += delta[3 * C + c];
-    u.e = U[4 * C + c] += delta[4 * C + c];
-    Prim<double> p = cons_to_prim(u, gamma);
-    q[c] = p.rho;
-    q[N + c] = p.u.x;
-    q[2 * N + c] = p.u.y;
-    q[3 * N + c] = p.u.z;
-    q[4 * N + c] = p.p;
+    u.rho = U[c] += d[0];
+    u.m.x = U[C + c] += d[1];
+    u.m.y = U[2 * (size_t)C + c] += d[2];
+    u.m.z = U[3 * (size_t)C + c] += d[3];
+    u.e = U[4 * (size_t)C + c] += d[4];
+    store_prim(q, N, c, cons_to_prim(u, gamma));
 }
 
 // ---- device-driven loops ------------------------------------------------------------------------
 //
-// The implicit step runs from one CUDA graph whose Newton, Arnoldi and Gram-Schmidt loops are
-// conditional WHILE nodes: the kernels below read the loop counters (GmresBatch::ctl) from device
-// memory instead of taking them as launch arguments, and the last kernel of each loop body sets
-// the loop's condition, so no iteration waits for the host. Each kernel does the same arithmetic
-// in the same order as the host-driven sequence it replaces, so the results keep their bits.
+// The implicit step runs from one CUDA graph whose Newton and Arnoldi loops are conditional WHILE
+// nodes: the kernels below read the loop counters (GmresBatch::ctl) from device memory instead of
+// taking them as launch arguments, and the last block of a body's last kernel sets the loop's
+// condition, so no iteration waits for the host.
 
-// Newton loop condition: go on while some instance iterates (count[0], set by k_newton_check) and
-// the step's iterations stay below NEWTON_LOOP_LIMIT; `enter` starts the count of the step
-__global__ void k_newton_next(GmresBatch gb, cudaGraphConditionalHandle h, int enter, int *err)
-{
-    const int n = enter ? 0 : gb.ctl[GC_N] + 1;
-    gb.ctl[GC_N] = n;
-    const bool going = gb.count[0] > 0;
-    if (going && n >= NEWTON_LOOP_LIMIT) {
-        atomicOr(err, ERR_LOOP_LIMIT);
-    }
-    cudaGraphSetConditional(h, (going && n < NEWTON_LOOP_LIMIT) ? 1u : 0u);
-}
-
-// start of an Arnoldi loop: k = 0; count[1] = instances whose Arnoldi flag is set; the loop's
-// condition from it
+// start of an Arnoldi loop (one thread): column 0 of every instance that iterates
 __global__ void k_arnoldi_enter(GmresBatch gb, cudaGraphConditionalHandle h)
 {
-    __shared__ int n;
-    if (threadIdx.x == 0) {
-        n = 0;
-        gb.ctl[GC_K] = 0;
-    }
-    __syncthreads();
-    int t = 0;
-    for (int i = threadIdx.x; i < gb.ninst; i += blockDim.x) {
-        t += gb.arnoldi(i) != 0;
-    }
-    atomicAdd(&n, t);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        cudaGraphSetConditional(h, n > 0 ? 1u : 0u);
-    }
+    const int n = gb.ctl[GC_IN_NEWTON];
+    gb.ctl[GC_K] = 0;
+    gb.ctl[GC_IN_ARNOLDI] = n;
+    cudaGraphSetConditional(h, n > 0 ? 1u : 0u);
 }
 
-// start of the Gram-Schmidt loop of column k: i = 0, condition on (the body runs at least once)
-__global__ void k_mgs_enter(GmresBatch gb, cudaGraphConditionalHandle h)
+// Krylov vector k, V_0 = -r / |r| or V_k = w / H[k][k-1] (gmres.c:75, :121-125), and the state it
+// perturbs, q1 = prim(U + eps V_k) with eps = fd_scale / |V_k| (gmres.c:26-36): V_k has just been
+// divided by its norm, so |V_k| is 1 to rounding and is not summed again (it scales a
+// finite-difference step, whose own truncation error is some ten orders larger).
+__global__ void k_krylov_vector(int C, int N, const double *__restrict__ U, const double *__restrict__ r,
+                                const double *__restrict__ w, GmresBatch gb, double gamma, double *__restrict__ V,
+                                double *__restrict__ q1)
 {
-    gb.ctl[GC_I] = 0;
-    cudaGraphSetConditional(h, 1u);
-}
-
-// per-piece partials of V_k . V_k (the norm of the vector being multiplied, gmres.c:26)
-__global__ void __launch_bounds__(BLOCK) k_piece_vnorm(Segments seg, int C, const double *__restrict__ V,
-                                                       GmresBatch gb, double *__restrict__ part)
-{
-    __shared__ double sh[BLOCK / 32];
-    const double *x = V + (size_t)gb.ctl[GC_K] * 5 * (size_t)C;
-    const int beg = seg.piece_beg[blockIdx.x], end = seg.piece_beg[blockIdx.x + 1];
-    if (!gb.arnoldi(gb.cell_inst[beg])) {  // the instance left its Arnoldi loop
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= C) {
         return;
     }
-    double t = 0;
-    for (int c = beg + threadIdx.x; c < end; c += BLOCK) {
+    const int i = gb.cell_inst[c];
+    const int k = gb.ctl[GC_K];
+    if (!gb.arnoldi(i)) {
+        return;
+    }
+    const double *x = (k == 0) ? r : w;
+    const double norm = (k == 0) ? -gb.s(i)[GS_NORM] : *gb.H(i, k, k - 1);
+    const double eps = gb.s(i)[GS_FD_SCALE];
+    double *Vk = V + (size_t)k * 5 * (size_t)C;
+    double u[5];
 #pragma unroll
-        for (int v = 0; v < 5; v++) {
-            t += x[(size_t)v * C + c] * x[(size_t)v * C + c];
+    for (int v = 0; v < 5; v++) {
+        const size_t j = (size_t)v * C + c;
+        const double y = x[j] / norm;
+        Vk[j] = y;
+        u[v] = U[j] + (eps * y);
+    }
+    store_prim(q1, N, c, cons_to_prim(Cons<double>{u[0], v3(u[1], u[2], u[3]), u[4]}, gamma));
+}
+
+// Sums of 8 values over the lanes of a warp in 9 exchanges (a butterfly that halves the values as it
+// halves the lanes); lane l returns the sum of value l / 4.
+__device__ __forceinline__ double warp_sum8(double (&a)[8], int lane)
+{
+#pragma unroll
+    for (int o = 16, n = 4; o >= 4; o >>= 1, n >>= 1) {
+        const bool hi = lane & o;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            if (j < n) {
+                const double send = hi ? a[j] : a[j + n], keep = hi ? a[j + n] : a[j];
+                a[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
         }
     }
-    double sum = block_sum<BLOCK>(t, sh);
-    if (threadIdx.x == 0) {
-        part[blockIdx.x] = sum;
+    double t = a[0];
+    t += __shfl_xor_sync(0xffffffffu, t, 2);
+    t += __shfl_xor_sync(0xffffffffu, t, 1);
+    return t;
+}
+
+// First pass of Arnoldi column k: w = V_k - step (R1 - R) / eps (gmres.c:41-46), t_i = V_i . w for
+// i <= k and G_ki = V_i . V_k for i < k; the instance's last block then gets column k of H.
+// Bound by the basis it reads (40 (k + 1) bytes a cell): w and V_k stay in registers, the loads of
+// KRYLOV_GROUP basis vectors are in flight together and their 2 x KRYLOV_GROUP products are
+// summed over the warp at once.
+__global__ void __launch_bounds__(KRYLOV_BLOCK, 2) k_arnoldi_dots(int C, const double *__restrict__ V,
+                                                                  const double *__restrict__ R1,
+                                                                  const double *__restrict__ R, GmresBatch gb,
+                                                                  double *__restrict__ w)
+{
+    constexpr int WARPS = KRYLOV_BLOCK / 32;
+    __shared__ double acc[WARPS][2 * KRYLOV_TILE];
+    const int beg = gb.chunk_beg[blockIdx.x], end = gb.chunk_beg[blockIdx.x + 1];
+    const int inst = gb.cell_inst[beg];
+    if (!gb.arnoldi(inst)) {
+        return;
+    }
+    const int k = gb.ctl[GC_K], dim = gb.dim;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const size_t n = 5 * (size_t)C;
+    const double *s = gb.s(inst);
+    const double eps = s[GS_FD_SCALE], step = s[GS_STEP];
+    for (int i0 = 0; i0 <= k; i0 += KRYLOV_TILE) {
+        const int ni = min(KRYLOV_TILE, k + 1 - i0);
+        for (int i = lane; i < 2 * KRYLOV_TILE; i += 32) {
+            acc[warp][i] = 0.0;
+        }
+        __syncwarp();
+        // whole warps take part in every round: lanes past the end hold zeros
+        for (int c0 = beg + 32 * warp; c0 < end; c0 += KRYLOV_BLOCK) {
+            const int c = c0 + lane;
+            const bool in = c < end;
+            double x[5], vk[5];
+#pragma unroll
+            for (int v = 0; v < 5; v++) {
+                const size_t j = (size_t)v * C + c;
+                x[v] = vk[v] = 0.0;
+                if (in) {
+                    vk[v] = V[(size_t)k * n + j];
+                    if (i0 == 0) {
+                        x[v] = vk[v] - ((step * (R1[j] - R[j])) / eps);
+                        w[j] = x[v];
+                    }
+                    else {
+                        x[v] = w[j];
+                    }
+                }
+            }
+            for (int i = 0; i < ni; i += KRYLOV_GROUP) {
+                double a[2 * KRYLOV_GROUP];
+#pragma unroll
+                for (int g = 0; g < KRYLOV_GROUP; g++) {
+                    double t = 0, u = 0;
+                    if (in && i + g < ni) {
+                        const double *Vi = V + (size_t)(i0 + i + g) * n + c;
+#pragma unroll
+                        for (int v = 0; v < 5; v++) {
+                            const double y = Vi[(size_t)v * C];
+                            t += y * x[v];
+                            u += y * vk[v];
+                        }
+                    }
+                    a[2 * g] = t;
+                    a[2 * g + 1] = u;
+                }
+                const double t = warp_sum8(a, lane);
+                if ((lane & 3) == 0) {
+                    acc[warp][2 * i + (lane >> 2)] += t;
+                }
+                __syncwarp();
+            }
+        }
+        __syncthreads();
+        // part rows: t_i in row i, G_ki in row dim + i
+        for (int i = threadIdx.x; i < 2 * ni; i += KRYLOV_BLOCK) {
+            double t = 0;
+#pragma unroll
+            for (int q = 0; q < WARPS; q++) {
+                t += acc[q][i];
+            }
+            const int row = i0 + (i >> 1);
+            gb.part[(size_t)((i & 1) ? dim + row : row) * gb.nchunks + blockIdx.x] = t;
+        }
+        __syncthreads();
+    }
+    if (!last_of_instance(gb, inst)) {
+        return;
+    }
+    for (int i = warp; i < 2 * k + 1; i += WARPS) {
+        const bool is_t = i <= k;
+        const int row = is_t ? i : i - (k + 1);
+        const double t = sum_chunks(gb, inst, is_t ? row : dim + row, lane);
+        if (lane == 0) {
+            *(is_t ? gb.H(inst, row, k) : gb.G(inst, k) + row) = t;
+        }
+    }
+    __syncthreads();
+    // h = (I + strictly lower G)^-1 t, column by column: h_j is final once all h_i, i < j, are subtracted
+    for (int j = 0; j < k; j++) {
+        const double hj = *(volatile double *)gb.H(inst, j, k);
+        for (int i = j + 1 + threadIdx.x; i <= k; i += KRYLOV_BLOCK) {
+            *gb.H(inst, i, k) -= gb.G(inst, i)[j] * hj;
+        }
+        __syncthreads();
     }
 }
 
-// One Gram-Schmidt row fused with the update of the row before it (gmres.c:92-99): with i > 0,
-// w -= H[i-1][k] V_{i-1} for the cells of Arnoldi instances, then the per-piece partials of
-// V_i . w; after the last row (`last`), w -= H[k][k] V_k and the partials of w . w.
-__global__ void __launch_bounds__(BLOCK) k_mgs_piece(Segments seg, int C, const double *__restrict__ V,
-                                                     GmresBatch gb, int last, double *__restrict__ w,
-                                                     double *__restrict__ part)
+// Second pass of Arnoldi column k: w -= sum of H[i][k] V_i, |w|; the instance's last block then applies
+// and extends the Givens rotations and the right-hand side (gmres.c:102-119); an instance that
+// converged (or filled the basis) stops with m = k + 1 and its coefficients (gmres.c:128-136); the
+// last instance sets the loop's condition. Bound by the basis it reads, as the first pass.
+__global__ void __launch_bounds__(KRYLOV_BLOCK) k_arnoldi_update(int C, const double *__restrict__ V, GmresBatch gb,
+                                                                 double *__restrict__ w,
+                                                                 cudaGraphConditionalHandle h)
 {
-    __shared__ double sh[BLOCK / 32];
-    const size_t n = 5 * (size_t)C;
-    const int k = gb.ctl[GC_K];
-    const int i = last ? k + 1 : gb.ctl[GC_I];
-    const int beg = seg.piece_beg[blockIdx.x], end = seg.piece_beg[blockIdx.x + 1];
-    const int inst = gb.cell_inst[beg];  // a piece lies in one instance
-    if (!gb.arnoldi(inst)) {  // the instance left its Arnoldi loop: nothing to update or sum
+    __shared__ double sh[KRYLOV_BLOCK / 32];
+    __shared__ int stop;
+    const int beg = gb.chunk_beg[blockIdx.x], end = gb.chunk_beg[blockIdx.x + 1];
+    const int inst = gb.cell_inst[beg];
+    if (!gb.arnoldi(inst)) {
         return;
     }
-    const bool update = i > 0;
-    const double h = update ? *gb.H(inst, i - 1, k) : 0.0;
-    const double *Vp = V + (size_t)(i > 0 ? i - 1 : 0) * n;
-    const double *x = last ? w : V + (size_t)i * n;
+    const int k = gb.ctl[GC_K], dim = gb.dim;
+    const size_t n = 5 * (size_t)C;
     double t = 0;
-    for (int c = beg + threadIdx.x; c < end; c += BLOCK) {
-        if (update) {
+    for (int c = beg + threadIdx.x; c < end; c += KRYLOV_BLOCK) {
+        double x[5];
+#pragma unroll
+        for (int v = 0; v < 5; v++) {
+            x[v] = w[(size_t)v * C + c];
+        }
+#pragma unroll 4
+        for (int i = 0; i <= k; i++) {
+            const double hi = *gb.H(inst, i, k);
+            const double *Vi = V + (size_t)i * n + c;
 #pragma unroll
             for (int v = 0; v < 5; v++) {
-                size_t j = (size_t)v * C + c;
-                w[j] -= h * Vp[j];
+                x[v] -= hi * Vi[(size_t)v * C];
             }
         }
 #pragma unroll
         for (int v = 0; v < 5; v++) {
-            size_t j = (size_t)v * C + c;
-            t += x[j] * w[j];
+            w[(size_t)v * C + c] = x[v];
+            t += x[v] * x[v];
         }
     }
-    double sum = block_sum<BLOCK>(t, sh);
+    t = block_sum<KRYLOV_BLOCK>(t, sh);
     if (threadIdx.x == 0) {
-        part[blockIdx.x] = sum;
+        gb.part[blockIdx.x] = t;
     }
-}
-
-// instance sums of the piece partials into H[row][k] (row: i, or k + 1 with the square root) or the
-// vector norm slot, for the Arnoldi instances; slot kinds: 0 = H[i][k], 1 = H[k+1][k] = sqrt, 2 =
-// GS_VNORM = sqrt
-__global__ void __launch_bounds__(GM_INST_BLOCK) k_inst_dot_at(Segments seg, const double *__restrict__ part,
-                                                              GmresBatch gb, int kind)
-{
-    __shared__ double sh[GM_INST_BLOCK / 32];
-    const int i = blockIdx.x;
-    if (!gb.arnoldi(i)) {
+    if (!last_of_instance(gb, inst)) {
         return;
     }
-    double t = 0;
-    for (int p = seg.inst_piece_off[i] + threadIdx.x; p < seg.inst_piece_off[i + 1]; p += GM_INST_BLOCK) {
-        t += part[p];
+    double *cs = gb.cs(inst), *sn = gb.sn(inst), *rhs = gb.rhs(inst), *coef = gb.coef(inst);
+    if (threadIdx.x < 32) {
+        const double norm = sqrt(sum_chunks(gb, inst, 0, threadIdx.x));
+        if (threadIdx.x == 0) {
+            *gb.H(inst, k + 1, k) = norm;
+            double top = *gb.H(inst, 0, k);
+#pragma unroll 4
+            for (int r = 0; r < k; r++) {
+                const double low = *gb.H(inst, r + 1, k);
+                *gb.H(inst, r, k) = (cs[r] * top) + (sn[r] * low);
+                top = (-sn[r] * top) + (cs[r] * low);
+            }
+            const double rot = sqrt((top * top) + (norm * norm));
+            cs[k] = top / rot;
+            sn[k] = norm / rot;
+            *gb.H(inst, k, k) = rot;
+            rhs[k + 1] = -sn[k] * rhs[k];
+            rhs[k] = cs[k] * rhs[k];
+            gb.m(inst) = k + 1;
+            stop = fabs(rhs[k + 1]) < gb.s(inst)[GS_KTOL] || k + 1 >= dim;
+        }
     }
-    double sum = block_sum<GM_INST_BLOCK>(t, sh);
+    __syncthreads();
+    if (stop) {
+        // back substitution, column by column
+        for (int i = threadIdx.x; i <= k; i += KRYLOV_BLOCK) {
+            coef[i] = rhs[i];
+        }
+        __syncthreads();
+        for (int j = k; j >= 0; j--) {
+            if (threadIdx.x == 0) {
+                coef[j] = coef[j] / *gb.H(inst, j, j);
+            }
+            __syncthreads();
+            const double a = *(volatile double *)(coef + j);
+            for (int i = threadIdx.x; i < j; i += KRYLOV_BLOCK) {
+                coef[i] -= *gb.H(inst, i, j) * a;
+            }
+            __syncthreads();
+        }
+    }
     if (threadIdx.x == 0) {
-        const int k = gb.ctl[GC_K];
-        if (kind == 0) {
-            *gb.H(i, gb.ctl[GC_I], k) = sum;
+        gb.arnoldi(inst) = !stop;
+        int going;
+        if (last_instance(gb, GC_IN_ARNOLDI, !stop, &going)) {
+            gb.ctl[GC_K] = k + 1;
+            cudaGraphSetConditional(h, (going > 0 && k + 1 < dim) ? 1u : 0u);
         }
-        else if (kind == 1) {
-            *gb.H(i, k + 1, k) = sqrt(sum);
-        }
-        else {
-            gb.s(i)[GS_VNORM] = sqrt(sum);
-        }
-    }
-}
-
-// next Gram-Schmidt row: i += 1; go on while i <= k
-__global__ void k_mgs_next(GmresBatch gb, cudaGraphConditionalHandle h)
-{
-    const int i = gb.ctl[GC_I] + 1;
-    gb.ctl[GC_I] = i;
-    cudaGraphSetConditional(h, (i <= gb.ctl[GC_K] && i < gb.dim) ? 1u : 0u);
-}
-
-// next Arnoldi column: k += 1; go on while some instance iterates (count[1], set by k_givens_at),
-// at most `dim` columns (k_givens_at already stops every instance there)
-__global__ void k_arnoldi_next(GmresBatch gb, cudaGraphConditionalHandle h)
-{
-    const int k = gb.ctl[GC_K] + 1;
-    gb.ctl[GC_K] = k;
-    cudaGraphSetConditional(h, (gb.count[1] > 0 && k < gb.dim) ? 1u : 0u);
-}
-
-// The matvec, Givens and normalisation steps of Arnoldi column k (k read from the device):
-// perturbed primitive state q1 = prim(U + eps V_k), eps = fd_scale / |V_k| (gmres.c:26-36)
-__global__ void k_perturb_at(int C, int N, const double *__restrict__ U, const double *__restrict__ V,
-                             GmresBatch gb, double gamma, double *__restrict__ q1)
-{
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C) {
-        return;
-    }
-    const int i = gb.cell_inst[c];
-    if (!gb.arnoldi(i)) {
-        return;
-    }
-    const double *v = V + (size_t)gb.ctl[GC_K] * 5 * (size_t)C;
-    const double eps = gb.s(i)[GS_FD_SCALE] / gb.s(i)[GS_VNORM];
-    Cons<double> u;
-    u.rho = U[c] + (eps * v[c]);
-    u.m.x = U[C + c] + (eps * v[C + c]);
-    u.m.y = U[2 * C + c] + (eps * v[2 * C + c]);
-    u.m.z = U[3 * C + c] + (eps * v[3 * C + c]);
-    u.e = U[4 * C + c] + (eps * v[4 * C + c]);
-    Prim<double> p = cons_to_prim(u, gamma);
-    q1[c] = p.rho;
-    q1[N + c] = p.u.x;
-    q1[2 * N + c] = p.u.y;
-    q1[3 * N + c] = p.u.z;
-    q1[4 * N + c] = p.p;
-}
-
-// w = V_k - step (R1 - R) / eps (gmres.c:41-46)
-__global__ void k_matvec_finish_at(int C, const double *__restrict__ V, const double *__restrict__ R1,
-                                   const double *__restrict__ R, GmresBatch gb, double *__restrict__ w)
-{
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C) {
-        return;
-    }
-    const int i = gb.cell_inst[c];
-    if (!gb.arnoldi(i)) {
-        return;
-    }
-    const double *v = V + (size_t)gb.ctl[GC_K] * 5 * (size_t)C;
-    const double *s = gb.s(i);
-    const double eps = s[GS_FD_SCALE] / s[GS_VNORM];
-    const double step = s[GS_STEP];
-#pragma unroll
-    for (int k = 0; k < 5; k++) {
-        size_t j = (size_t)k * C + c;
-        w[j] = v[j] - ((step * (R1[j] - R[j])) / eps);
-    }
-}
-
-// Givens rotations of column k, new rotation, right-hand side and convergence test per Arnoldi
-// instance (gmres.c:102-119); an instance that converged (or filled the basis) stops with m = k + 1;
-// count[1] = instances that go on
-__global__ void k_givens_at(GmresBatch gb)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int k = gb.ctl[GC_K];
-    if (i >= gb.ninst || !gb.arnoldi(i)) {
-        return;
-    }
-    double *cs = gb.cs(i), *sn = gb.sn(i), *rhs = gb.rhs(i);
-    for (int r = 0; r < k; r++) {
-        double hrk = *gb.H(i, r, k), hr1k = *gb.H(i, r + 1, k);
-        double tmp = (cs[r] * hrk) + (sn[r] * hr1k);
-        *gb.H(i, r + 1, k) = (-sn[r] * hrk) + (cs[r] * hr1k);
-        *gb.H(i, r, k) = tmp;
-    }
-    double hkk = *gb.H(i, k, k), hk1k = *gb.H(i, k + 1, k);
-    double rot = sqrt((hkk * hkk) + (hk1k * hk1k));
-    cs[k] = hkk / rot;
-    sn[k] = hk1k / rot;
-    *gb.H(i, k, k) = rot;
-    rhs[k + 1] = -sn[k] * rhs[k];
-    rhs[k] = cs[k] * rhs[k];
-    gb.m(i) = k + 1;
-    if (fabs(rhs[k + 1]) < gb.s(i)[GS_KTOL] || k + 1 >= gb.dim) {
-        gb.arnoldi(i) = 0;
-        return;
-    }
-    atomicAdd(&gb.count[1], 1);
-}
-
-// V_{k+1} = w / H[k+1][k] (gmres.c:121-125)
-__global__ void k_normalize_at(int C, const double *__restrict__ w, GmresBatch gb, double *__restrict__ V)
-{
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C) {
-        return;
-    }
-    const int i = gb.cell_inst[c];
-    if (!gb.arnoldi(i)) {
-        return;
-    }
-    const int k = gb.ctl[GC_K];
-    double *Vk1 = V + (size_t)(k + 1) * 5 * (size_t)C;
-    const double h = *gb.H(i, k + 1, k);
-#pragma unroll
-    for (int v = 0; v < 5; v++) {
-        size_t j = (size_t)v * C + c;
-        Vk1[j] = w[j] / h;
     }
 }
 
