@@ -1,11 +1,11 @@
 """Autotuner of the hot kernels' launch shapes.
 
 Builds the library once per candidate of (face-flux block size, face-flux blocks resident per SM,
-face geometry staged by bulk copies or loaded, cell-gather block size) into a scratch directory,
+cell-gather block size) into a scratch directory,
 times a fixed number of RK steps of a workload on the current GPU with each build (a fresh process
 per build, selected with TEAL_B200_LIBRARY), and writes the fastest shape to
-teal_b200/csrc/tuned.h (and to --out when given). Shapes and the Navier-Stokes staging switch are
-tuned on the Taylor-Green vortex, the Euler staging switch on the unstructured ramp.
+teal_b200/csrc/tuned.h (and to --out when given). Shapes are tuned on the Taylor-Green vortex, the
+Euler staging switch (face geometry staged by bulk copies or loaded) on the unstructured ramp.
 
     python -m teal_b200.autotune [--n 96] [--ramp-n 64] [--steps 10] [--precision fp64] [--out tuned_candidate.h]
 
@@ -26,12 +26,11 @@ CSRC = os.path.join(HERE, "csrc")
 ROOT = os.path.dirname(HERE)
 
 # face-flux block size x resident face threads per SM (65536 registers / threads = the cap per
-# thread: 512 -> 128, 640 -> 102, 768 -> 85) x geometry staged in shared memory by bulk copies or
-# loaded by the threads x cell-gather block size. The Navier-Stokes workload tunes the shapes and
-# its staging switch; the Euler staging switch is then tuned on the unstructured ramp with the
-# chosen shapes.
+# thread: 384 -> 168, 512 -> 128, 640 -> 102, 768 -> 85) x cell-gather block size. The Navier-Stokes
+# workload tunes the shapes; the Euler staging switch (face geometry staged in shared memory by bulk
+# copies or loaded by the threads) is then tuned on the unstructured ramp with the chosen shapes.
 FACE_BLOCKS = [32, 64, 128]
-FACE_THREADS = [512, 640, 768]
+FACE_THREADS = [384, 512, 640, 768]
 STAGED = [0, 1]
 CELL_BLOCKS = [256]
 # then cell-gather block size x blocks resident per SM (1536 threads -> 42 registers per thread)
@@ -109,8 +108,8 @@ def time_variant(lib, n, steps, precision, workload="tgv"):
 
 def write_header(path, best):
     lines = ["// Launch shapes of the hot kernels, chosen by teal_b200/autotune.py on a B200 (fastest measured",
-             "// RK step: TGV for the face, cell and gradient shapes and the Navier-Stokes staging switch, the",
-             "// ramp for the Euler staging switch; times within 0.5 % of the fastest count as ties, resolved to",
+             "// RK step: TGV for the face, cell and gradient shapes, the ramp for the Euler staging switch",
+             "// and the Euler face occupancy; times within 0.5 % of the fastest count as ties, resolved to",
              "// fewer resident face blocks, i.e. more registers per thread). A value given with -D at build",
              "// time wins.",
              "#pragma once", ""]
@@ -120,7 +119,6 @@ def write_header(path, best):
              "TG_FACE_MINB_FP32": "FP32-flux face-flux blocks kept resident per SM (caps registers per thread)",
              "TG_CELL_BLOCK": "threads per cell-gather block",
              "TG_CELL_MINB": "cell-gather blocks kept resident per SM (caps registers per thread)",
-             "TG_FACE_STAGED_NS": "Navier-Stokes face kernel: geometry staged by bulk copies (1) or loaded (0)",
              "TG_FACE_STAGED_EULER": "Euler face kernel: geometry staged by bulk copies (1) or loaded (0)",
              "TG_GRAD_MINB": "gradient blocks (160 threads) kept resident per SM (caps registers per thread)"}
     for k, v in best.items():
@@ -138,8 +136,8 @@ def main():
     ap.add_argument("--out", default=None, help="also write the chosen header here")
     ap.add_argument("--jobs", type=int, default=os.cpu_count() or 8)
     args = ap.parse_args()
-    variants = [{"TG_FACE_BLOCK": fb, "TG_FACE_MINB": ft // fb, "TG_CELL_BLOCK": cb, "TG_FACE_STAGED_NS": st}
-                for fb, ft, st, cb in itertools.product(FACE_BLOCKS, FACE_THREADS, STAGED, CELL_BLOCKS)]
+    variants = [{"TG_FACE_BLOCK": fb, "TG_FACE_MINB": ft // fb, "TG_CELL_BLOCK": cb}
+                for fb, ft, cb in itertools.product(FACE_BLOCKS, FACE_THREADS, CELL_BLOCKS)]
 
     def sweep(variants, workload, n, work, per):
         with concurrent.futures.ThreadPoolExecutor(max_workers=4) as pool:

@@ -1,6 +1,5 @@
 // Face-flux kernel: reconstruction, viscous and convective flux of one face per thread.
 #pragma once
-
 #include "common.cuh"
 #include "tma.cuh"
 
@@ -59,15 +58,14 @@ struct DirectGeo {
 // asynchronous copies (one per SoA row, all in flight at once, completing on one mbarrier) so the
 // streamed face geometry costs the threads neither registers nor load instructions; rows: area,
 // basis (9 in the exact form; the normal's 3 otherwise, see frame_of), offsets left / right
-// (3 + 3, second order), correction (4, Navier-Stokes).
-template <typename R, int ORDER, bool NS>
+// (3 + 3, second order).
+template <typename R, int ORDER>
 struct FaceTile {
     static constexpr int PAD = 16 / int(sizeof(R));
     static constexpr int SROW = FACE_BLOCK + PAD;
     static constexpr int NBASIS = kExact ? 9 : 3;
-    static constexpr int ROWS = 1 + NBASIS + (ORDER == 2 ? 6 + (NS ? 4 : 0) : 0);
+    static constexpr int ROWS = 1 + NBASIS + (ORDER == 2 ? 6 : 0);
     static constexpr int R_AREA = 0, R_BASIS = 1, R_OFFL = 1 + NBASIS, R_OFFR = R_OFFL + 3;
-    static constexpr int R_CORR = (ORDER == 2) ? R_OFFR + 3 : R_OFFL;
     R geo[ROWS][SROW];
     int2 lr[FACE_BLOCK + 2];
     uint64_t bar;
@@ -78,8 +76,7 @@ struct FaceTile {
         if (r == R_AREA) return g.area;
         if (r < R_BASIS + NBASIS) return g.basis + (size_t)(r - R_BASIS) * F;
         if (ORDER == 2 && r < R_OFFL + 3) return g.offl + (size_t)(r - R_OFFL) * F;
-        if (ORDER == 2 && r < R_OFFR + 3) return g.offr + (size_t)(r - R_OFFR) * F;
-        return g.corr + (size_t)(r - R_CORR) * F;
+        return g.offr + (size_t)(r - R_OFFR) * F;
     }
 
     // thread 0 issues the copies of faces [f0, f0 + n); every thread then waits (bounded).
@@ -133,51 +130,64 @@ struct FaceTile {
     __device__ __forceinline__ V3<R> offl(int i) const { return v3_at(R_OFFL, i); }
     __device__ __forceinline__ V3<R> offr(int i) const { return v3_at(R_OFFR, i); }
     __device__ __forceinline__ R area(int i) const { return at(R_AREA, i); }
-    __device__ __forceinline__ V3<R> corr(int i) const { return v3_at(R_CORR, i); }
-    __device__ __forceinline__ R corr_norm(int i) const { return at(R_CORR + 3, i); }
 };
 
-// Viscous flux of face f (element i of its tile): the face average of both cells' states and
-// unlimited gradients, corrected along the centre-to-centre direction, in the face normal's frame
-template <typename R, typename Geo>
+// The reconstructed states of a face's two sides while its viscous flux runs: in registers in FP64 (at 128 of
+// them, 16 blocks an SM), in shared memory in the FP32-flux form (at 64 registers, 32 blocks an SM; a
+// thread's own column, volatile so that the values do not stay in registers all the same)
+template <typename R>
+struct Sides {
+    R v[10];
+    __device__ __forceinline__ explicit Sides(R *) {}
+    __device__ __forceinline__ void set(int k, R x) { v[k] = x; }
+    __device__ __forceinline__ R get(int k) const { return v[k]; }
+};
+template <>
+struct Sides<float> {
+    volatile float *p;
+    __device__ __forceinline__ explicit Sides(float *column) : p(column) {}
+    __device__ __forceinline__ void set(int k, float x) { p[k * FACE_BLOCK] = x; }
+    __device__ __forceinline__ float get(int k) const { return p[k * FACE_BLOCK]; }
+};
+
+// Viscous flux of face f (element i of its tile) and the reconstructed states pl, pr of its sides, from
+// one pass over both cells' states and gradient records: the face average of the states and unlimited
+// gradients, corrected along the centre-to-centre direction (derivative.c:71-89), in the face normal's frame.
+template <typename R, bool FOLD, typename Geo>
 __device__ __forceinline__ Cons<R> viscous_face(const Geo &geo, int i, bool boundary, int2 c, int N,
-                                                const double *__restrict__ q, const R *__restrict__ rec, R gamma,
-                                                R mu, R prandtl)
+                                                const double *__restrict__ q, const R *__restrict__ rec, double pref,
+                                                R gamma, R mu, R prandtl, Sides<R> &sides)
 {
-    // face average corrected along the centre-to-centre direction (derivative.c:71-89)
-    Prim<R> ql = reload_prim<R>(q, N, c.x);
-    Prim<R> qr = reload_prim<R>(q, N, c.y);
-    R qlv[5] = {ql.rho, ql.u.x, ql.u.y, ql.u.z, ql.p};
-    R qrv[5] = {qr.rho, qr.u.x, qr.u.y, qr.u.z, qr.p};
     R qm[5], gm[15];
-#pragma unroll
-    for (int v = 0; v < 5; v++) {
-        qm[v] = (qlv[v] + qrv[v]) / R(2);
-    }
-#pragma unroll
-    for (int v = 0; v < 5; v++) {
-        R ax, ay, az, ap, bx, by, bz, bp;
-        grad_rec_load(rec, c.x, v, ax, ay, az, ap);
-        if (boundary) {
-            gm[3 * v] = ax, gm[3 * v + 1] = ay, gm[3 * v + 2] = az;
-        }
-        else {
-            grad_rec_load(rec, c.y, v, bx, by, bz, bp);
-            gm[3 * v] = (ax + bx) / R(2), gm[3 * v + 1] = (ay + by) / R(2), gm[3 * v + 2] = (az + bz) / R(2);
-        }
-    }
-    V3<R> unit = geo.corr(i);
+    const V3<R> unit = geo.corr(i), offl = geo.offl(i), offr = geo.offr(i);
     const R cnorm = geo.corr_norm(i);
     const R inv_norm = R(1) / cnorm;
 #pragma unroll
     for (int v = 0; v < 5; v++) {
-        V3<R> gv = v3(gm[3 * v], gm[3 * v + 1], gm[3 * v + 2]);
-        const R dq = qrv[v] - qlv[v];
-        R adjust = dot(gv, unit) - (kExact ? (dq / cnorm) : (dq * inv_norm));
-        gv = sub(gv, mul(adjust, unit));
-        gm[3 * v] = gv.x;
-        gm[3 * v + 1] = gv.y;
-        gm[3 * v + 2] = gv.z;
+        const double ql = __ldg(q + (size_t)v * N + c.x), qr = __ldg(q + (size_t)v * N + c.y);
+        R ax, ay, az, ap;
+        grad_rec_load(rec, c.x, v, ax, ay, az, ap);
+        // FP32 fluxes reconstruct the pressure relative to the instance's reference (Local::dp); the
+        // difference is taken in FP64, before the rounding to FP32
+        const double p0 = (v == 4 && sizeof(R) == sizeof(float)) ? pref : 0.0;
+        V3<R> ga = v3(ax, ay, az);
+        sides.set(v, R(ql - p0) + dot(FOLD ? ga : v3(ax * ap, ay * ap, az * ap), offl));
+        if (boundary) {  // the ghost state enters unreconstructed (derivative.c:203-211)
+            sides.set(5 + v, R(qr - p0));
+        }
+        else {
+            R bx, by, bz, bp;
+            grad_rec_load(rec, c.y, v, bx, by, bz, bp);
+            sides.set(5 + v, R(qr - p0) + dot(FOLD ? v3(bx, by, bz) : v3(bx * bp, by * bp, bz * bp), offr));
+            ga = v3((ax + bx) / R(2), (ay + by) / R(2), (az + bz) / R(2));
+        }
+        qm[v] = (R(ql) + R(qr)) / R(2);
+        const R dq = R(qr) - R(ql);
+        const R adjust = dot(ga, unit) - (kExact ? (dq / cnorm) : (dq * inv_norm));
+        ga = sub(ga, mul(adjust, unit));
+        gm[3 * v] = ga.x;
+        gm[3 * v + 1] = ga.y;
+        gm[3 * v + 2] = ga.z;
     }
     Grad<R> gg;
     gg.rho = v3(gm[0], gm[1], gm[2]);
@@ -193,16 +203,76 @@ __device__ __forceinline__ Cons<R> viscous_face(const Geo &geo, int i, bool boun
     return viscous_central(prim_from(qm), gg, gamma, mu, prandtl, nb);
 }
 
-// The flux record of face f (element i of its tile). The convective flux comes first (its
-// reconstruction streams the limited gradients), the viscous flux second (its face-averaged
-// gradient re-reads the unlimited gradients, which are still in L1).
+// Flux record of a face with a viscous flux. Its bound is the L1 data pipe and the latency of the gathers
+// (66 % of peak LSU wavefronts, 25 % L1 hits with one pass for either flux), so both cells' states and
+// gradient records are read once: the pass gives the viscous flux and the reconstructed states, then the
+// convective flux follows. `column`: this thread's shared-memory column (FP32-flux form). Measured
+// against two passes at 96 / 64 registers, TGV 128^3: FP64 0.467 -> 0.421 ms (0.464 at 96 registers with
+// the states in shared memory, 0.438 at 80), FP32-flux 0.301 -> 0.267 ms (0.275-0.298 at fewer
+// resident blocks).
+template <typename R, int FK, bool FOLD, typename Geo>
+__device__ __forceinline__ void face_flux_ns(const Geo &geo, int i, int f, const Sizes &s,
+                                             const double *__restrict__ q, const R *__restrict__ rec, R gamma, R mu,
+                                             R prandtl, R *__restrict__ G, const PressureRefOf<R> &pr_ref,
+                                             R *column)
+{
+    const bool boundary = (f >= s.F_in) && (f < s.F_bd);
+    const int2 c = geo.cells(i);
+    double pref = 0.0;
+    if constexpr (sizeof(R) == sizeof(float)) {
+        pref = pr_ref.of(c.x);
+    }
+    Sides<R> sides(column);
+    const Cons<R> fv = viscous_face<R, FOLD>(geo, i, boundary, c, s.N, q, rec, pref, gamma, mu, prandtl, sides);
+    R pl[5], pr[5];
+#pragma unroll
+    for (int v = 0; v < 5; v++) {
+        pl[v] = sides.get(v);
+        pr[v] = sides.get(5 + v);
+    }
+    Cons<R> fc{R(0), v3(R(0), R(0), R(0)), R(0)};
+    if (FK != FK_NONE) {
+        Basis<R> b;
+        if constexpr (kExact) {
+            b = geo.basis_again(i);
+        }
+        else {
+            b = frame_of(geo.normal_again(i));
+        }
+        const Local<R> l = make_local(prim_from(pl), gamma, b, R(pref));
+        const Local<R> r = make_local(prim_from(pr), gamma, b, R(pref));
+        fc = convective_flux_local<FK>(l, r, gamma);
+        if constexpr (kExact) {
+            fc.m = to_global(geo.basis_again(i), fc.m);
+        }
+        else {
+            fc.m = to_global(frame_of(geo.normal_again(i)), fc.m);
+        }
+    }
+    const R area = geo.area(i);
+    R gf[5] = {fc.rho * area, fc.m.x * area, fc.m.y * area, fc.m.z * area, fc.e * area};
+    if constexpr (kExact) {
+        const R gv[5] = {fv.rho * area, fv.m.x * area, fv.m.y * area, fv.m.z * area, fv.e * area};
+        flux_rec_store(G + flux_rec2_offset(s.F), s.F, f, gv);
+    }
+    else {
+        gf[0] -= fv.rho * area;
+        gf[1] -= fv.m.x * area;
+        gf[2] -= fv.m.y * area;
+        gf[3] -= fv.m.z * area;
+        gf[4] -= fv.e * area;
+    }
+    flux_rec_store(G, s.F, f, gf);
+}
+
+// The flux record of face f (element i of its tile) without a viscous flux.
 // Records: G[f] = (convective - viscous) * area; in the exact translation units with a viscous
 // flux, G[f] = convective * area and G[flux_rec2_offset(F) + f] = viscous * area instead, because teal adds all of a
 // cell's viscous terms before its convective ones (derivative.c:279-292) and the cell gather must
 // repeat that order.
-template <typename R, int FK, bool NS, int ORDER, bool FOLD, typename Geo>
+template <typename R, int FK, int ORDER, bool FOLD, typename Geo>
 __device__ __forceinline__ void face_flux(const Geo &geo, int i, int f, const Sizes &s, const double *__restrict__ q,
-                                          const R *__restrict__ rec, R gamma, R mu, R prandtl, R *__restrict__ G,
+                                          const R *__restrict__ rec, R gamma, R *__restrict__ G,
                                           const PressureRefOf<R> &pr_ref)
 {
     const int N = s.N;
@@ -266,20 +336,6 @@ __device__ __forceinline__ void face_flux(const Geo &geo, int i, int f, const Si
     R area = geo.area(i);
     R gf[5] = {fc.rho * area, fc.m.x * area, fc.m.y * area, fc.m.z * area, fc.e * area};
 
-    if (NS && ORDER == 2) {
-        const Cons<R> fv = viscous_face<R>(geo, i, boundary, c, N, q, rec, gamma, mu, prandtl);
-        if constexpr (kExact) {
-            const R gv[5] = {fv.rho * area, fv.m.x * area, fv.m.y * area, fv.m.z * area, fv.e * area};
-            flux_rec_store(G + flux_rec2_offset(s.F), s.F, f, gv);
-        }
-        else {
-            gf[0] -= fv.rho * area;
-            gf[1] -= fv.m.x * area;
-            gf[2] -= fv.m.y * area;
-            gf[3] -= fv.m.z * area;
-            gf[4] -= fv.e * area;
-        }
-    }
     flux_rec_store(G, s.F, f, gf);
 }
 
@@ -297,28 +353,36 @@ __global__ void __launch_bounds__(FACE_BLOCK, face_minb<R>(NS)) k_face(Sizes s, 
         return;
     }
     DirectGeo<R> geo{g, s.F, f};
-    face_flux<R, FK, NS, ORDER, FOLD>(geo, 0, f, s, q, rec, gamma, mu, prandtl, G, pr_ref);
+    if constexpr (NS && ORDER == 2) {
+        __shared__ R aside[sizeof(R) == sizeof(float) ? 10 * FACE_BLOCK : 1];
+        face_flux_ns<R, FK, FOLD>(geo, 0, f, s, q, rec, gamma, mu, prandtl, G, pr_ref,
+                                  aside + (sizeof(R) == sizeof(float) ? threadIdx.x : 0));
+    }
+    else {
+        face_flux<R, FK, ORDER, FOLD>(geo, 0, f, s, q, rec, gamma, G, pr_ref);
+    }
 }
 
 // One tile of FACE_BLOCK faces per block, its geometry staged in shared memory by bulk copies
-// before the threads (one face each) start. A wait that gives up sets ERR_TIMEOUT in the error
+// before the threads (one face each) start (no viscous flux: its register budget leaves too few blocks
+// resident to hide the copies). A wait that gives up sets ERR_TIMEOUT in the error
 // word and ends the block.
-template <typename R, int FK, bool NS, int ORDER, bool FOLD, bool X>
-__global__ void __launch_bounds__(FACE_BLOCK, face_minb<R>(NS)) k_face_staged(Sizes s, Geometry<R> g,
+template <typename R, int FK, int ORDER, bool FOLD, bool X>
+__global__ void __launch_bounds__(FACE_BLOCK, face_minb<R>(false)) k_face_staged(Sizes s, Geometry<R> g,
                                                           const double *__restrict__ q,
-                                                          const R *__restrict__ rec, R gamma, R mu,
-                                                          R prandtl, R *__restrict__ G, int *err,
+                                                          const R *__restrict__ rec, R gamma,
+                                                          R *__restrict__ G, int *err,
                                                           PressureRefOf<R> pr_ref, int polls)
 {
     static_assert(X == kExact, "exact kernels live in the exact translation units only");
-    __shared__ __align__(16) FaceTile<R, ORDER, NS> t;
+    __shared__ __align__(16) FaceTile<R, ORDER> t;
     const int f0 = s.lo + blockIdx.x * FACE_BLOCK;
     const int n = min(FACE_BLOCK, s.hi - f0);
     if (!t.stage(g, s.F, f0, n, err, polls)) {
         return;
     }
     if (threadIdx.x < n) {
-        face_flux<R, FK, NS, ORDER, FOLD>(t, threadIdx.x, f0 + threadIdx.x, s, q, rec, gamma, mu, prandtl, G,
+        face_flux<R, FK, ORDER, FOLD>(t, threadIdx.x, f0 + threadIdx.x, s, q, rec, gamma, G,
                                           pr_ref);
     }
 }

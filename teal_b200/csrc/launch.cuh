@@ -38,23 +38,24 @@ inline void launch_face_v(bool staged, const FaceLaunch &a, const Geometry<R> &g
     if constexpr (sizeof(R) == sizeof(float)) {
         pref = a.pr_ref;
     }
-    if (staged) {
-        k_face_staged<R, FK, NS, ORDER, FOLD, X>
-            <<<grid, FACE_BLOCK, 0, st>>>(a.s, g, a.q, rec, gm, mu, pr, G, a.err, pref, a.polls);
+    if constexpr (!NS) {
+        if (staged) {
+            k_face_staged<R, FK, ORDER, FOLD, X>
+                <<<grid, FACE_BLOCK, 0, st>>>(a.s, g, a.q, rec, gm, G, a.err, pref, a.polls);
+            return;
+        }
     }
-    else {
-        k_face<R, FK, NS, ORDER, FOLD, X><<<grid, FACE_BLOCK, 0, st>>>(a.s, g, a.q, rec, gm, mu, pr, G, pref);
-    }
+    k_face<R, FK, NS, ORDER, FOLD, X><<<grid, FACE_BLOCK, 0, st>>>(a.s, g, a.q, rec, gm, mu, pr, G, pref);
 }
 
-// staged geometry (bulk copies into shared memory) or thread loads, per physics (tuned.h)
+// staged geometry (bulk copies into shared memory) or thread loads without a viscous flux (tuned.h)
 template <int FK, typename R>
 inline cudaError_t launch_face_r(bool ns, int order, bool fold, const FaceLaunch &a, cudaStream_t st)
 {
     const Geometry<R> &g = *static_cast<const Geometry<R> *>(a.geom);
     const R *rec = static_cast<const R *>(a.rec);
     R *G = static_cast<R *>(a.G);
-    const bool staged = ns ? (TG_FACE_STAGED_NS != 0) : (TG_FACE_STAGED_EULER != 0);
+    const bool staged = !ns && TG_FACE_STAGED_EULER != 0;
     if (order == 1) {
         launch_face_v<R, FK, false, 1, true>(staged, a, g, rec, G, st);
     }
