@@ -295,6 +295,55 @@ __global__ void k_slot_finish(int C, int SL, const int2 *__restrict__ lr, const 
     }
 }
 
+// side records of each face's cells (side_index), from the cells' slots
+__global__ void k_face_slots(int C, int SL, const int *__restrict__ slot_face, const uint8_t *__restrict__ slot_cnt,
+                             int2 *__restrict__ sides)
+{
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= C) {
+        return;
+    }
+    for (int j = 0; j < slot_cnt[c]; j++) {
+        const int sf = slot_face[(size_t)j * SL + c];
+        if (sf >= 0) {
+            sides[sf].x = side_index(c, j);
+        }
+        else {
+            sides[~sf].y = side_index(c, j);
+        }
+    }
+}
+
+// faces between a cell and a state row (boundary ghosts, owners of periodic ghosts, other ranks' cells), and
+// the cells that own periodic ghosts
+__global__ void k_face_rows(int F, int F_in, int F_bd, int C, const int2 *__restrict__ lr, int2 *__restrict__ sides,
+                            unsigned *__restrict__ records)
+{
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= F) {
+        return;
+    }
+    const int2 c = lr[f];
+    if (c.x >= C) {
+        sides[f].x = ~c.x;
+    }
+    if (f >= F_in || c.y >= C) {
+        sides[f].y = ~c.y;
+    }
+    if (f >= F_bd && c.y < C) {
+        atomicOr(records + (c.y >> 5), 1u << (c.y & 31));
+    }
+}
+
+// the cells a partition sends
+__global__ void k_mark_rows(int n, const int *__restrict__ rows, unsigned *__restrict__ records)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) {
+        atomicOr(records + (rows[i] >> 5), 1u << (rows[i] & 31));
+    }
+}
+
 // Gradient tiles (grad_tile_bytes) from the pitched slot arrays: block t fills tile t, lane l the
 // column of cell 32 t + l; columns past the last cell hold zeros (their threads never read them)
 template <typename G>

@@ -25,9 +25,16 @@ __host__ __device__ constexpr int face_minb(bool ns)
 {
     return sizeof(R) == sizeof(float) ? FACE_MINB_FP32 : ns ? FACE_MINB : FACE_MINB_EULER;
 }
+constexpr int SIDE_BLOCK = TG_SIDE_BLOCK;
+template <typename R>
+__host__ __device__ constexpr int side_minb()
+{
+    return sizeof(R) == sizeof(float) ? TG_SIDE_MINB_FP32 : TG_SIDE_MINB;
+}
 constexpr int CELL_BLOCK = TG_CELL_BLOCK;
 constexpr int CELL_MINB = TG_CELL_MINB;
 constexpr int GRAD_MINB = TG_GRAD_MINB;
+constexpr int GRAD_MINB_SIDES = TG_GRAD_MINB_SIDES;
 constexpr int REDUCE_BLOCK = 1024;
 
 // ---- small helpers ---------------------------------------------------------------------------
@@ -191,6 +198,34 @@ __device__ __forceinline__ void grad_rec_load(const float *rec, int c, int v, fl
     const float2 *p = reinterpret_cast<const float2 *>(rec + ((size_t)c * 5 + v) * 4);
     const float2 a = __ldg(p), b = __ldg(p + 1);
     gx = a.x, gy = a.y, gz = b.x, psi = b.y;
+}
+
+// Side records: the reconstructed state of every (cell, slot), as arrays [5][E]. Slot j of cell c is element
+// side_index(c, j): tiles of 32 cells as in the gradient kernel, so that each of its warps stores whole
+// rows of its variable. (Records of four values and one, loaded as 256 + 64 bits, made the face kernel
+// 5 % faster, ramp of 513 k cells 43.4 against 45.3 us, and the gradient kernel, which had to bring a
+// record's values together in shared memory, 9 % slower, 73.4 against 67.6 us.)
+constexpr int SIDE_TILE = MAX_SLOTS * 32;
+__host__ __device__ constexpr int side_index(int c, int j)
+{
+    return (c >> 5) * SIDE_TILE + j * 32 + (c & 31);
+}
+__host__ __device__ constexpr int side_cell(int e)
+{
+    return (e / SIDE_TILE) * 32 + (e & 31);
+}
+// elements of a row for C cells; SL is C rounded up to 4
+__host__ __device__ constexpr size_t side_elements(int SL)
+{
+    return (size_t)((SL + 31) / 32) * SIDE_TILE;
+}
+template <typename R>
+__device__ __forceinline__ void side_load(const R *side, int SL, int e, R (&v)[5])
+{
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+        v[k] = __ldg(side + (size_t)k * side_elements(SL) + e);
+    }
 }
 
 // Per-face flux records, 5 values per face without padding: components 0-3 as [F][4] (one 256-bit

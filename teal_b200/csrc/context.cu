@@ -229,6 +229,9 @@ struct tg_ctx {
 
     // device mesh
     int2 *lr = nullptr;
+    int2 *sides = nullptr;     // side records of each face (contexts that use them, use_sides)
+    unsigned *side_records = nullptr;  // cells whose gradient records are read too, a bit each per gradient tile
+    void *side_rec = nullptr;        // the side records
     int *slot_nbr = nullptr, *slot_face = nullptr;
     uint8_t *slot_cnt = nullptr;
     bool full_slots = true;    // every inner cell has MAX_SLOTS faces
@@ -370,7 +373,7 @@ static void free_ctx(tg_ctx *c)
         if (s) cudaStreamDestroy(s);
     }
     void *ptrs[] = {c->bcenter, c->ccenter, c->S, c->dprop, c->pref,
-                    c->lr, c->slot_nbr, c->slot_face, c->slot_cnt, c->owner, c->bface_ent, c->bkind, c->bctx,
+                    c->lr, c->sides, c->side_records, c->side_rec, c->slot_nbr, c->slot_face, c->slot_cnt, c->owner, c->bface_ent, c->bkind, c->bctx,
                     c->volume, c->proj, c->eps2, c->gb.area, c->gb.basis, c->gb.offl, c->gb.offr, c->gb.corr,
                     c->gb.slot_w, c->gb.slot_off, c->gb.area32, c->gb.basis32, c->gb.offl32, c->gb.offr32,
                     c->gb.corr32, c->gb.tile64, c->gb.tile32, c->gb.toff64, c->gb.toff32, c->q, c->U0, c->R, c->qs, c->grad, c->G,
@@ -909,6 +912,23 @@ static int create_ctx(MeshInput &in, const tg_equations *e, int precision, tg_ct
                 c->gb.slot_w = c->gb.slot_off = nullptr;
             }
 
+            // side records of each face, where the residuals use them (use_sides)
+            if (e->space_order == 2 && e->viscous != TG_VISCOUS_CENTRAL && precision != TG_PRECISION_FP64_EXACT) {
+                TRY(dalloc(&c->sides, s.F));
+                k_face_slots<<<grid_of(s.C), BLOCK, 0, st>>>(s.C, s.SL, c->slot_face, c->slot_cnt, c->sides);
+                if (s.F > s.F_bd || !in.send_rows.empty()) {
+                    const size_t ntiles = (s.C + GRAD_CELLS - 1) / GRAD_CELLS;
+                    TRY(dalloc(&c->side_records, ntiles));
+                    CU(cudaMemsetAsync(c->side_records, 0, sizeof(unsigned) * ntiles, st));
+                }
+                k_face_rows<<<grid_of(s.F), BLOCK, 0, st>>>(s.F, s.F_in, s.F_bd, s.C, c->lr, c->sides, c->side_records);
+                CU(cudaGetLastError());
+                // FP64 size in every form, as the gradient records
+                double *rec = nullptr;
+                TRY(dalloc(&rec, 5 * side_elements(s.SL)));
+                c->side_rec = rec;
+            }
+
             // face geometry, structure of arrays
             TRY(upload(&c->gb.area, m->face_area, s.F, st));
             TRY(dalloc(&d_tmp, 9 * (size_t)s.F > 3 * (size_t)s.C ? 9 * (size_t)s.F : 3 * (size_t)s.C));
@@ -956,9 +976,9 @@ static int create_ctx(MeshInput &in, const tg_equations *e, int precision, tg_ct
             TRY(to_float(c->gb.offr, c->gb.offr32, 3 * (size_t)s.F, st));
             TRY(to_float(c->gb.corr, c->gb.corr32, 4 * (size_t)s.F, st));
         }
-        c->g64 = Geometry<double>{c->lr,       c->gb.area,  c->gb.basis,   c->gb.offl,   c->gb.offr,   c->gb.corr,
+        c->g64 = Geometry<double>{c->lr,       c->sides,    c->gb.area,  c->gb.basis,   c->gb.offl,   c->gb.offr,   c->gb.corr,
                                   c->slot_nbr, c->slot_face, c->slot_cnt, c->gb.tile64, c->gb.toff64};
-        c->g32 = Geometry<float>{c->lr,         c->gb.area32, c->gb.basis32, c->gb.offl32,   c->gb.offr32,
+        c->g32 = Geometry<float>{c->lr,         c->sides,     c->gb.area32, c->gb.basis32, c->gb.offl32,   c->gb.offr32,
                                  c->gb.corr32, c->slot_nbr,  c->slot_face,  c->slot_cnt, c->gb.tile32,
                                  c->gb.toff32};
 
@@ -979,6 +999,10 @@ static int create_ctx(MeshInput &in, const tg_equations *e, int precision, tg_ct
             c->halo = in.halo;
             c->nsend = (int)in.send_rows.size();
             TRY(upload(&c->send_rows, in.send_rows.data(), in.send_rows.size(), st));
+            if (c->sides && c->nsend > 0) {
+                k_mark_rows<<<grid_of(c->nsend), BLOCK, 0, st>>>(c->nsend, c->send_rows, c->side_records);
+                CU(cudaGetLastError());
+            }
             TRY(dalloc(&c->send_q, 5 * (size_t)c->nsend));
             TRY(dalloc(&c->recv_q, 5 * (size_t)c->halo));
             CU(cudaMalloc(&c->send_rec, 20 * rsz * (size_t)(c->nsend > 0 ? c->nsend : 1)));
@@ -1449,42 +1473,69 @@ static Sizes face_sizes(const tg_ctx *c)
     return s;
 }
 
+// residuals whose face kernel reads the reconstructed states of the cells' sides instead of gradient
+// records: second order without a viscous flux (which needs the unlimited gradients), and not the
+// exact form
+static bool use_sides(const tg_ctx *c)
+{
+    return c->order == 2 && c->viscous != TG_VISCOUS_CENTRAL && !is_exact(c) && c->sides;
+}
+
+static PressureRef pressure_ref(const tg_ctx *c)
+{
+    return PressureRef{c->precision == TG_PRECISION_FP32_FLUX ? c->pref : nullptr, c->cell_inst};
+}
+
 template <typename R, bool MIXED>
-static void launch_gradient_s(tg_ctx *c, const Geometry<R> &g, bool fold, const double *q)
+static void launch_gradient_s(tg_ctx *c, const Geometry<R> &g, bool fold, bool sides, const double *q)
 {
     const Sizes s = cell_sizes(c);
     if (s.hi <= s.lo) return;
     dim3 grid((s.hi - s.lo + GRAD_CELLS - 1) / GRAD_CELLS);
     R *rec = (R *)c->grad;
+    PressureRefOf<R> pref{};
+    if constexpr (sizeof(R) == sizeof(float)) pref = pressure_ref(c);
+    auto launch = [&](auto kernel) {
+        kernel<<<grid, GRAD_THREADS, 0, c->stream>>>(s, g, c->eps2, q, rec, c->st.error, c->wait_polls, pref,
+                                                   SideOut<R>{(R *)c->side_rec, c->side_records});
+    };
     switch (c->limiter) {
         case TG_LIMITER_NONE:
-            k_gradient<R, 0, true, MIXED, false><<<grid, GRAD_THREADS, 0, c->stream>>>(s, g, c->eps2, q, rec, c->st.error, c->wait_polls);
+            if (sides)
+                launch(k_gradient<R, 0, true, MIXED, false, true>);
+            else
+                launch(k_gradient<R, 0, true, MIXED, false>);
             break;
         case TG_LIMITER_BARTH_JESPERSEN:
-            if (fold)
-                k_gradient<R, 1, true, MIXED, false><<<grid, GRAD_THREADS, 0, c->stream>>>(s, g, c->eps2, q, rec, c->st.error, c->wait_polls);
+            if (sides)
+                launch(k_gradient<R, 1, true, MIXED, false, true>);
+            else if (fold)
+                launch(k_gradient<R, 1, true, MIXED, false>);
             else
-                k_gradient<R, 1, false, MIXED, false><<<grid, GRAD_THREADS, 0, c->stream>>>(s, g, c->eps2, q, rec, c->st.error, c->wait_polls);
+                launch(k_gradient<R, 1, false, MIXED, false>);
             break;
         default:
-            if (fold)
-                k_gradient<R, 2, true, MIXED, false><<<grid, GRAD_THREADS, 0, c->stream>>>(s, g, c->eps2, q, rec, c->st.error, c->wait_polls);
+            if (sides)
+                launch(k_gradient<R, 2, true, MIXED, false, true>);
+            else if (fold)
+                launch(k_gradient<R, 2, true, MIXED, false>);
             else
-                k_gradient<R, 2, false, MIXED, false><<<grid, GRAD_THREADS, 0, c->stream>>>(s, g, c->eps2, q, rec, c->st.error, c->wait_polls);
+                launch(k_gradient<R, 2, false, MIXED, false>);
             break;
     }
 }
 
 template <typename R>
-static void launch_gradient(tg_ctx *c, const Geometry<R> &g, bool fold, const double *q)
+static void launch_gradient(tg_ctx *c, const Geometry<R> &g, bool fold, bool sides, const double *q)
 {
     if (c->full_slots)
-        launch_gradient_s<R, false>(c, g, fold, q);
+        launch_gradient_s<R, false>(c, g, fold, sides, q);
     else
-        launch_gradient_s<R, true>(c, g, fold, q);
+        launch_gradient_s<R, true>(c, g, fold, sides, q);
 }
 
-// gradient with an explicit limiter choice (tg_gradient reports the unlimited one on request)
+// gradient with an explicit limiter choice (tg_gradient reports the unlimited one on request, always
+// as gradient records)
 static int run_gradient(tg_ctx *c, const double *q, int limiter_override = -1)
 {
     int saved = c->limiter;
@@ -1499,10 +1550,11 @@ static int run_gradient(tg_ctx *c, const double *q, int limiter_override = -1)
         CU(e);
         return TG_OK;
     }
+    const bool sides = limiter_override < 0 && use_sides(c);
     if (c->precision == TG_PRECISION_FP64)
-        launch_gradient<double>(c, c->g64, fold, q);
+        launch_gradient<double>(c, c->g64, fold, sides, q);
     else
-        launch_gradient<float>(c, c->g32, fold, q);
+        launch_gradient<float>(c, c->g32, fold, sides, q);
     c->limiter = saved;
     CU(cudaGetLastError());
     return TG_OK;
@@ -1520,7 +1572,8 @@ static int run_face(tg_ctx *c, const double *q)
     a.prandtl = c->prop[2];
     a.G = c->G;
     a.err = c->st.error;
-    a.pr_ref = PressureRef{c->precision == TG_PRECISION_FP32_FLUX ? c->pref : nullptr, c->cell_inst};
+    a.pr_ref = pressure_ref(c);
+    a.side = use_sides(c) ? c->side_rec : nullptr;
     a.polls = c->wait_polls;
     bool ns = c->viscous == TG_VISCOUS_CENTRAL;
     bool fold = fold_psi(c);

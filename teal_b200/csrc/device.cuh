@@ -23,6 +23,8 @@ constexpr int MAX_SLOTS = 6;  // teal's MAX_CELL_FACES (src/mesh.h:7-11)
 template <typename G>
 struct Geometry {
     const int2 *lr;       // [F] left, right (right redirected to the owner for periodic faces)
+    const int2 *sides;    // [F] side records (side_index) of the left and right cell, or ~row for a state row:
+                          // a boundary ghost, a periodic ghost's owner, another rank's cell
     const G *area;        // [F]
     const G *basis;       // [9][F] rows x, y, z
     const G *offl;        // [3][F] face centre - left centre

@@ -26,7 +26,7 @@ __device__ __forceinline__ void reconstruct(const Prim<R> &q, const R *__restric
         if (!FOLD) {
             gv = v3(gv.x * ps, gv.y * ps, gv.z * ps);
         }
-        out[v] = qv[v] + dot(gv, off);
+        out[v] = at_face(qv[v], gv, off);
     }
 }
 
@@ -171,14 +171,14 @@ __device__ __forceinline__ Cons<R> viscous_face(const Geo &geo, int i, bool boun
         // difference is taken in FP64, before the rounding to FP32
         const double p0 = (v == 4 && sizeof(R) == sizeof(float)) ? pref : 0.0;
         V3<R> ga = v3(ax, ay, az);
-        sides.set(v, R(ql - p0) + dot(FOLD ? ga : v3(ax * ap, ay * ap, az * ap), offl));
+        sides.set(v, at_face(R(ql - p0), FOLD ? ga : v3(ax * ap, ay * ap, az * ap), offl));
         if (boundary) {  // the ghost state enters unreconstructed (derivative.c:203-211)
             sides.set(5 + v, R(qr - p0));
         }
         else {
             R bx, by, bz, bp;
             grad_rec_load(rec, c.y, v, bx, by, bz, bp);
-            sides.set(5 + v, R(qr - p0) + dot(FOLD ? v3(bx, by, bz) : v3(bx * bp, by * bp, bz * bp), offr));
+            sides.set(5 + v, at_face(R(qr - p0), FOLD ? v3(bx, by, bz) : v3(bx * bp, by * bp, bz * bp), offr));
             ga = v3((ax + bx) / R(2), (ay + by) / R(2), (az + bz) / R(2));
         }
         qm[v] = (R(ql) + R(qr)) / R(2);
@@ -336,6 +336,62 @@ __device__ __forceinline__ void face_flux(const Geo &geo, int i, int f, const Si
     R area = geo.area(i);
     R gf[5] = {fc.rho * area, fc.m.x * area, fc.m.y * area, fc.m.z * area, fc.e * area};
 
+    flux_rec_store(G, s.F, f, gf);
+}
+
+// Flux record of a face between two side records (k_gradient SIDES): the reconstructed states are read,
+// not formed, so a face costs two records, its normal and its area, and no gather of states or gradients.
+template <typename R, int FK>
+__global__ void __launch_bounds__(SIDE_BLOCK, side_minb<R>()) k_face_sides(Sizes s, Geometry<R> g,
+                                                   const double *__restrict__ q, const R *__restrict__ side,
+                                                   const R *__restrict__ rec, R gamma, R *__restrict__ G,
+                                                   PressureRefOf<R> pr_ref)
+{
+    static_assert(sizeof(R) == 0 || !kExact, "the exact form has no side records");
+    const int f = s.lo + blockIdx.x * SIDE_BLOCK + threadIdx.x;
+    if (f >= s.hi) {
+        return;
+    }
+    const int2 e = __ldg(g.sides + f);
+    const V3<R> n = load_v3(g.basis, s.F, f);
+    const R area = __ldg(g.area + f);
+    double pref = 0.0;
+    R pl[5], pr[5];
+    if constexpr (sizeof(R) == sizeof(float)) {
+        pref = pr_ref.of(side_cell(e.x >= 0 ? e.x : e.y));
+    }
+    auto row_state = [&](int row) {
+        if constexpr (sizeof(R) == sizeof(float)) {
+            return load_prim_rel<R>(q, s.N, row, pref);
+        }
+        else {
+            return load_prim<R>(q, s.N, row);
+        }
+    };
+    if (e.x >= 0) {
+        side_load(side, s.SL, e.x, pl);
+    }
+    else {
+        reconstruct<R, true>(row_state(~e.x), rec, ~e.x, load_v3(g.offl, s.F, f), pl);
+    }
+    if (e.y >= 0) {
+        side_load(side, s.SL, e.y, pr);
+    }
+    else if (f >= s.F_in && f < s.F_bd) {  // the ghost state enters unreconstructed (derivative.c:203-211)
+        const Prim<R> qr = row_state(~e.y);
+        pr[0] = qr.rho, pr[1] = qr.u.x, pr[2] = qr.u.y, pr[3] = qr.u.z, pr[4] = qr.p;
+    }
+    else {
+        reconstruct<R, true>(row_state(~e.y), rec, ~e.y, load_v3(g.offr, s.F, f), pr);
+    }
+    const Basis<R> b = frame_of(n);
+    Cons<R> fc{R(0), v3(R(0), R(0), R(0)), R(0)};
+    if (FK != FK_NONE) {
+        fc = convective_flux_local<FK>(make_local(prim_from(pl), gamma, b, R(pref)),
+                                       make_local(prim_from(pr), gamma, b, R(pref)), gamma);
+        fc.m = to_global(b, fc.m);
+    }
+    const R gf[5] = {fc.rho * area, fc.m.x * area, fc.m.y * area, fc.m.z * area, fc.e * area};
     flux_rec_store(G, s.F, f, gf);
 }
 

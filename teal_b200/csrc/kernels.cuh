@@ -54,21 +54,34 @@ __global__ void k_boundary(Sizes s, const int2 *__restrict__ lr, const double *_
 // gather the neighbours' states while the weights and offsets are still on their way. Each
 // gradient component is summed over the cell's slots in face order, as teal's face loop adds it.
 // Output: one gradient record per cell, (gx, gy, gz, psi) per variable (grad_rec_store); FOLD
-// multiplies psi in (Euler: only the limited gradient is used), otherwise the record keeps the
-// unlimited gradient for the viscous flux.
+// multiplies psi in (only the limited gradient is used), otherwise the record keeps the unlimited
+// gradient for the viscous flux.
+// SIDES writes the reconstructed states of the cell's sides instead, q + psi g . offset per slot
+// (derivative.c:158-164; side_index), for the face kernel to read two states of 40 bytes in place of two
+// gradient records, two states and two offsets (448 bytes): the thread has all of it at hand. Cells
+// flagged in SideOut::records store their gradient records as well: periodic faces have no slot in their
+// right cell, whose state is reconstructed with the face's own offset, and a partition sends records.
+template <typename R>
+struct SideOut {
+    R *rec = nullptr;                   // side records
+    const unsigned *records = nullptr;  // [tiles] cells whose gradient records are read, a bit each (null: none)
+};
+
 constexpr int GRAD_CELLS = 32;
 constexpr int GRAD_THREADS = 5 * GRAD_CELLS;
 
-template <typename R, int LIM, bool FOLD, bool MIXED, bool X>
-__global__ void __launch_bounds__(GRAD_THREADS, GRAD_MINB) k_gradient(Sizes s, Geometry<R> g,
+template <typename R, int LIM, bool FOLD, bool MIXED, bool X, bool SIDES = false>
+__global__ void __launch_bounds__(GRAD_THREADS, SIDES ? GRAD_MINB_SIDES : GRAD_MINB) k_gradient(Sizes s, Geometry<R> g,
                                                            const double *__restrict__ eps2,
                                                            const double *__restrict__ q,
-                                                           R *__restrict__ rec, int *err, int polls)
+                                                           R *__restrict__ rec, int *err, int polls,
+                                                           PressureRefOf<R> pr_ref, SideOut<R> side)
 {
     static_assert(X == kExact, "exact kernels live in the exact translation units only");
     __shared__ __align__(16) int s_nbr[MIXED ? MAX_SLOTS : 1][GRAD_CELLS];
+    constexpr bool OFFS = LIM != 0 || SIDES;  // the face offsets are used
     __shared__ __align__(16) R s_w[3 * MAX_SLOTS][GRAD_CELLS];
-    __shared__ __align__(16) R s_off[(LIM != 0) ? 3 * MAX_SLOTS : 1][GRAD_CELLS];
+    __shared__ __align__(16) R s_off[OFFS ? 3 * MAX_SLOTS : 1][GRAD_CELLS];
     __shared__ int s_cnt[MIXED ? GRAD_CELLS : 1];
     __shared__ uint64_t bar;
     __shared__ int s_J;
@@ -90,10 +103,10 @@ __global__ void __launch_bounds__(GRAD_THREADS, GRAD_MINB) k_gradient(Sizes s, G
             const unsigned char *tile_p = g.gtile + t0;
             const uint32_t nb = uint32_t(grad_tile_nbr_bytes<R>(J)), vb = uint32_t(grad_tile_vec_bytes<R>(J));
             mbar_init(&bar, 1);
-            mbar_arrive_expect_tx(&bar, nb + vb + (LIM != 0 ? vb : 0u));
+            mbar_arrive_expect_tx(&bar, nb + vb + (OFFS ? vb : 0u));
             bulk_g2s(&s_nbr[0][0], tile_p, nb, &bar);
             bulk_g2s(&s_w[0][0], tile_p + nb, vb, &bar);
-            if (LIM != 0) {
+            if (OFFS) {
                 bulk_g2s(&s_off[0][0], tile_p + nb + vb, vb, &bar);
             }
         }
@@ -111,9 +124,9 @@ __global__ void __launch_bounds__(GRAD_THREADS, GRAD_MINB) k_gradient(Sizes s, G
         constexpr uint32_t vb = uint32_t(grad_tile_vec_bytes<R>(MAX_SLOTS));
         if (threadIdx.x == 0) {
             mbar_init(&bar, 1);
-            mbar_arrive_expect_tx(&bar, vb + (LIM != 0 ? vb : 0u));
+            mbar_arrive_expect_tx(&bar, vb + (OFFS ? vb : 0u));
             bulk_g2s(&s_w[0][0], tile_p + nb, vb, &bar);
-            if (LIM != 0) {
+            if (OFFS) {
                 bulk_g2s(&s_off[0][0], tile_p + nb + vb, vb, &bar);
             }
         }
@@ -228,7 +241,28 @@ __global__ void __launch_bounds__(GRAD_THREADS, GRAD_MINB) k_gradient(Sizes s, G
         gy *= psi;
         gz *= psi;
     }
-    grad_rec_store(rec, c, v, gx, gy, gz, psi);
+    if constexpr (SIDES) {
+        double p0 = 0.0;
+        if constexpr (sizeof(R) == sizeof(float)) {
+            p0 = (v == 4) ? pr_ref.of(c) : 0.0;  // pressures relative to the reference (Local::dp)
+        }
+        const R q0 = R(qc - p0);
+        R *row_out = side.rec + (size_t)v * side_elements(s.SL) + (size_t)tile * SIDE_TILE;
+        if (side.records && ((__ldg(side.records + tile) >> l) & 1u)) {
+            grad_rec_store(rec, c, v, gx, gy, gz, psi);
+        }
+#pragma unroll
+        for (int j = 0; j < MAX_SLOTS; j++) {
+            if (j >= jmax) break;
+            if (j < cnt) {
+                row_out[j * GRAD_CELLS + l] =
+                    at_face(q0, v3(gx, gy, gz), v3(s_off[3 * j + 0][l], s_off[3 * j + 1][l], s_off[3 * j + 2][l]));
+            }
+        }
+    }
+    else {
+        grad_rec_store(rec, c, v, gx, gy, gz, psi);
+    }
 }
 
 // per-cell time step of the equations' Timestep plugin

@@ -18,6 +18,7 @@ struct FaceLaunch {
     int *err;  // device error word (bounded waits that give up set ERR_TIMEOUT)
     PressureRef pr_ref;  // FP32-flux form: reference pressure per instance
     int polls;           // limit of the staged kernel's first wait (MBAR_POLLS unless a test lowers it)
+    const void *side;    // side records (k_gradient SIDES), or null: gradient records only
 };
 
 // The launchers below are local to each translation unit (unnamed namespace): the exact and the plain
@@ -55,12 +56,31 @@ inline cudaError_t launch_face_r(bool ns, int order, bool fold, const FaceLaunch
     const Geometry<R> &g = *static_cast<const Geometry<R> *>(a.geom);
     const R *rec = static_cast<const R *>(a.rec);
     R *G = static_cast<R *>(a.G);
+    if constexpr (!kExact) {
+        if (a.side) {
+            if (a.s.hi <= a.s.lo) {
+                return cudaSuccess;
+            }
+            PressureRefOf<R> pref{};
+            if constexpr (sizeof(R) == sizeof(float)) {
+                pref = a.pr_ref;
+            }
+            k_face_sides<R, FK><<<(a.s.hi - a.s.lo + SIDE_BLOCK - 1) / SIDE_BLOCK, SIDE_BLOCK, 0, st>>>(
+                a.s, g, a.q, static_cast<const R *>(a.side), rec, R(a.gamma), G, pref);
+            return cudaGetLastError();
+        }
+    }
     const bool staged = !ns && TG_FACE_STAGED_EULER != 0;
     if (order == 1) {
         launch_face_v<R, FK, false, 1, true>(staged, a, g, rec, G, st);
     }
     else if (!ns) {
-        launch_face_v<R, FK, false, 2, true>(staged, a, g, rec, G, st);
+        if constexpr (kExact) {  // the other forms have side records
+            launch_face_v<R, FK, false, 2, true>(staged, a, g, rec, G, st);
+        }
+        else {
+            return cudaErrorInvalidValue;
+        }
     }
     else if (fold) {
         launch_face_v<R, FK, true, 2, true>(staged, a, g, rec, G, st);

@@ -58,6 +58,19 @@ __device__ __forceinline__ R dot(V3<R> a, V3<R> b)
     return ((a.x * b.x) + (a.y * b.y)) + (a.z * b.z);
 }
 
+// q + g . off, a cell's value at a face centre (derivative.c:158-164); contracted the same way in every
+// kernel that forms it, so that they agree bit for bit
+template <typename R>
+__device__ __forceinline__ R at_face(R q, V3<R> g, V3<R> off)
+{
+    if constexpr (kExact) {
+        return q + dot(g, off);
+    }
+    else {
+        return q + fma(g.z, off.z, fma(g.y, off.y, g.x * off.x));
+    }
+}
+
 // face basis: rows x (unit normal), y, z (tangents); row-major as teal's Matrix (src/matrix.h)
 template <typename R>
 struct Basis {

@@ -16,18 +16,18 @@ static void gradient_m(const GradientLaunch &a, cudaStream_t st)
     if (a.s.hi <= a.s.lo) return;
     dim3 grid((a.s.hi - a.s.lo + GRAD_CELLS - 1) / GRAD_CELLS);
     switch (a.limiter) {
-        case 0: k_gradient<double, 0, true, MIXED, true><<<grid, GRAD_THREADS, 0, st>>>(a.s, a.g, a.eps2, a.q, a.rec, a.err, a.polls); break;
+        case 0: k_gradient<double, 0, true, MIXED, true><<<grid, GRAD_THREADS, 0, st>>>(a.s, a.g, a.eps2, a.q, a.rec, a.err, a.polls, NoPressureRef{}, SideOut<double>{}); break;
         case 1:
             if (a.fold)
-                k_gradient<double, 1, true, MIXED, true><<<grid, GRAD_THREADS, 0, st>>>(a.s, a.g, a.eps2, a.q, a.rec, a.err, a.polls);
+                k_gradient<double, 1, true, MIXED, true><<<grid, GRAD_THREADS, 0, st>>>(a.s, a.g, a.eps2, a.q, a.rec, a.err, a.polls, NoPressureRef{}, SideOut<double>{});
             else
-                k_gradient<double, 1, false, MIXED, true><<<grid, GRAD_THREADS, 0, st>>>(a.s, a.g, a.eps2, a.q, a.rec, a.err, a.polls);
+                k_gradient<double, 1, false, MIXED, true><<<grid, GRAD_THREADS, 0, st>>>(a.s, a.g, a.eps2, a.q, a.rec, a.err, a.polls, NoPressureRef{}, SideOut<double>{});
             break;
         default:
             if (a.fold)
-                k_gradient<double, 2, true, MIXED, true><<<grid, GRAD_THREADS, 0, st>>>(a.s, a.g, a.eps2, a.q, a.rec, a.err, a.polls);
+                k_gradient<double, 2, true, MIXED, true><<<grid, GRAD_THREADS, 0, st>>>(a.s, a.g, a.eps2, a.q, a.rec, a.err, a.polls, NoPressureRef{}, SideOut<double>{});
             else
-                k_gradient<double, 2, false, MIXED, true><<<grid, GRAD_THREADS, 0, st>>>(a.s, a.g, a.eps2, a.q, a.rec, a.err, a.polls);
+                k_gradient<double, 2, false, MIXED, true><<<grid, GRAD_THREADS, 0, st>>>(a.s, a.g, a.eps2, a.q, a.rec, a.err, a.polls, NoPressureRef{}, SideOut<double>{});
             break;
     }
 }

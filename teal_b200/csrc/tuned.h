@@ -19,6 +19,15 @@
 #ifndef TG_FACE_MINB_EULER
 #define TG_FACE_MINB_EULER 28  // Euler face-flux blocks kept resident per SM (caps registers per thread)
 #endif
+#ifndef TG_SIDE_BLOCK
+#define TG_SIDE_BLOCK 128  // threads per face-flux block between side records
+#endif
+#ifndef TG_SIDE_MINB
+#define TG_SIDE_MINB 6  // its blocks kept resident per SM, FP64
+#endif
+#ifndef TG_SIDE_MINB_FP32
+#define TG_SIDE_MINB_FP32 8  // its blocks kept resident per SM, FP32-flux form
+#endif
 #ifndef TG_CELL_BLOCK
 #define TG_CELL_BLOCK 128  // threads per cell-gather block
 #endif
@@ -30,4 +39,7 @@
 #endif
 #ifndef TG_GRAD_MINB
 #define TG_GRAD_MINB 12  // gradient blocks (160 threads) kept resident per SM (caps registers per thread)
+#endif
+#ifndef TG_GRAD_MINB_SIDES
+#define TG_GRAD_MINB_SIDES 10  // the same for the gradient kernel that writes side records
 #endif
