@@ -28,89 +28,89 @@ __global__ void __launch_bounds__(BLOCK) k_piece_average(Segments seg, int N, co
     for (int k = 0; k < 5; k++) {
         double sum = block_sum<BLOCK>(t[k], sh);
         if (threadIdx.x == 0) {
-            part[5 * blockIdx.x + k] = sum;
+            part[(size_t)k * seg.npieces + blockIdx.x] = sum;
         }
     }
 }
 
-// avg[i] = sum of instance i's piece sums / its volume
+// avg[i] = sum of instance i's piece sums / its volume, one warp per instance
 __global__ void k_inst_average(Segments seg, const double *__restrict__ part, double *__restrict__ avg)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= seg.ninst) {
-        return;
-    }
+    const int i = blockIdx.x, beg = seg.inst_piece_off[i], end = seg.inst_piece_off[i + 1];
     for (int k = 0; k < 5; k++) {
-        double t = 0;
-        for (int p = seg.inst_piece_off[i]; p < seg.inst_piece_off[i + 1]; p++) {
-            t += part[5 * p + k];
+        const double t = sum_partials(part + (size_t)k * seg.npieces + beg, end - beg, threadIdx.x);
+        if (threadIdx.x == 0) {
+            avg[5 * i + k] = t / seg.sum_volume[i];
         }
-        avg[5 * i + k] = t / seg.sum_volume[i];
     }
 }
 
 // ---- per-instance reductions (deterministic: fixed pieces, fixed order) ---------------------
 
-// per piece: minimum cell time step and (with `res`) the sums of V * R^2 per variable
+// minimum of the cell time steps and (with `res`) the sums of V * R^2 per variable of one piece, by a
+// block of BLOCK threads: part_min[piece], part_sum[k][piece]
+__device__ __forceinline__ void reduce_piece(const Segments &seg, int C, const double *__restrict__ dtc,
+                                             const double *__restrict__ R, const double *__restrict__ volume,
+                                             bool res, double *part_min, double *part_sum)
+{
+    const int beg = seg.piece_beg[blockIdx.x], end = seg.piece_beg[blockIdx.x + 1];
+    double t[6] = {0, 0, 0, 0, 0, DBL_MAX};
+    for (int c = beg + threadIdx.x; c < end; c += BLOCK) {
+        t[5] = fmin(t[5], dtc[c]);
+        if (res) {
+            const double v = volume[c];
+#pragma unroll
+            for (int k = 0; k < 5; k++) {
+                const double r = R[(size_t)k * C + c];
+                t[k] += v * (r * r);
+            }
+        }
+    }
+    const double x = block_reduce6(t);
+    const int k = threadIdx.x;
+    if (k == 5) {
+        part_min[blockIdx.x] = x;
+    }
+    else if (k < 5 && res) {
+        part_sum[(size_t)k * seg.npieces + blockIdx.x] = x;
+    }
+}
+
 __global__ void __launch_bounds__(BLOCK) k_piece_reduce(Segments seg, int C, const double *__restrict__ dtc,
                                                         const double *__restrict__ R,
                                                         const double *__restrict__ volume, int res,
                                                         double *__restrict__ part_min,
                                                         double *__restrict__ part_sum)
 {
-    __shared__ double sh[BLOCK / 32];
-    const int beg = seg.piece_beg[blockIdx.x], end = seg.piece_beg[blockIdx.x + 1];
-    double m = DBL_MAX;
-    double t[5] = {0, 0, 0, 0, 0};
-    for (int c = beg + threadIdx.x; c < end; c += BLOCK) {
-        m = fmin(m, dtc[c]);
-        if (res) {
-            double v = volume[c];
-#pragma unroll
-            for (int k = 0; k < 5; k++) {
-                double r = R[k * C + c];
-                t[k] += v * (r * r);
-            }
-        }
-    }
-    m = block_min<BLOCK>(m, sh);
-    if (threadIdx.x == 0) {
-        part_min[blockIdx.x] = m;
-    }
-    if (res) {
-#pragma unroll
-        for (int k = 0; k < 5; k++) {
-            double sum = block_sum<BLOCK>(t[k], sh);
-            if (threadIdx.x == 0) {
-                part_sum[5 * blockIdx.x + k] = sum;
-            }
-        }
+    reduce_piece(seg, C, dtc, R, volume, res != 0, part_min, part_sum);
+}
+
+constexpr int INST_BLOCK = 32;
+
+// start of a step of instance i from the minimum m of its cells' steps: step0 = courant * m, step =
+// min(step0, clip)
+__device__ __forceinline__ void begin_step(const Steps &st, int i, double courant, double m)
+{
+    const double step0 = courant * m;
+    const double clip = st.use_max_time ? (st.max_time[i] - st.time[i]) : st.max_step[i];
+    st.step0[i] = step0;
+    st.step[i] = fmin(step0, clip);
+    if (!isfinite(step0) || !(step0 > 0)) {  // the instance stops; the others go on
+        atomicOr(st.error, ERR_NONFINITE);
+        st.fail[i] = 1;
+        st.active[i] = 0;
+        atomicSub(st.num_active, 1);
     }
 }
 
-constexpr int INST_BLOCK = 128;
-
-// start of a step, one block per instance: step0 = courant * min, step = min(step0, clip)
+// start of a step, one warp per instance
 __global__ void __launch_bounds__(INST_BLOCK) k_inst_begin(Segments seg, const double *__restrict__ part_min,
                                                            double courant, Steps st)
 {
-    __shared__ double sh[INST_BLOCK / 32];
-    const int i = blockIdx.x;
-    double m = DBL_MAX;
-    for (int p = seg.inst_piece_off[i] + threadIdx.x; p < seg.inst_piece_off[i + 1]; p += INST_BLOCK) {
-        m = fmin(m, part_min[p]);
-    }
-    m = block_min<INST_BLOCK>(m, sh);
+    const int i = blockIdx.x, beg = seg.inst_piece_off[i], end = seg.inst_piece_off[i + 1];
+    const double m = min_partials(part_min + beg, end - beg, threadIdx.x);
     if (threadIdx.x == 0 && st.active[i]) {
-        double step0 = courant * m;
-        double clip = st.use_max_time ? (st.max_time[i] - st.time[i]) : st.max_step[i];
-        st.step0[i] = step0;
-        st.step[i] = fmin(step0, clip);
-        if (!isfinite(step0) || !(step0 > 0)) {  // the instance stops; the others go on
-            atomicOr(st.error, ERR_NONFINITE);
-            st.fail[i] = 1;
-            st.active[i] = 0;
-        }
+        begin_step(st, i, courant, m);
     }
 }
 
@@ -120,30 +120,43 @@ __device__ __forceinline__ bool is_close(double a, double b)
     return fabs(a - b) <= fmax(1e-8, 1e-5 * fmax(fabs(a), fabs(b)));
 }
 
-// end of a step (or a bare residual), one block per instance: residual = sqrt(sum / sum_volume);
-// with `advance`: time += step, iteration count, and the run loop's stop tests
-// (src/simulation/run.c:68-83): iterations, residual threshold, end time
-__global__ void __launch_bounds__(INST_BLOCK) k_inst_end(Segments seg, const double *__restrict__ part_sum,
-                                                         int advance, Steps st)
+// End of a step (or a bare residual, `advance` off): the partials of every piece, then by the last block of
+// each instance residual = sqrt(sum / sum_volume) and, with `advance`, time += step, the iteration
+// count and the run loop's stop tests (src/simulation/run.c:68-83): iterations, residual threshold, end
+// time. With `begin` an instance that goes on also starts its next step (a run loop's replayed
+// steps: one launch between the last stage of a step and the first of the next, where the pieces,
+// the instances, the count of active instances and the start were four).
+__global__ void __launch_bounds__(BLOCK) k_step_end(Segments seg, int C, const double *__restrict__ dtc,
+                                                    const double *__restrict__ R, const double *__restrict__ volume,
+                                                    double *part_min, double *part_sum, int advance, int begin,
+                                                    double courant, Steps st)
 {
-    __shared__ double sh[INST_BLOCK / 32];
-    const int i = blockIdx.x;
-    const bool was_active = st.active[i] != 0;
-    double res[5];
-    for (int k = 0; k < 5; k++) {
-        double t = 0;
-        for (int p = seg.inst_piece_off[i] + threadIdx.x; p < seg.inst_piece_off[i + 1]; p += INST_BLOCK) {
-            t += part_sum[5 * p + k];
-        }
-        res[k] = block_sum<INST_BLOCK>(t, sh);
-    }
-    if (threadIdx.x != 0 || (advance && !was_active)) {
+    __shared__ double s_res[6];
+    const int i = seg.cell_inst[seg.piece_beg[blockIdx.x]];
+    if (advance && !st.active[i]) {
         return;
     }
-    double mx = 0;
+    reduce_piece(seg, C, dtc, R, volume, true, part_min, part_sum);
+    if (!last_of_instance(seg, i)) {
+        return;
+    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp < 6) {
+        const int beg = seg.inst_piece_off[i], n = seg.inst_piece_off[i + 1] - beg;
+        const double t = (warp == 5) ? min_partials(part_min + beg, n, lane)
+                                     : sum_partials(part_sum + (size_t)warp * seg.npieces + beg, n, lane);
+        if (lane == 0) {
+            s_res[warp] = t;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) {
+        return;
+    }
+    double res[5], mx = 0;
     bool finite = true;
     for (int k = 0; k < 5; k++) {
-        res[k] = sqrt(res[k] / seg.sum_volume[i]);
+        res[k] = sqrt(s_res[k] / seg.sum_volume[i]);
         st.residual[5 * i + k] = res[k];
         mx = (res[k] > mx) ? res[k] : mx;
         finite = finite && isfinite(res[k]);
@@ -156,13 +169,12 @@ __global__ void __launch_bounds__(INST_BLOCK) k_inst_end(Segments seg, const dou
     }
     if (!finite) {  // the instance stops with its step counted; the others go on
         st.fail[i] = 1;
-        st.active[i] = 0;
     }
     double t = st.time[i] + st.step[i];
     st.time[i] = t;
     int it = st.iter[i] + 1;
     st.iter[i] = it;
-    bool stop = it >= st.max_iter[i];
+    bool stop = !finite || it >= st.max_iter[i];
     if (st.threshold[i] > 0) {
         int v = st.variable[i];
         stop = stop || (((v >= 0) ? res[v] : mx) < st.threshold[i]);
@@ -173,25 +185,10 @@ __global__ void __launch_bounds__(INST_BLOCK) k_inst_end(Segments seg, const dou
     }
     if (stop) {
         st.active[i] = 0;
+        atomicSub(st.num_active, 1);
     }
-}
-
-// number of active instances after a step
-__global__ void k_count_active(int ninst, Steps st)
-{
-    __shared__ int sh;
-    if (threadIdx.x == 0) {
-        sh = 0;
-    }
-    __syncthreads();
-    int n = 0;
-    for (int i = threadIdx.x; i < ninst; i += blockDim.x) {
-        n += st.active[i] != 0;
-    }
-    atomicAdd(&sh, n);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        *st.num_active = sh;
+    else if (begin) {
+        begin_step(st, i, courant, s_res[5]);
     }
 }
 

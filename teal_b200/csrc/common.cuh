@@ -336,4 +336,84 @@ __device__ __forceinline__ double block_min(double v, double *sh)
     return r;
 }
 
+// Sums over the block (threads of BLOCK) of t[0..4] and the minimum of t[5], valid in threads 0-5 (thread k:
+// value k); fixed shape
+__device__ __forceinline__ double block_reduce6(double (&t)[6])
+{
+    __shared__ double sh[6][BLOCK / 32];
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double x = __shfl_down_sync(0xffffffffu, t[k], o);
+            t[k] = (k == 5) ? fmin(t[k], x) : t[k] + x;
+        }
+    }
+    if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+        for (int k = 0; k < 6; k++) {
+            sh[k][threadIdx.x >> 5] = t[k];
+        }
+    }
+    __syncthreads();
+    const int k = threadIdx.x;
+    double x = 0;
+    if (k < 6) {
+        x = sh[k][0];
+        for (int w = 1; w < BLOCK / 32; w++) {
+            x = (k == 5) ? fmin(x, sh[k][w]) : x + sh[k][w];
+        }
+    }
+    return x;
+}
+
+// ---- sums over the pieces of an instance by its last block ------------------------------------
+
+// Whether this block is the last one of its instance to finish the current pass over the pieces: the
+// partials of all its pieces are then visible to it. The same answer in every thread.
+__device__ __forceinline__ bool last_of_instance(const Segments &seg, int inst)
+{
+    __shared__ int last;
+    __threadfence();  // this thread's partials before the ticket
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const int n = seg.inst_piece_off[inst + 1] - seg.inst_piece_off[inst];
+        last = atomicAdd(seg.ticket + inst, 1) == n - 1;
+        if (last) {
+            seg.ticket[inst] = 0;  // for the next pass
+        }
+    }
+    __syncthreads();
+    if (last) {
+        __threadfence();
+    }
+    return last != 0;
+}
+
+// One warp's sum (in every lane) and minimum of n partials
+__device__ __forceinline__ double sum_partials(const double *part, int n, int lane)
+{
+    double t = 0;
+    for (int p = lane; p < n; p += 32) {
+        t += __ldcg(part + p);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        t += __shfl_xor_sync(0xffffffffu, t, o);
+    }
+    return t;
+}
+__device__ __forceinline__ double min_partials(const double *part, int n, int lane)
+{
+    double t = DBL_MAX;
+    for (int p = lane; p < n; p += 32) {
+        t = fmin(t, __ldcg(part + p));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        t = fmin(t, __shfl_xor_sync(0xffffffffu, t, o));
+    }
+    return t;
+}
+
 }  // namespace tg

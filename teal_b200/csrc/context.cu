@@ -168,11 +168,7 @@ struct Gmres {
     double *w = nullptr;      // [5][C]
     double *q1 = nullptr;     // [5][N] perturbed primitive state
     double *R1 = nullptr;     // [5][C] derivative of the perturbed state
-    int nchunks = 0;          // cell chunks of the Krylov vectors
-    int *chunk_beg = nullptr;       // [nchunks + 1]
-    int *inst_chunk_off = nullptr;  // [ninst + 1]
-    double *part = nullptr;   // [2 dim + 1][nchunks] partial sums
-    int *ticket = nullptr;    // [ninst] chunks that have finished the current pass
+    double *part = nullptr;   // [2 dim + 1][pieces] partial sums
     double *sc = nullptr;     // per-instance device scalars (GmresScalar)
     int *flag = nullptr;      // per-instance progress (GmresFlag)
     int *ctl = nullptr;       // [GC_COUNT] loop counters of the graph-driven loops
@@ -223,6 +219,7 @@ struct tg_ctx {
     int *rowmap = nullptr;          // teal row of an instance -> arena state row (periodic: owner)
     std::vector<int> h_inst_cell_off;
     int *cell_inst = nullptr, *inst_cell_off = nullptr, *piece_beg = nullptr, *inst_piece_off = nullptr;
+    int *ticket = nullptr;
     double *sum_volume = nullptr;
     int npieces = 0;
     Segments seg{};
@@ -351,8 +348,7 @@ static const double LSERK_ALPHA[3][6][7] = {
 
 static void free_gmres(Gmres &g)
 {
-    void *p[] = {g.U,    g.r,      g.V,  g.w,    g.q1,  g.R1, g.chunk_beg, g.inst_chunk_off,
-                 g.part, g.ticket, g.sc, g.flag, g.ctl, g.Rm};
+    void *p[] = {g.U, g.r, g.V, g.w, g.q1, g.R1, g.part, g.sc, g.flag, g.ctl, g.Rm};
     for (void *x : p) {
         if (x) cudaFree(x);
     }
@@ -378,7 +374,7 @@ static void free_ctx(tg_ctx *c)
                     c->gb.slot_w, c->gb.slot_off, c->gb.area32, c->gb.basis32, c->gb.offl32, c->gb.offr32,
                     c->gb.corr32, c->gb.tile64, c->gb.tile32, c->gb.toff64, c->gb.toff32, c->q, c->U0, c->R, c->qs, c->grad, c->G,
                     c->dtc, c->part_min, c->part_sum, c->sd, c->si, c->aos, c->rowmap, c->cell_inst,
-                    c->inst_cell_off, c->piece_beg, c->inst_piece_off, c->sum_volume, c->src_avg,
+                    c->inst_cell_off, c->piece_beg, c->inst_piece_off, c->ticket, c->sum_volume, c->src_avg,
                     c->send_rows, c->send_q, c->recv_q, c->send_rec, c->recv_rec};
     for (void *p : ptrs) {
         if (p) cudaFree(p);
@@ -821,7 +817,8 @@ static int create_ctx(MeshInput &in, const tg_equations *e, int precision, tg_ct
         std::vector<int> cell_inst(s.C), piece_beg, inst_piece_off(1, 0);
         for (int i = 0; i < c->ninst; i++) {
             for (int x = in.inst_cell_off[i]; x < in.inst_cell_off[i + 1]; x++) cell_inst[x] = i;
-            for (int x = in.inst_cell_off[i]; x < in.inst_cell_off[i + 1]; x += PIECE) piece_beg.push_back(x);
+            const int per = piece_cells(in.inst_cell_off[i + 1] - in.inst_cell_off[i]);
+            for (int x = in.inst_cell_off[i]; x < in.inst_cell_off[i + 1]; x += per) piece_beg.push_back(x);
             inst_piece_off.push_back((int)piece_beg.size());
         }
         c->npieces = (int)piece_beg.size();
@@ -832,8 +829,10 @@ static int create_ctx(MeshInput &in, const tg_equations *e, int precision, tg_ct
         TRY(upload(&c->inst_piece_off, inst_piece_off.data(), inst_piece_off.size(), st));
         TRY(upload(&c->sum_volume, in.sum_volume.data(), in.sum_volume.size(), st));
         TRY(upload(&c->rowmap, in.rowmap.data(), in.rowmap.size(), st));
+        TRY(dalloc(&c->ticket, c->ninst));
+        CU(cudaMemsetAsync(c->ticket, 0, sizeof(int) * c->ninst, st));
         c->seg = Segments{c->ninst, c->npieces, c->cell_inst, c->inst_cell_off, c->piece_beg, c->inst_piece_off,
-                          c->sum_volume};
+                          c->sum_volume, c->ticket};
 
         // raw teal arrays -> device temporaries
         int *d_face_cell = nullptr, *d_err = nullptr, *d_cnt = nullptr;
@@ -1695,7 +1694,7 @@ static int run_fluxes_pre(tg_ctx *c, double *q, bool masked)
         // the Prepare pass: volume averages of the state being differentiated, per instance
         Launch l(c, TG_PROF_REDUCE);
         k_piece_average<<<c->npieces, BLOCK, 0, c->stream>>>(c->seg, c->s.N, q, c->volume, c->part_sum);
-        k_inst_average<<<(c->ninst + 127) / 128, 128, 0, c->stream>>>(c->seg, c->part_sum, c->src_avg);
+        k_inst_average<<<c->ninst, 32, 0, c->stream>>>(c->seg, c->part_sum, c->src_avg);
         CU(cudaGetLastError());
     }
     if (c->source == TG_SOURCE_DEVICE) {
@@ -1732,6 +1731,24 @@ static int run_pieces(tg_ctx *c, int res)
     return TG_OK;
 }
 
+// end of a step, or with advance off the residual norm of c->R alone (k_step_end)
+static int run_step_end(tg_ctx *c, int advance, int begin, double courant)
+{
+    Launch l(c, TG_PROF_REDUCE);
+    k_step_end<<<c->npieces, BLOCK, 0, c->stream>>>(c->seg, c->s.C, c->dtc, c->R, c->volume, c->part_min, c->part_sum,
+                                                    advance, begin, courant, c->st);
+    CU(cudaGetLastError());
+    return TG_OK;
+}
+
+static int run_inst_begin(tg_ctx *c, double courant)
+{
+    Launch l(c, TG_PROF_REDUCE);
+    k_inst_begin<<<c->ninst, INST_BLOCK, 0, c->stream>>>(c->seg, c->part_min, courant, c->st);
+    CU(cudaGetLastError());
+    return TG_OK;
+}
+
 static int run_prepare(tg_ctx *c)
 {
     CellData cd{c->volume, c->proj, c->eps2};
@@ -1759,6 +1776,8 @@ static int read_steps(tg_ctx *c)
 
 static int write_steps(tg_ctx *c)
 {
+    hi_num_active(c) = 0;
+    for (int i = 0; i < c->ninst; i++) hi_num_active(c) += hi_at(c, SI_ACTIVE, i) != 0;
     CU(cudaMemcpyAsync(c->sd, c->hd, sizeof(double) * SD_COUNT * c->ninst, cudaMemcpyHostToDevice, c->stream));
     CU(cudaMemcpyAsync(c->si, c->hi, sizeof(int) * (SI_COUNT * c->ninst + 2), cudaMemcpyHostToDevice, c->stream));
     return TG_OK;
@@ -1848,8 +1867,7 @@ extern "C" int tg_timestep(tg_ctx *c, double *step)
     }
     c->st.use_max_time = 0;
     TRY(write_steps(c));
-    k_inst_begin<<<c->ninst, INST_BLOCK, 0, c->stream>>>(c->seg, c->part_min, 1.0, c->st);
-    CU(cudaGetLastError());
+    TRY(run_inst_begin(c, 1.0));
     TRY(read_steps(c));
     *step = hd_at(c, SD_STEP0, 0);
     return TG_OK;
@@ -1862,9 +1880,7 @@ extern "C" int tg_residual(tg_ctx *c, const double *deriv, double *residual)
     TRY(h2d(c, c->aos, deriv, 5 * (size_t)c->s.C));
     k_aos5_to_soa<<<grid_of(c->s.C), BLOCK, 0, c->stream>>>(c->s.C, c->aos, c->R);
     CU(cudaGetLastError());
-    TRY(run_pieces(c, 1));
-    k_inst_end<<<c->ninst, INST_BLOCK, 0, c->stream>>>(c->seg, c->part_sum, 0, c->st);
-    CU(cudaGetLastError());
+    TRY(run_step_end(c, 0, 0, 0.0));
     TRY(read_steps(c));
     residual_of(c, 0, residual);
     c->prepared = false;  // the piece minima were recomputed from stale cell steps
@@ -1894,30 +1910,19 @@ static int rk_params(const tg_ctx *c, int method, const void *context, int *stag
     return TG_OK;
 }
 
-// one explicit step of every active instance (U0 and the piece minima must be current)
+// one explicit step of every active instance (U0 and the piece minima must be current). A run loop's
+// steps (use_max_time) find their time step begun by the launch before and begin the next one
 static int enqueue_explicit_step(tg_ctx *c, int stages, const double *alpha, double courant)
 {
-    {
-        Launch l(c, TG_PROF_REDUCE);
-        k_inst_begin<<<c->ninst, INST_BLOCK, 0, c->stream>>>(c->seg, c->part_min, courant, c->st);
-    }
-    CU(cudaGetLastError());
+    const int begin_next = c->st.use_max_time;
+    if (!begin_next) TRY(run_inst_begin(c, courant));
     for (int i = 0; i < stages; i++) {
         // the residual of stage i at time + alpha_i step (advance.c:100)
         c->t_time = c->st.time, c->t_step = c->st.step, c->t_coef = alpha[i];
         TRY(run_fluxes(c, c->q, true));
         TRY(launch_cell<1>(c, alpha[i + 1], i == stages - 1, c->q, c->R));
     }
-    TRY(run_pieces(c, 1));
-    {
-        Launch l(c, TG_PROF_REDUCE);
-        k_inst_end<<<c->ninst, INST_BLOCK, 0, c->stream>>>(c->seg, c->part_sum, 1, c->st);
-    }
-    {
-        Launch l(c, TG_PROF_REDUCE);
-        k_count_active<<<1, 256, 0, c->stream>>>(c->ninst, c->st);
-    }
-    CU(cudaGetLastError());
+    TRY(run_step_end(c, 1, begin_next, courant));
     return TG_OK;
 }
 
@@ -2105,11 +2110,7 @@ static int advance_chunked(tg_ctx *c, int stages, const double *alpha, double co
     const long N = c->s.N;
     const int rows = c->inst_row_off[1];
     std::vector<char> fl(K, 0);
-    {
-        Launch l(c, TG_PROF_REDUCE);
-        k_inst_begin<<<c->ninst, INST_BLOCK, 0, c->stream>>>(c->seg, c->part_min, courant, c->st);
-    }
-    CU(cudaGetLastError());
+    TRY(run_inst_begin(c, courant));
     // the stages before the last one as in an unsplit step
     int i = 0;
     for (; i < stages - 1; i++) {
@@ -2156,16 +2157,7 @@ static int advance_chunked(tg_ctx *c, int stages, const double *alpha, double co
         CU(cudaMemcpyAsync(out + 5 * (size_t)C, c->aos + 5 * (size_t)C, sizeof(double) * 5 * (size_t)n,
                            cudaMemcpyDeviceToHost, p.copy));
     }
-    TRY(run_pieces(c, 1));
-    {
-        Launch l(c, TG_PROF_REDUCE);
-        k_inst_end<<<c->ninst, INST_BLOCK, 0, c->stream>>>(c->seg, c->part_sum, 1, c->st);
-    }
-    {
-        Launch l(c, TG_PROF_REDUCE);
-        k_count_active<<<1, 256, 0, c->stream>>>(c->ninst, c->st);
-    }
-    CU(cudaGetLastError());
+    TRY(run_step_end(c, 1, 0, courant));
     CU(cudaStreamSynchronize(p.copy));
     return TG_OK;
 }
@@ -2227,6 +2219,7 @@ static int run_instances(tg_ctx *c, int method, const void *context, double cour
     if (!c->prepared) TRY(run_prepare(c));
     TRY(write_steps(c));
     TRY(step_graph(c, method, stages, alpha, courant, 1));
+    TRY(run_inst_begin(c, courant));
     for (int it = 0; it < max_launch;) {
         int n = (max_launch - it < every) ? max_launch - it : every;
         for (int k = 0; k < n; k++) TRY(launch_step(c, stages, alpha, courant));
@@ -2347,21 +2340,7 @@ static int gm_alloc(tg_ctx *c, int dim)
     TRY(dalloc(&g.q1, 5 * (size_t)c->s.N));
     CU(cudaMemset(g.q1, 0, 5 * sizeof(double) * c->s.N));
     TRY(dalloc(&g.R1, n));
-    std::vector<int> beg, off(1, 0);
-    for (int i = 0; i < c->ninst; i++) {
-        const int lo = c->h_inst_cell_off[i], hi = c->h_inst_cell_off[i + 1];
-        const int per = krylov_chunk(hi - lo);
-        for (int x = lo; x < hi; x += per) beg.push_back(x);
-        off.push_back((int)beg.size());
-    }
-    g.nchunks = (int)beg.size();
-    beg.push_back(c->s.C);
-    TRY(dalloc(&g.chunk_beg, beg.size()));
-    TRY(dalloc(&g.inst_chunk_off, off.size()));
-    CU(cudaMemcpy(g.chunk_beg, beg.data(), sizeof(int) * beg.size(), cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(g.inst_chunk_off, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice));
-    TRY(dalloc(&g.part, (size_t)(2 * dim + 1) * g.nchunks));
-    TRY(dalloc(&g.ticket, (size_t)c->ninst));
+    TRY(dalloc(&g.part, (size_t)(2 * dim + 1) * c->npieces));
     TRY(dalloc(&g.sc, (size_t)c->ninst * gmres_scn(dim)));
     TRY(dalloc(&g.flag, (size_t)GF_COUNT * c->ninst));
     CU(cudaMemset(g.flag, 0, sizeof(int) * GF_COUNT * c->ninst));
@@ -2375,8 +2354,7 @@ static int gm_alloc(tg_ctx *c, int dim)
 static GmresBatch gm_batch(tg_ctx *c, int dim)
 {
     const Gmres &g = c->gm;
-    return GmresBatch{dim,    gmres_scn(dim), c->ninst, g.nchunks, c->cell_inst, g.chunk_beg, g.inst_chunk_off,
-                      g.part, g.ticket,       g.sc,     g.flag,    g.ctl};
+    return GmresBatch{dim, gmres_scn(dim), c->ninst, c->seg, g.part, g.sc, g.flag, g.ctl};
 }
 
 // ---- device-driven loops of a captured graph ---------------------------------------------------
@@ -2471,8 +2449,8 @@ static int gm_solve(tg_ctx *c, const GmresBatch &gb)
     k_krylov_vector<<<cb, BLOCK, 0, c->stream>>>(C, c->s.N, g.U, g.r, g.w, gb, c->prop[0], g.V, g.q1);
     CU(cudaGetLastError());
     TRY(gm_derivative(c, g.q1, g.R1, c->precision));
-    k_arnoldi_dots<<<g.nchunks, KRYLOV_BLOCK, 0, c->stream>>>(C, g.V, g.R1, g.Rm ? g.Rm : c->R, gb, g.w);
-    k_arnoldi_update<<<g.nchunks, KRYLOV_BLOCK, 0, c->stream>>>(C, g.V, gb, g.w, arnoldi.h);
+    k_arnoldi_dots<<<c->npieces, KRYLOV_BLOCK, 0, c->stream>>>(C, g.V, g.R1, g.Rm ? g.Rm : c->R, gb, g.w);
+    k_arnoldi_update<<<c->npieces, KRYLOV_BLOCK, 0, c->stream>>>(C, g.V, gb, g.w, arnoldi.h);
     CU(cudaGetLastError());
     c->launches += 3;
     TRY(while_end(c, arnoldi));
@@ -2496,7 +2474,7 @@ static int newton_params(const void *context, double *newton_tol, double *krylov
 
 // One implicit Euler step of every active instance (advance.c:119-195), enqueued on a capturing
 // stream: CFL step, Newton iterations (a device loop) with a GMRES solve each, then the residual
-// norm and the run loop's time / iteration / stop bookkeeping (k_inst_end). The device step arrays
+// norm and the run loop's time / iteration / stop bookkeeping (k_step_end). The device step arrays
 // must be current when the graph runs.
 static int enqueue_implicit_step(tg_ctx *c, double courant, double newton_tol, double krylov_tol, int dim)
 {
@@ -2510,11 +2488,7 @@ static int enqueue_implicit_step(tg_ctx *c, double courant, double newton_tol, d
 
     // step from the CFL condition; U = cons(q) (advance.c:136-143)
     TRY(run_prepare(c));
-    {
-        Launch l(c, TG_PROF_REDUCE);
-        k_inst_begin<<<c->ninst, INST_BLOCK, 0, c->stream>>>(c->seg, c->part_min, courant, c->st);
-    }
-    CU(cudaGetLastError());
+    TRY(run_inst_begin(c, courant));
     CU(cudaMemcpyAsync(g.U, c->U0, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
     c->prepared = false;
 
@@ -2522,7 +2496,7 @@ static int enqueue_implicit_step(tg_ctx *c, double courant, double newton_tol, d
     auto newton_residual = [&](cudaGraphConditionalHandle h, int first) -> int {
         TRY(gm_derivative(c, c->q, c->R, newton_precision(c)));
         if (g.Rm) TRY(gm_derivative(c, c->q, g.Rm, c->precision));
-        k_newton_residual<<<g.nchunks, KRYLOV_BLOCK, 0, c->stream>>>(C, g.U, c->U0, c->R, gb, c->seg, c->st, fd_rel,
+        k_newton_residual<<<c->npieces, KRYLOV_BLOCK, 0, c->stream>>>(C, g.U, c->U0, c->R, gb, c->st, fd_rel,
                                                                      newton_tol, krylov_tol, first, g.r, h);
         CU(cudaGetLastError());
         c->launches += 1;
@@ -2544,13 +2518,7 @@ static int enqueue_implicit_step(tg_ctx *c, double courant, double newton_tol, d
     }
     TRY(while_end(c, newton));
     // residual of the last derivative (advance.c:188), time, iteration and the run loop's tests
-    TRY(run_pieces(c, 1));
-    {
-        Launch l(c, TG_PROF_REDUCE);
-        k_inst_end<<<c->ninst, INST_BLOCK, 0, c->stream>>>(c->seg, c->part_sum, 1, c->st);
-        k_count_active<<<1, 256, 0, c->stream>>>(c->ninst, c->st);
-    }
-    CU(cudaGetLastError());
+    TRY(run_step_end(c, 1, 0, courant));
     return TG_OK;
 }
 
@@ -2907,7 +2875,7 @@ extern "C" int tg_part_residual_sums(tg_ctx *c, double *sums)
     CU(cudaStreamSynchronize(c->stream));
     for (int k = 0; k < 5; k++) {
         double t = 0;
-        for (int p = 0; p < c->npieces; p++) t += part[5 * (size_t)p + k];
+        for (int p = 0; p < c->npieces; p++) t += part[(size_t)k * c->npieces + p];
         sums[k] = t;
     }
     return TG_OK;

@@ -74,9 +74,20 @@ struct Sizes {
 };
 
 // Instances packed in one arena (a single mesh is one instance). Inner cells of instance i are
-// [inst_cell_off[i], inst_cell_off[i+1]); reductions run over "pieces", cell ranges of at most
-// PIECE cells that never straddle two instances, first per piece, then per instance in piece order.
-constexpr int PIECE = 4096;
+// [inst_cell_off[i], inst_cell_off[i+1]); reductions run over "pieces", cell ranges that never
+// straddle two instances, one block each, and then over the instance's pieces in order: deterministic,
+// and the same bits for an instance alone or in a batch. A piece is PIECE_CELLS cells (one a thread, so
+// that a small mesh still spreads over the SMs: 16 k cells took 4 blocks with pieces of 4096) up
+// to PIECE_COUNT pieces an instance (two blocks on each of 148 SMs); larger instances get larger
+// pieces, so that the one block that finishes last can sum an instance's partials.
+constexpr int PIECE_CELLS = 256;
+constexpr int PIECE_COUNT = 296;
+inline int piece_cells(long cells)
+{
+    const long per = (cells + PIECE_COUNT - 1) / PIECE_COUNT;
+    const long n = (per + PIECE_CELLS - 1) / PIECE_CELLS * PIECE_CELLS;
+    return (int)(n > 0 ? n : PIECE_CELLS);
+}
 
 struct Segments {
     int ninst;
@@ -86,6 +97,7 @@ struct Segments {
     const int *piece_beg;      // [npieces + 1]
     const int *inst_piece_off; // [ninst + 1]
     const double *sum_volume;  // [ninst]
+    int *ticket;               // [ninst] pieces of an instance that have finished the current pass (0 between)
 };
 
 // Per-instance step bookkeeping in device memory, so whole steps replay from a CUDA graph and
@@ -103,7 +115,7 @@ struct Steps {
     int *max_iter;
     int *active;       // updates and clocks of an inactive instance stand still
     int *fail;         // nonzero once the instance's time step or residual was non-finite (it stops)
-    int *num_active;   // active instances after the last step
+    int *num_active;   // active instances (the host sets it with `active`, an instance that stops counts down)
     int *error;        // nonzero once a non-finite step or norm was seen
     int use_max_time;  // clip by max_time - time instead of max_step
 };

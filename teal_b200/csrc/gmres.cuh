@@ -43,32 +43,19 @@ enum GmresControl {
 // bound keeps every device loop of the step graph finite
 constexpr int NEWTON_LOOP_LIMIT = 1000;
 
-// Cell chunks of the Krylov vectors: ranges of cells that never straddle two instances, one block
-// each. A chunk is KRYLOV_BLOCK cells (one per thread, so the vector being orthogonalised stays in
-// registers) up to KRYLOV_CHUNKS chunks an instance, two resident blocks on each of 148 SMs; larger
-// instances get larger chunks, so that one block can still sum an instance's partials.
-constexpr int KRYLOV_BLOCK = 256;
-constexpr int KRYLOV_CHUNKS = 296;
+// threads of a block over one piece: one cell each in pieces of PIECE_CELLS, so that the vector being
+// orthogonalised stays in registers
+constexpr int KRYLOV_BLOCK = PIECE_CELLS;
 // basis vectors per shared-memory accumulator tile, and loaded together
 constexpr int KRYLOV_TILE = 64;
 constexpr int KRYLOV_GROUP = 4;
-
-inline int krylov_chunk(long cells)
-{
-    const long per = (cells + KRYLOV_CHUNKS - 1) / KRYLOV_CHUNKS;
-    return (int)((per + KRYLOV_BLOCK - 1) / KRYLOV_BLOCK * KRYLOV_BLOCK);
-}
 
 struct GmresBatch {
     int dim;    // Krylov dimension
     int scn;    // doubles per instance block of `sc`
     int ninst;
-    int nchunks;
-    const int *__restrict__ cell_inst;
-    const int *__restrict__ chunk_beg;       // [nchunks + 1]
-    const int *__restrict__ inst_chunk_off;  // [ninst + 1]
-    double *part;  // [2 dim + 1][nchunks] partial sums of the chunks
-    int *ticket;   // [ninst] chunks of the instance that have finished the current pass
+    Segments seg;
+    double *part;  // [2 dim + 1][pieces] partial sums
     double *sc;    // [ninst][scn]
     int *flag;     // [GF_COUNT][ninst]
     int *ctl;      // [GC_COUNT]
@@ -91,41 +78,11 @@ __host__ __device__ inline int gmres_scn(int dim)
     return GS_HEAD + (dim + 1) * dim + 4 * dim + 2 + dim * dim;
 }
 
-// Whether this block is the last one of its instance to finish the current pass: its chunk's
-// partials are then visible to it with those of all other chunks. The same answer in every thread.
-__device__ __forceinline__ bool last_of_instance(const GmresBatch &gb, int inst)
+// One warp's sum of row v of the partial sums over the instance's pieces, in every lane
+__device__ __forceinline__ double sum_pieces(const GmresBatch &gb, int inst, int v, int lane)
 {
-    __shared__ int last;
-    __threadfence();  // this thread's partials before the ticket
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const int n = gb.inst_chunk_off[inst + 1] - gb.inst_chunk_off[inst];
-        last = atomicAdd(gb.ticket + inst, 1) == n - 1;
-        if (last) {
-            gb.ticket[inst] = 0;  // for the next pass
-        }
-    }
-    __syncthreads();
-    if (last) {
-        __threadfence();
-    }
-    return last != 0;
-}
-
-// One warp's sum of partial-sum row v over the instance's chunks, in every lane
-__device__ __forceinline__ double sum_chunks(const GmresBatch &gb, int inst, int v, int lane)
-{
-    const int beg = gb.inst_chunk_off[inst], end = gb.inst_chunk_off[inst + 1];
-    const double *p = gb.part + (size_t)v * gb.nchunks;
-    double t = 0;
-    for (int c = beg + lane; c < end; c += 32) {
-        t += __ldcg(p + c);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        t += __shfl_xor_sync(0xffffffffu, t, o);
-    }
-    return t;
+    const int beg = gb.seg.inst_piece_off[inst], end = gb.seg.inst_piece_off[inst + 1];
+    return sum_partials(gb.part + (size_t)v * gb.seg.npieces + beg, end - beg, lane);
 }
 
 // An instance has finished the current Newton iteration or Arnoldi column and goes on or not. True in
@@ -164,7 +121,6 @@ __global__ void __launch_bounds__(KRYLOV_BLOCK) k_newton_begin(GmresBatch gb, St
         gb.arnoldi(i) = 0;
         gb.m(i) = 0;
         gb.iter(i) = 0;
-        gb.ticket[i] = 0;
         if (on) {
             gb.s(i)[GS_STEP] = st.step[i];
             atomicAdd(&n, 1);
@@ -187,18 +143,18 @@ __global__ void __launch_bounds__(KRYLOV_BLOCK) k_newton_begin(GmresBatch gb, St
 //   loop test (advance.c:162-165): iterate while |r| > tol |r0| and within 128 (cells + 1) iterations;
 //   a non-finite norm marks the instance failed;
 //   an instance that iterates starts its GMRES cycle (gmres.c:68-83): rhs = (norm, 0, ...), Arnoldi on.
-// 360 bytes a cell are read and written once; the rest is latency (a ticket and a sum over chunks).
+// 360 bytes a cell are read and written once; the rest is latency (a ticket and a sum over the pieces).
 __global__ void __launch_bounds__(KRYLOV_BLOCK) k_newton_residual(int C, const double *__restrict__ U,
                                                                   const double *__restrict__ U0,
                                                                   const double *__restrict__ R, GmresBatch gb,
-                                                                  Segments seg, Steps st, double fd_rel,
+                                                                  Steps st, double fd_rel,
                                                                   double newton_tol, double krylov_tol, int first,
                                                                   double *__restrict__ r,
                                                                   cudaGraphConditionalHandle h)
 {
     __shared__ double sh[KRYLOV_BLOCK / 32];
-    const int beg = gb.chunk_beg[blockIdx.x], end = gb.chunk_beg[blockIdx.x + 1];
-    const int inst = gb.cell_inst[beg];
+    const int beg = gb.seg.piece_beg[blockIdx.x], end = gb.seg.piece_beg[blockIdx.x + 1];
+    const int inst = gb.seg.cell_inst[beg];
     if (!gb.newton(inst)) {
         return;
     }
@@ -220,13 +176,13 @@ __global__ void __launch_bounds__(KRYLOV_BLOCK) k_newton_residual(int C, const d
     uu = block_sum<KRYLOV_BLOCK>(uu, sh);
     if (threadIdx.x == 0) {
         gb.part[blockIdx.x] = rr;
-        gb.part[gb.nchunks + blockIdx.x] = uu;
+        gb.part[gb.seg.npieces + blockIdx.x] = uu;
     }
-    if (!last_of_instance(gb, inst) || threadIdx.x >= 32) {
+    if (!last_of_instance(gb.seg, inst) || threadIdx.x >= 32) {
         return;
     }
-    const double norm = sqrt(sum_chunks(gb, inst, 0, threadIdx.x));
-    const double cons = sqrt(sum_chunks(gb, inst, 1, threadIdx.x));
+    const double norm = sqrt(sum_pieces(gb, inst, 0, threadIdx.x));
+    const double cons = sqrt(sum_pieces(gb, inst, 1, threadIdx.x));
     if (threadIdx.x != 0) {
         return;
     }
@@ -242,7 +198,7 @@ __global__ void __launch_bounds__(KRYLOV_BLOCK) k_newton_residual(int C, const d
         on = false;
     }
     else {
-        const long max_iter = 128L * (seg.inst_cell_off[inst + 1] - seg.inst_cell_off[inst] + 1);
+        const long max_iter = 128L * (gb.seg.inst_cell_off[inst + 1] - gb.seg.inst_cell_off[inst] + 1);
         on = norm > s[GS_TOL_NORM] && gb.iter(inst) < max_iter;
     }
     gb.newton(inst) = on;
@@ -277,7 +233,7 @@ __global__ void k_newton_update(int C, int N, double *__restrict__ U, const doub
     if (c >= C) {
         return;
     }
-    const int i = gb.cell_inst[c];
+    const int i = gb.seg.cell_inst[c];
     if (!gb.newton(i)) {
         return;
     }
@@ -330,7 +286,7 @@ __global__ void k_krylov_vector(int C, int N, const double *__restrict__ U, cons
     if (c >= C) {
         return;
     }
-    const int i = gb.cell_inst[c];
+    const int i = gb.seg.cell_inst[c];
     const int k = gb.ctl[GC_K];
     if (!gb.arnoldi(i)) {
         return;
@@ -383,8 +339,8 @@ __global__ void __launch_bounds__(KRYLOV_BLOCK, 2) k_arnoldi_dots(int C, const d
 {
     constexpr int WARPS = KRYLOV_BLOCK / 32;
     __shared__ double acc[WARPS][2 * KRYLOV_TILE];
-    const int beg = gb.chunk_beg[blockIdx.x], end = gb.chunk_beg[blockIdx.x + 1];
-    const int inst = gb.cell_inst[beg];
+    const int beg = gb.seg.piece_beg[blockIdx.x], end = gb.seg.piece_beg[blockIdx.x + 1];
+    const int inst = gb.seg.cell_inst[beg];
     if (!gb.arnoldi(inst)) {
         return;
     }
@@ -452,17 +408,17 @@ __global__ void __launch_bounds__(KRYLOV_BLOCK, 2) k_arnoldi_dots(int C, const d
                 t += acc[q][i];
             }
             const int row = i0 + (i >> 1);
-            gb.part[(size_t)((i & 1) ? dim + row : row) * gb.nchunks + blockIdx.x] = t;
+            gb.part[(size_t)((i & 1) ? dim + row : row) * gb.seg.npieces + blockIdx.x] = t;
         }
         __syncthreads();
     }
-    if (!last_of_instance(gb, inst)) {
+    if (!last_of_instance(gb.seg, inst)) {
         return;
     }
     for (int i = warp; i < 2 * k + 1; i += WARPS) {
         const bool is_t = i <= k;
         const int row = is_t ? i : i - (k + 1);
-        const double t = sum_chunks(gb, inst, is_t ? row : dim + row, lane);
+        const double t = sum_pieces(gb, inst, is_t ? row : dim + row, lane);
         if (lane == 0) {
             *(is_t ? gb.H(inst, row, k) : gb.G(inst, k) + row) = t;
         }
@@ -488,8 +444,8 @@ __global__ void __launch_bounds__(KRYLOV_BLOCK) k_arnoldi_update(int C, const do
 {
     __shared__ double sh[KRYLOV_BLOCK / 32];
     __shared__ int stop;
-    const int beg = gb.chunk_beg[blockIdx.x], end = gb.chunk_beg[blockIdx.x + 1];
-    const int inst = gb.cell_inst[beg];
+    const int beg = gb.seg.piece_beg[blockIdx.x], end = gb.seg.piece_beg[blockIdx.x + 1];
+    const int inst = gb.seg.cell_inst[beg];
     if (!gb.arnoldi(inst)) {
         return;
     }
@@ -521,12 +477,12 @@ __global__ void __launch_bounds__(KRYLOV_BLOCK) k_arnoldi_update(int C, const do
     if (threadIdx.x == 0) {
         gb.part[blockIdx.x] = t;
     }
-    if (!last_of_instance(gb, inst)) {
+    if (!last_of_instance(gb.seg, inst)) {
         return;
     }
     double *cs = gb.cs(inst), *sn = gb.sn(inst), *rhs = gb.rhs(inst), *coef = gb.coef(inst);
     if (threadIdx.x < 32) {
-        const double norm = sqrt(sum_chunks(gb, inst, 0, threadIdx.x));
+        const double norm = sqrt(sum_pieces(gb, inst, 0, threadIdx.x));
         if (threadIdx.x == 0) {
             *gb.H(inst, k + 1, k) = norm;
             double top = *gb.H(inst, 0, k);

@@ -7,8 +7,8 @@
 // derivative, the volumes and the result are the caller's device buffers, and the partial sums go to
 // a fixed array compiled into this library (one copy per device).
 //
-// The reduction is the same as the context path's (per piece of PIECE cells, one block sums
-// volume * r^2 per variable; one block of INST_BLOCK threads sums the pieces and takes
+// The reduction is the same as the context path's (k_step_end: per piece of piece_cells(num_cells) cells,
+// one block sums volume * r^2 per variable; one warp per variable sums the pieces and takes
 // sqrt(sum / sum_volume)), with the same loop order, so both give the same bits.
 #include <cuda_runtime.h>
 
@@ -25,28 +25,24 @@ int tg_record_error(int code, const char *msg);  // sets tg_last_error (context.
 
 namespace {
 
-constexpr int NA_BLOCK = BLOCK;         // threads per piece, as k_piece_reduce
-constexpr int NA_FINISH_BLOCK = 128;    // threads of the finishing block, as k_inst_end
-constexpr long NA_MAX_PIECES = (long)TG_NOALLOC_MAX_CELLS / PIECE;
+constexpr int NA_BLOCK = BLOCK;         // threads per piece, as k_step_end
+constexpr int NA_FINISH_BLOCK = 5 * 32; // a warp per variable
 constexpr int NA_MAX_DEVICES = 64;
-
-static_assert((long)TG_NOALLOC_MAX_CELLS % PIECE == 0, "the cell limit is a whole number of pieces");
 
 }  // namespace
 
-// partial sums, [piece][5]: 16384 pieces x 5 doubles = 640 KiB per device. Every slot the finishing
-// kernel reads is written by the partial kernel of the same call, so nothing has to start at zero.
-static __device__ __align__(256) double g_noalloc_partials[5 * NA_MAX_PIECES];
+// partial sums, [5][pieces]: at most PIECE_COUNT pieces (12 KiB) per device. Every slot the finishing kernel
+// reads is written by the partial kernel of the same call, so nothing has to start at zero.
+static __device__ __align__(256) double g_noalloc_partials[5 * PIECE_COUNT];
 
-// one block per piece of PIECE cells: partials[p][k] = sum over the piece of volume * r_k^2
-__global__ void __launch_bounds__(NA_BLOCK) k_noalloc_residual_pieces(int C, const double *__restrict__ deriv,
+// one block per piece of `per` cells: partials[k][p] = sum over the piece of volume * r_k^2
+__global__ void __launch_bounds__(NA_BLOCK) k_noalloc_residual_pieces(int C, int per, const double *__restrict__ deriv,
                                                                       const double *__restrict__ volume,
                                                                       double *__restrict__ partials)
 {
-    __shared__ double sh[NA_BLOCK / 32];
-    const int beg = blockIdx.x * PIECE;
-    const int end = min(C, beg + PIECE);
-    double t[5] = {0, 0, 0, 0, 0};
+    const int beg = blockIdx.x * per;
+    const int end = min(C, beg + per);
+    double t[6] = {0, 0, 0, 0, 0, DBL_MAX};
     for (int c = beg + threadIdx.x; c < end; c += NA_BLOCK) {
         double v = volume[c];
 #pragma unroll
@@ -55,34 +51,22 @@ __global__ void __launch_bounds__(NA_BLOCK) k_noalloc_residual_pieces(int C, con
             t[k] += v * (r * r);
         }
     }
-#pragma unroll
-    for (int k = 0; k < 5; k++) {
-        double sum = block_sum<NA_BLOCK>(t[k], sh);
-        if (threadIdx.x == 0) {
-            partials[5 * blockIdx.x + k] = sum;
-        }
+    const double x = block_reduce6(t);
+    if (threadIdx.x < 5) {
+        partials[threadIdx.x * gridDim.x + blockIdx.x] = x;
     }
 }
 
-// one block: residual[k] = sqrt(sum over pieces / sum_volume)
+// one block, a warp per variable: residual[k] = sqrt(sum over pieces / sum_volume)
 __global__ void __launch_bounds__(NA_FINISH_BLOCK) k_noalloc_residual_finish(int npieces,
                                                                              const double *__restrict__ partials,
                                                                              double sum_volume,
                                                                              double *__restrict__ residual)
 {
-    __shared__ double sh[NA_FINISH_BLOCK / 32];
-    double res[5];
-    for (int k = 0; k < 5; k++) {
-        double t = 0;
-        for (int p = threadIdx.x; p < npieces; p += NA_FINISH_BLOCK) {
-            t += partials[5 * p + k];
-        }
-        res[k] = block_sum<NA_FINISH_BLOCK>(t, sh);
-    }
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < 5; k++) {
-            residual[k] = sqrt(res[k] / sum_volume);
-        }
+    const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const double t = sum_partials(partials + (size_t)k * npieces, npieces, lane);
+    if (lane == 0) {
+        residual[k] = sqrt(t / sum_volume);
     }
 }
 
@@ -165,9 +149,10 @@ extern "C" int tg_residual_noalloc(const double *derivative, const double *volum
         return status;
     }
     cudaStream_t s = (cudaStream_t)stream;
-    const int npieces = (num_cells + PIECE - 1) / PIECE;
+    const int per = piece_cells(num_cells);
+    const int npieces = (int)(((long)num_cells + per - 1) / per);
     if (npieces > 0) {
-        k_noalloc_residual_pieces<<<npieces, NA_BLOCK, 0, s>>>(num_cells, derivative, volume, partials);
+        k_noalloc_residual_pieces<<<npieces, NA_BLOCK, 0, s>>>(num_cells, per, derivative, volume, partials);
     }
     k_noalloc_residual_finish<<<1, NA_FINISH_BLOCK, 0, s>>>(npieces, partials, sum_volume, residual);
     cudaError_t e = cudaGetLastError();
