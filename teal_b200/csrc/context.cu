@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -12,6 +13,8 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "../../include/teal_b200.h"
@@ -256,6 +259,7 @@ struct tg_ctx {
     size_t aos_len = 0;
     double *pinned = nullptr;  // pinned host staging buffer
     size_t pinned_len = 0;
+    std::vector<cudaEvent_t> read_ev;  // chunks of a staged read-back
     bool prepared = false;     // U0, dtc and the piece minima valid for the resident state
 
     // implicit solver workspace (allocated on first use)
@@ -317,6 +321,11 @@ static double &hd_at(tg_ctx *c, int field, int i) { return c->hd[(size_t)field *
 static int &hi_at(tg_ctx *c, int field, int i) { return c->hi[(size_t)field * c->ninst + i]; }
 static int &hi_num_active(tg_ctx *c) { return c->hi[(size_t)SI_COUNT * c->ninst]; }
 static int &hi_error(tg_ctx *c) { return c->hi[(size_t)SI_COUNT * c->ninst + 1]; }
+// the step arrays lie in one block (doubles, then ints), so that they move in one copy
+static size_t steps_bytes(const tg_ctx *c)
+{
+    return (sizeof(double) * SD_COUNT + sizeof(int) * SI_COUNT) * (size_t)c->ninst + 2 * sizeof(int);
+}
 
 static const double LSERK_ALPHA[3][6][7] = {
     // tabulated low-storage RK coefficients, teal's table (src/simulation/advance.c:50-75)
@@ -373,7 +382,7 @@ static void free_ctx(tg_ctx *c)
                     c->volume, c->proj, c->eps2, c->gb.area, c->gb.basis, c->gb.offl, c->gb.offr, c->gb.corr,
                     c->gb.slot_w, c->gb.slot_off, c->gb.area32, c->gb.basis32, c->gb.offl32, c->gb.offr32,
                     c->gb.corr32, c->gb.tile64, c->gb.tile32, c->gb.toff64, c->gb.toff32, c->q, c->U0, c->R, c->qs, c->grad, c->G,
-                    c->dtc, c->part_min, c->part_sum, c->sd, c->si, c->aos, c->rowmap, c->cell_inst,
+                    c->dtc, c->part_min, c->part_sum, c->sd, c->aos, c->rowmap, c->cell_inst,
                     c->inst_cell_off, c->piece_beg, c->inst_piece_off, c->ticket, c->sum_volume, c->src_avg,
                     c->send_rows, c->send_q, c->recv_q, c->send_rec, c->recv_rec};
     for (void *p : ptrs) {
@@ -381,8 +390,8 @@ static void free_ctx(tg_ctx *c)
     }
     free_gmres(c->gm);
     if (c->hd) cudaFreeHost(c->hd);
-    if (c->hi) cudaFreeHost(c->hi);
     if (c->pinned) cudaFreeHost(c->pinned);
+    for (cudaEvent_t e : c->read_ev) cudaEventDestroy(e);
     if (c->io) {
         if (c->io->copy) cudaStreamDestroy(c->io->copy);
         for (cudaEvent_t e : c->io->ev) cudaEventDestroy(e);
@@ -1021,12 +1030,11 @@ static int create_ctx(MeshInput &in, const tg_equations *e, int precision, tg_ct
         TRY(dalloc(&c->part_min, c->npieces));
         TRY(dalloc(&c->part_sum, 5 * (size_t)c->npieces));
         TRY(dalloc(&c->src_avg, 5 * (size_t)c->ninst));
-        TRY(dalloc(&c->sd, (size_t)SD_COUNT * c->ninst));
-        TRY(dalloc(&c->si, (size_t)SI_COUNT * c->ninst + 2));
-        CU(cudaMallocHost(&c->hd, sizeof(double) * SD_COUNT * c->ninst));
-        CU(cudaMallocHost(&c->hi, sizeof(int) * (SI_COUNT * c->ninst + 2)));
-        memset(c->hd, 0, sizeof(double) * SD_COUNT * c->ninst);
-        memset(c->hi, 0, sizeof(int) * (SI_COUNT * c->ninst + 2));
+        TRY(dalloc(&c->sd, steps_bytes(c) / sizeof(double)));
+        c->si = reinterpret_cast<int *>(c->sd + (size_t)SD_COUNT * c->ninst);
+        CU(cudaMallocHost(&c->hd, steps_bytes(c)));
+        c->hi = reinterpret_cast<int *>(c->hd + (size_t)SD_COUNT * c->ninst);
+        memset(c->hd, 0, steps_bytes(c));
         for (int i = 0; i < c->ninst; i++) {
             hd_at(c, SD_MAX_STEP, i) = DBL_MAX;
             hd_at(c, SD_MAX_TIME, i) = DBL_MAX;
@@ -1035,8 +1043,7 @@ static int create_ctx(MeshInput &in, const tg_equations *e, int precision, tg_ct
             hi_at(c, SI_ACTIVE, i) = 1;
         }
         // the device copy starts as the host mirror (error word clear)
-        CU(cudaMemcpyAsync(c->sd, c->hd, sizeof(double) * SD_COUNT * c->ninst, cudaMemcpyHostToDevice, st));
-        CU(cudaMemcpyAsync(c->si, c->hi, sizeof(int) * (SI_COUNT * c->ninst + 2), cudaMemcpyHostToDevice, st));
+        CU(cudaMemcpyAsync(c->sd, c->hd, steps_bytes(c), cudaMemcpyHostToDevice, st));
         int n = c->ninst;
         c->st = Steps{c->sd + SD_TIME * n,     c->sd + SD_STEP * n,      c->sd + SD_STEP0 * n,
                       c->sd + SD_MAX_STEP * n, c->sd + SD_MAX_TIME * n,  c->sd + SD_THRESHOLD * n,
@@ -1333,9 +1340,51 @@ static int d2h(tg_ctx *c, double *dst, const double *src, size_t n)
         return TG_OK;
     }
     TRY(ensure_pinned(c, n));
-    CU(cudaMemcpyAsync(c->pinned, src, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    // Large pageable arrays: the host's copy out of the staging buffer (and the page faults of a fresh
+    // array) takes several times the transfer, so it runs on READ_THREADS threads, each chunk as soon
+    // as it has arrived.
+    constexpr int READ_THREADS = 4;
+    constexpr size_t READ_CHUNK = (size_t)1 << 17;  // doubles: 1 MiB
+    const int chunks = (int)((n + READ_CHUNK - 1) / READ_CHUNK);
+    if (chunks < 2) {
+        CU(cudaMemcpyAsync(c->pinned, src, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+        CU(cudaStreamSynchronize(c->stream));
+        memcpy(dst, c->pinned, n * sizeof(double));
+        return TG_OK;
+    }
+    while ((int)c->read_ev.size() < chunks) {
+        cudaEvent_t e;
+        CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        c->read_ev.push_back(e);
+    }
+    auto span = [&](int k) { return std::min(READ_CHUNK, n - (size_t)k * READ_CHUNK); };
+    for (int k = 0; k < chunks; k++) {
+        const size_t o = (size_t)k * READ_CHUNK;
+        CU(cudaMemcpyAsync(c->pinned + o, src + o, span(k) * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+        CU(cudaEventRecord(c->read_ev[k], c->stream));
+    }
+    std::atomic<int> next(0), failed(0);
+    auto copy = [&]() {
+        if (cudaSetDevice(c->device) != cudaSuccess) failed = 1;
+        for (int k; !failed && (k = next++) < chunks;) {
+            if (cudaEventSynchronize(c->read_ev[k]) != cudaSuccess) {
+                failed = 1;
+                break;
+            }
+            const size_t o = (size_t)k * READ_CHUNK;
+            memcpy(dst + o, c->pinned + o, span(k) * sizeof(double));
+        }
+    };
+    std::vector<std::thread> threads;
+    try {
+        for (int t = 1; t < std::min(READ_THREADS, chunks); t++) threads.emplace_back(copy);
+    }
+    catch (const std::system_error &) {  // no more threads: fewer, or this one alone
+    }
+    copy();
+    for (std::thread &t : threads) t.join();
     CU(cudaStreamSynchronize(c->stream));
-    memcpy(dst, c->pinned, n * sizeof(double));
+    if (failed) return fail(TG_ERR_CUDA, "reading the device's rows back failed");
     return TG_OK;
 }
 
@@ -1766,10 +1815,15 @@ static int run_prepare(tg_ctx *c)
 
 // ---- step bookkeeping transfers ---------------------------------------------------------------
 
+static int read_steps_async(tg_ctx *c)
+{
+    CU(cudaMemcpyAsync(c->hd, c->sd, steps_bytes(c), cudaMemcpyDeviceToHost, c->stream));
+    return TG_OK;
+}
+
 static int read_steps(tg_ctx *c)
 {
-    CU(cudaMemcpyAsync(c->hd, c->sd, sizeof(double) * SD_COUNT * c->ninst, cudaMemcpyDeviceToHost, c->stream));
-    CU(cudaMemcpyAsync(c->hi, c->si, sizeof(int) * (SI_COUNT * c->ninst + 2), cudaMemcpyDeviceToHost, c->stream));
+    TRY(read_steps_async(c));
     CU(cudaStreamSynchronize(c->stream));
     return TG_OK;
 }
@@ -1778,8 +1832,7 @@ static int write_steps(tg_ctx *c)
 {
     hi_num_active(c) = 0;
     for (int i = 0; i < c->ninst; i++) hi_num_active(c) += hi_at(c, SI_ACTIVE, i) != 0;
-    CU(cudaMemcpyAsync(c->sd, c->hd, sizeof(double) * SD_COUNT * c->ninst, cudaMemcpyHostToDevice, c->stream));
-    CU(cudaMemcpyAsync(c->si, c->hi, sizeof(int) * (SI_COUNT * c->ninst + 2), cudaMemcpyHostToDevice, c->stream));
+    CU(cudaMemcpyAsync(c->sd, c->hd, steps_bytes(c), cudaMemcpyHostToDevice, c->stream));
     return TG_OK;
 }
 
@@ -1827,8 +1880,8 @@ extern "C" int tg_derivative(tg_ctx *c, const double *prim, double *deriv, doubl
     TRY(launch_cell<0>(c, 0.0, 0, q, c->R));
     k_soa5_to_aos<<<grid_of(c->s.C), BLOCK, 0, c->stream>>>(c->s.C, c->R, c->aos);
     CU(cudaGetLastError());
+    TRY(read_steps_async(c));
     TRY(d2h(c, deriv, c->aos, 5 * (size_t)c->s.C));
-    TRY(read_steps(c));
     TRY(check_error(c));
     return TG_OK;
 }
@@ -2228,8 +2281,6 @@ static int run_instances(tg_ctx *c, int method, const void *context, double cour
         TRY(check_error(c));
         if (hi_num_active(c) == 0) break;
     }
-    TRY(read_steps(c));
-    TRY(check_error(c));
     c->prepared = false;  // cells of stopped instances carry no current step estimate
     return TG_OK;
 }
