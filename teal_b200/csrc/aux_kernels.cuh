@@ -132,7 +132,11 @@ __global__ void __launch_bounds__(BLOCK) k_step_end(Segments seg, int C, const d
                                                     double courant, Steps st)
 {
     __shared__ double s_res[6];
+    let_next_start();
     const int i = seg.cell_inst[seg.piece_beg[blockIdx.x]];
+    wait_for_previous();
+    dtc = after_wait(dtc);
+    R = after_wait(R);
     if (advance && !st.active[i]) {
         return;
     }

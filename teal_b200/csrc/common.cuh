@@ -14,6 +14,28 @@ namespace tg {
 enum DeviceError { ERR_NONFINITE = 1, ERR_TIMEOUT = 2, ERR_LOOP_LIMIT = 4 };
 
 constexpr int BLOCK = 256;
+
+// ---- programmatic dependent launch -------------------------------------------------------------
+//
+// A kernel launched with launch_next (launch.cuh) may start while the kernel before it drains: its blocks
+// read what no kernel writes (connectivity, geometry) and then wait for that kernel to complete. The
+// pointers of everything else are passed through after_wait, so that no load of it, read-only ones
+// included, can be moved above the wait. Every thread of every block waits, so that completion carries
+// over from one kernel to the next.
+__device__ __forceinline__ void let_next_start()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void wait_for_previous()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename T>
+__device__ __forceinline__ T *after_wait(T *p)
+{
+    asm volatile("" : "+l"(p)::"memory");
+    return p;
+}
 constexpr int FACE_BLOCK = TG_FACE_BLOCK;
 constexpr int FACE_MINB = TG_FACE_MINB;
 constexpr int FACE_MINB_EULER = TG_FACE_MINB_EULER;

@@ -1482,9 +1482,8 @@ static int run_boundary(tg_ctx *c, double *q, bool masked = false)
         CU(launch_boundary_exact(a, c->stream));
     }
     else {
-        k_boundary<false><<<grid_of(nbf), BLOCK, 0, c->stream>>>(c->s, c->lr, c->gb.basis, c->bface_ent, c->bkind,
-                                                                 c->bctx, q, c->prop[0], c->cell_inst,
-                                                                 masked ? c->st.active : nullptr);
+        launch_next(k_boundary<false>, dim3(grid_of(nbf)), dim3(BLOCK), c->stream, c->s, c->lr, c->gb.basis,
+                    c->bface_ent, c->bkind, c->bctx, q, c->prop[0], c->cell_inst, masked ? c->st.active : nullptr);
     }
     CU(cudaGetLastError());
     // custom boundaries: their device functions, face by face of each boundary
@@ -1665,7 +1664,8 @@ static void launch_cell_s(tg_ctx *c, double alpha, int last, double *q, double *
                c->source == TG_SOURCE_DEVICE ? c->S : c->src_avg};
     const Sizes s = cell_sizes(c);
     if (s.hi <= s.lo) return;
-    k_cell<MODE, NS, GT, SRC, false><<<(s.hi - s.lo + CELL_BLOCK - 1) / CELL_BLOCK, CELL_BLOCK, 0, c->stream>>>(
+    launch_next(k_cell<MODE, NS, GT, SRC, false>, dim3((s.hi - s.lo + CELL_BLOCK - 1) / CELL_BLOCK), dim3(CELL_BLOCK),
+                c->stream,
         s, c->slot_face, c->slot_cnt, cd, (const GT *)c->G, c->U0, q, Rout, c->seg, c->st, alpha, last,
         props_of(c), c->dtc, src, 0);
 }
@@ -1781,12 +1781,17 @@ static int run_pieces(tg_ctx *c, int res)
 }
 
 // end of a step, or with advance off the residual norm of c->R alone (k_step_end)
-static int run_step_end(tg_ctx *c, int advance, int begin, double courant)
+static int run_step_end(tg_ctx *c, int advance, int begin, double courant, bool after_kernel = true)
 {
     Launch l(c, TG_PROF_REDUCE);
-    k_step_end<<<c->npieces, BLOCK, 0, c->stream>>>(c->seg, c->s.C, c->dtc, c->R, c->volume, c->part_min, c->part_sum,
-                                                    advance, begin, courant, c->st);
-    CU(cudaGetLastError());
+    if (!after_kernel) {  // behind a conditional node
+        k_step_end<<<c->npieces, BLOCK, 0, c->stream>>>(c->seg, c->s.C, c->dtc, c->R, c->volume, c->part_min,
+                                                        c->part_sum, advance, begin, courant, c->st);
+        CU(cudaGetLastError());
+        return TG_OK;
+    }
+    CU(launch_next(k_step_end, dim3(c->npieces), dim3(BLOCK), c->stream, c->seg, c->s.C, c->dtc, c->R, c->volume,
+                   c->part_min, c->part_sum, advance, begin, courant, c->st));
     return TG_OK;
 }
 
@@ -2500,9 +2505,9 @@ static int gm_solve(tg_ctx *c, const GmresBatch &gb)
     k_krylov_vector<<<cb, BLOCK, 0, c->stream>>>(C, c->s.N, g.U, g.r, g.w, gb, c->prop[0], g.V, g.q1);
     CU(cudaGetLastError());
     TRY(gm_derivative(c, g.q1, g.R1, c->precision));
-    k_arnoldi_dots<<<c->npieces, KRYLOV_BLOCK, 0, c->stream>>>(C, g.V, g.R1, g.Rm ? g.Rm : c->R, gb, g.w);
-    k_arnoldi_update<<<c->npieces, KRYLOV_BLOCK, 0, c->stream>>>(C, g.V, gb, g.w, arnoldi.h);
-    CU(cudaGetLastError());
+    CU(launch_next(k_arnoldi_dots, dim3(c->npieces), dim3(KRYLOV_BLOCK), c->stream, C, g.V, g.R1, g.Rm ? g.Rm : c->R, gb,
+                   g.w));
+    CU(launch_next(k_arnoldi_update, dim3(c->npieces), dim3(KRYLOV_BLOCK), c->stream, C, g.V, gb, g.w, arnoldi.h));
     c->launches += 3;
     TRY(while_end(c, arnoldi));
     return TG_OK;
@@ -2547,9 +2552,8 @@ static int enqueue_implicit_step(tg_ctx *c, double courant, double newton_tol, d
     auto newton_residual = [&](cudaGraphConditionalHandle h, int first) -> int {
         TRY(gm_derivative(c, c->q, c->R, newton_precision(c)));
         if (g.Rm) TRY(gm_derivative(c, c->q, g.Rm, c->precision));
-        k_newton_residual<<<c->npieces, KRYLOV_BLOCK, 0, c->stream>>>(C, g.U, c->U0, c->R, gb, c->st, fd_rel,
-                                                                     newton_tol, krylov_tol, first, g.r, h);
-        CU(cudaGetLastError());
+        CU(launch_next(k_newton_residual, dim3(c->npieces), dim3(KRYLOV_BLOCK), c->stream, C, g.U, c->U0, c->R, gb, c->st,
+                       fd_rel, newton_tol, krylov_tol, first, g.r, h));
         c->launches += 1;
         return TG_OK;
     };
@@ -2569,7 +2573,7 @@ static int enqueue_implicit_step(tg_ctx *c, double courant, double newton_tol, d
     }
     TRY(while_end(c, newton));
     // residual of the last derivative (advance.c:188), time, iteration and the run loop's tests
-    TRY(run_step_end(c, 1, 0, courant));
+    TRY(run_step_end(c, 1, 0, courant, false));
     return TG_OK;
 }
 

@@ -218,6 +218,9 @@ __device__ __forceinline__ void face_flux_ns(const Geo &geo, int i, int f, const
 {
     const bool boundary = (f >= s.F_in) && (f < s.F_bd);
     const int2 c = geo.cells(i);
+    wait_for_previous();
+    q = after_wait(q);
+    rec = after_wait(rec);
     double pref = 0.0;
     if constexpr (sizeof(R) == sizeof(float)) {
         pref = pr_ref.of(c.x);
@@ -278,6 +281,9 @@ __device__ __forceinline__ void face_flux(const Geo &geo, int i, int f, const Si
     const int N = s.N;
     const bool boundary = (f >= s.F_in) && (f < s.F_bd);
     const int2 c = geo.cells(i);
+    wait_for_previous();
+    q = after_wait(q);
+    rec = after_wait(rec);
     // FP32 fluxes work with the pressure relative to the instance's reference (Local::dp); the
     // difference is taken in FP64, before the rounding to FP32
     double pref = 0.0;
@@ -348,13 +354,19 @@ __global__ void __launch_bounds__(SIDE_BLOCK, side_minb<R>()) k_face_sides(Sizes
                                                    PressureRefOf<R> pr_ref)
 {
     static_assert(sizeof(R) == 0 || !kExact, "the exact form has no side records");
+    let_next_start();
     const int f = s.lo + blockIdx.x * SIDE_BLOCK + threadIdx.x;
+    const int fc_ = min(f, s.hi - 1);
+    const int2 e = __ldg(g.sides + fc_);
+    const V3<R> n = load_v3(g.basis, s.F, fc_);
+    const R area = __ldg(g.area + fc_);
+    wait_for_previous();
+    q = after_wait(q);
+    side = after_wait(side);
+    rec = after_wait(rec);
     if (f >= s.hi) {
         return;
     }
-    const int2 e = __ldg(g.sides + f);
-    const V3<R> n = load_v3(g.basis, s.F, f);
-    const R area = __ldg(g.area + f);
     double pref = 0.0;
     R pl[5], pr[5];
     if constexpr (sizeof(R) == sizeof(float)) {
@@ -404,8 +416,10 @@ __global__ void __launch_bounds__(FACE_BLOCK, face_minb<R>(NS)) k_face(Sizes s, 
                                                    R *__restrict__ G, PressureRefOf<R> pr_ref)
 {
     static_assert(X == kExact, "exact kernels live in the exact translation units only");
+    let_next_start();
     const int f = s.lo + blockIdx.x * FACE_BLOCK + threadIdx.x;
     if (f >= s.hi) {
+        wait_for_previous();
         return;
     }
     DirectGeo<R> geo{g, s.F, f};
@@ -432,12 +446,17 @@ __global__ void __launch_bounds__(FACE_BLOCK, face_minb<R>(false)) k_face_staged
 {
     static_assert(X == kExact, "exact kernels live in the exact translation units only");
     __shared__ __align__(16) FaceTile<R, ORDER> t;
+    let_next_start();
     const int f0 = s.lo + blockIdx.x * FACE_BLOCK;
     const int n = min(FACE_BLOCK, s.hi - f0);
     if (!t.stage(g, s.F, f0, n, err, polls)) {
+        wait_for_previous();
         return;
     }
-    if (threadIdx.x < n) {
+    if (threadIdx.x >= n) {
+        wait_for_previous();
+    }
+    else {
         face_flux<R, FK, ORDER, FOLD>(t, threadIdx.x, f0 + threadIdx.x, s, q, rec, gamma, G,
                                           pr_ref);
     }

@@ -153,6 +153,11 @@ __global__ void __launch_bounds__(KRYLOV_BLOCK) k_newton_residual(int C, const d
                                                                   cudaGraphConditionalHandle h)
 {
     __shared__ double sh[KRYLOV_BLOCK / 32];
+    let_next_start();
+    wait_for_previous();
+    U = after_wait(U);
+    U0 = after_wait(U0);
+    R = after_wait(R);
     const int beg = gb.seg.piece_beg[blockIdx.x], end = gb.seg.piece_beg[blockIdx.x + 1];
     const int inst = gb.seg.cell_inst[beg];
     if (!gb.newton(inst)) {
@@ -339,6 +344,11 @@ __global__ void __launch_bounds__(KRYLOV_BLOCK, 2) k_arnoldi_dots(int C, const d
 {
     constexpr int WARPS = KRYLOV_BLOCK / 32;
     __shared__ double acc[WARPS][2 * KRYLOV_TILE];
+    let_next_start();
+    wait_for_previous();
+    V = after_wait(V);
+    R1 = after_wait(R1);
+    R = after_wait(R);
     const int beg = gb.seg.piece_beg[blockIdx.x], end = gb.seg.piece_beg[blockIdx.x + 1];
     const int inst = gb.seg.cell_inst[beg];
     if (!gb.arnoldi(inst)) {
@@ -444,6 +454,9 @@ __global__ void __launch_bounds__(KRYLOV_BLOCK) k_arnoldi_update(int C, const do
 {
     __shared__ double sh[KRYLOV_BLOCK / 32];
     __shared__ int stop;
+    let_next_start();
+    wait_for_previous();
+    V = after_wait(V);
     const int beg = gb.seg.piece_beg[blockIdx.x], end = gb.seg.piece_beg[blockIdx.x + 1];
     const int inst = gb.seg.cell_inst[beg];
     if (!gb.arnoldi(inst)) {

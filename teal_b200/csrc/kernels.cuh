@@ -20,12 +20,15 @@ __global__ void k_boundary(Sizes s, const int2 *__restrict__ lr, const double *_
                            const int *__restrict__ cell_inst, const int *__restrict__ active)
 {
     static_assert(X == kExact, "exact kernels live in the exact translation units only");
+    let_next_start();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     int f = s.F_in + i;
+    const int2 c = f < s.F_bd ? lr[f] : make_int2(0, 0);
+    wait_for_previous();
+    q = after_wait(q);
     if (f >= s.F_bd) {
         return;
     }
-    int2 c = lr[f];
     if (active && !active[cell_inst[c.x]]) {
         return;
     }
@@ -91,8 +94,8 @@ __global__ void __launch_bounds__(GRAD_THREADS, SIDES ? GRAD_MINB_SIDES : GRAD_M
     const int v = threadIdx.x / GRAD_CELLS;  // variable of this warp
     const int l = threadIdx.x % GRAD_CELLS;
     const int c = base + min(l, ncell - 1);
-    const double *qv = q + (size_t)v * s.N;
-    double qn[MAX_SLOTS];
+    let_next_start();
+    int row[MIXED ? 1 : MAX_SLOTS];
     if constexpr (MIXED) {
         // the whole tile by bulk copies; its slot count is the tile's largest, so a warp of
         // tetrahedra stops after 4
@@ -133,7 +136,18 @@ __global__ void __launch_bounds__(GRAD_THREADS, SIDES ? GRAD_MINB_SIDES : GRAD_M
         const int *nbr = reinterpret_cast<const int *>(tile_p);
 #pragma unroll
         for (int j = 0; j < MAX_SLOTS; j++) {
-            qn[j] = __ldg(qv + __ldg(nbr + j * GRAD_CELLS + l));
+            row[j] = __ldg(nbr + j * GRAD_CELLS + l);
+        }
+    }
+    // the mesh's part is on its way; the states come from the kernel before this one
+    wait_for_previous();
+    q = after_wait(q);
+    const double *qv = q + (size_t)v * s.N;
+    double qn[MAX_SLOTS];
+    if constexpr (!MIXED) {
+#pragma unroll
+        for (int j = 0; j < MAX_SLOTS; j++) {
+            qn[j] = __ldg(qv + row[j]);
         }
     }
     // the cell's own state does not depend on the tile: its load overlaps the copies
@@ -329,6 +343,10 @@ __global__ void __launch_bounds__(CELL_BLOCK, CELL_MINB) k_cell(Sizes s, const i
                                                 double *__restrict__ dtc, Source src, int two)
 {
     static_assert(X == kExact, "exact kernels live in the exact translation units only");
+    // nothing is read ahead of the wait: the slot indices held across it cost registers (spills at 40)
+    let_next_start();
+    wait_for_previous();
+    G = after_wait(G);
     const int C = s.C, N = s.N;
     int c = s.lo + blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= s.hi) {
@@ -440,11 +458,11 @@ __global__ void __launch_bounds__(CELL_BLOCK, CELL_MINB) k_cell(Sizes s, const i
         return;
     }
     Cons<double> u;
-    u.rho = __ldg(U0 + c) + ((r[0] * alpha) * step);
-    u.m.x = __ldg(U0 + C + c) + ((r[1] * alpha) * step);
-    u.m.y = __ldg(U0 + 2 * C + c) + ((r[2] * alpha) * step);
-    u.m.z = __ldg(U0 + 3 * C + c) + ((r[3] * alpha) * step);
-    u.e = __ldg(U0 + 4 * C + c) + ((r[4] * alpha) * step);
+    u.rho = U0[c] + ((r[0] * alpha) * step);
+    u.m.x = U0[C + c] + ((r[1] * alpha) * step);
+    u.m.y = U0[2 * C + c] + ((r[2] * alpha) * step);
+    u.m.z = U0[3 * C + c] + ((r[3] * alpha) * step);
+    u.e = U0[4 * C + c] + ((r[4] * alpha) * step);
     Prim<double> p = cons_to_prim(u, prop.v[0]);
     store_prim(q, N, c, p);
     if (last) {

@@ -8,6 +8,23 @@
 
 namespace tg {
 
+// Launch of a kernel that waits for the one before it itself (wait_for_previous): it may start while that
+// kernel drains
+template <typename... K, typename... A>
+inline cudaError_t launch_next(void (*kernel)(K...), dim3 grid, dim3 block, cudaStream_t st, const A &...args)
+{
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, K(args)...);
+}
+
 struct FaceLaunch {
     Sizes s;
     const void *geom;  // Geometry<R>*
@@ -41,12 +58,12 @@ inline void launch_face_v(bool staged, const FaceLaunch &a, const Geometry<R> &g
     }
     if constexpr (!NS) {
         if (staged) {
-            k_face_staged<R, FK, ORDER, FOLD, X>
-                <<<grid, FACE_BLOCK, 0, st>>>(a.s, g, a.q, rec, gm, G, a.err, pref, a.polls);
+            launch_next(k_face_staged<R, FK, ORDER, FOLD, X>, grid, dim3(FACE_BLOCK), st, a.s, g, a.q, rec, gm, G,
+                        a.err, pref, a.polls);
             return;
         }
     }
-    k_face<R, FK, NS, ORDER, FOLD, X><<<grid, FACE_BLOCK, 0, st>>>(a.s, g, a.q, rec, gm, mu, pr, G, pref);
+    launch_next(k_face<R, FK, NS, ORDER, FOLD, X>, grid, dim3(FACE_BLOCK), st, a.s, g, a.q, rec, gm, mu, pr, G, pref);
 }
 
 // staged geometry (bulk copies into shared memory) or thread loads without a viscous flux (tuned.h)
@@ -65,9 +82,9 @@ inline cudaError_t launch_face_r(bool ns, int order, bool fold, const FaceLaunch
             if constexpr (sizeof(R) == sizeof(float)) {
                 pref = a.pr_ref;
             }
-            k_face_sides<R, FK><<<(a.s.hi - a.s.lo + SIDE_BLOCK - 1) / SIDE_BLOCK, SIDE_BLOCK, 0, st>>>(
-                a.s, g, a.q, static_cast<const R *>(a.side), rec, R(a.gamma), G, pref);
-            return cudaGetLastError();
+            return launch_next(k_face_sides<R, FK>, dim3((a.s.hi - a.s.lo + SIDE_BLOCK - 1) / SIDE_BLOCK),
+                               dim3(SIDE_BLOCK), st, a.s, g, a.q, static_cast<const R *>(a.side), rec, R(a.gamma), G,
+                               pref);
         }
     }
     const bool staged = !ns && TG_FACE_STAGED_EULER != 0;
