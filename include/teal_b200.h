@@ -429,7 +429,7 @@ int tg_layout(tg_ctx *ctx, const char *name, void *out, long count);
  *   residual    device double[5], written on `stream` (a cudaStream_t; null = legacy default)
  * All three buffers must be 8-byte aligned memory of the current device, or managed memory, else
  * TG_ERR_INVALID (memory of another GPU is refused before any launch).
- * The partial sums go to a fixed 12 KiB array compiled into the library, one per device. num_cells is
+ * The partial sums go to a fixed 24 KiB array compiled into the library, one per device. num_cells is
  * limited to TG_NOALLOC_MAX_CELLS; a larger num_cells returns TG_ERR_INVALID.
  * The first call on each device does a set-up (it looks up that array's device address, which can
  * initialise the device's CUDA context); make that first call before any stream capture. The

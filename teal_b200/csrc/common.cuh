@@ -54,7 +54,12 @@ __host__ __device__ constexpr int side_minb()
     return sizeof(R) == sizeof(float) ? TG_SIDE_MINB_FP32 : TG_SIDE_MINB;
 }
 constexpr int CELL_BLOCK = TG_CELL_BLOCK;
-constexpr int CELL_MINB = TG_CELL_MINB;
+// resident cell-gather blocks per SM, FP64 or FP32 flux records
+template <typename GT>
+__host__ __device__ constexpr int cell_minb()
+{
+    return sizeof(GT) == sizeof(float) ? TG_CELL_MINB_FP32 : TG_CELL_MINB;
+}
 constexpr int GRAD_MINB = TG_GRAD_MINB;
 constexpr int GRAD_MINB_SIDES = TG_GRAD_MINB_SIDES;
 constexpr int REDUCE_BLOCK = 1024;

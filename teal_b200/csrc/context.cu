@@ -262,6 +262,9 @@ struct tg_ctx {
     std::vector<cudaEvent_t> read_ev;  // chunks of a staged read-back
     bool prepared = false;     // U0, dtc and the piece minima valid for the resident state
 
+    // instances the next residuals are evaluated for ([ninst] device flags; null: all), see Mask
+    const int *eval_on = nullptr;
+
     // implicit solver workspace (allocated on first use)
     Gmres gm{};
 
@@ -1478,12 +1481,12 @@ static int run_boundary(tg_ctx *c, double *q, bool masked = false)
     Launch l(c, TG_PROF_BOUNDARY);
     if (is_exact(c)) {
         BoundaryLaunch a{c->s,   c->lr,      c->gb.basis, c->bface_ent, c->bkind, c->bctx, q,
-                         c->prop[0], c->cell_inst, masked ? c->st.active : nullptr};
+                         c->prop[0], c->cell_inst, masked ? c->st.active : c->eval_on};
         CU(launch_boundary_exact(a, c->stream));
     }
     else {
         launch_next(k_boundary<false>, dim3(grid_of(nbf)), dim3(BLOCK), c->stream, c->s, c->lr, c->gb.basis,
-                    c->bface_ent, c->bkind, c->bctx, q, c->prop[0], c->cell_inst, masked ? c->st.active : nullptr);
+                    c->bface_ent, c->bkind, c->bctx, q, c->prop[0], c->cell_inst, masked ? c->st.active : c->eval_on);
     }
     CU(cudaGetLastError());
     // custom boundaries: their device functions, face by face of each boundary
@@ -1501,6 +1504,11 @@ static int run_boundary(tg_ctx *c, double *q, bool masked = false)
         CU(cudaLaunchKernel(c->bd_kernel[b], dim3((n + 127) / 128), dim3(128), args, 0, c->stream));
     }
     return TG_OK;
+}
+
+static Mask mask_of(const tg_ctx *c)
+{
+    return Mask{c->eval_on, c->cell_inst};
 }
 
 // the context's sizes with the work range of its next cell-wise or face-wise launch
@@ -1543,8 +1551,8 @@ static void launch_gradient_s(tg_ctx *c, const Geometry<R> &g, bool fold, bool s
     PressureRefOf<R> pref{};
     if constexpr (sizeof(R) == sizeof(float)) pref = pressure_ref(c);
     auto launch = [&](auto kernel) {
-        kernel<<<grid, GRAD_THREADS, 0, c->stream>>>(s, g, c->eps2, q, rec, c->st.error, c->wait_polls, pref,
-                                                   SideOut<R>{(R *)c->side_rec, c->side_records});
+        launch_next(kernel, grid, dim3(GRAD_THREADS), c->stream, s, g, c->eps2, q, rec, c->st.error, c->wait_polls, pref,
+                    SideOut<R>{(R *)c->side_rec, c->side_records}, mask_of(c));
     };
     switch (c->limiter) {
         case TG_LIMITER_NONE:
@@ -1591,7 +1599,7 @@ static int run_gradient(tg_ctx *c, const double *q, int limiter_override = -1)
     Launch l(c, TG_PROF_GRADIENT);
     if (is_exact(c)) {
         GradientLaunch a{cell_sizes(c), c->g64, c->eps2,  q, (double *)c->grad, c->limiter, fold, !c->full_slots,
-                         c->st.error, c->wait_polls};
+                         c->st.error, c->wait_polls, mask_of(c)};
         cudaError_t e = launch_gradient_exact(a, c->stream);
         c->limiter = saved;
         CU(e);
@@ -1607,7 +1615,7 @@ static int run_gradient(tg_ctx *c, const double *q, int limiter_override = -1)
     return TG_OK;
 }
 
-static int run_face(tg_ctx *c, const double *q)
+static FaceLaunch face_args(tg_ctx *c, const double *q)
 {
     FaceLaunch a;
     a.s = face_sizes(c);
@@ -1620,8 +1628,15 @@ static int run_face(tg_ctx *c, const double *q)
     a.G = c->G;
     a.err = c->st.error;
     a.pr_ref = pressure_ref(c);
+    a.mask = mask_of(c);
     a.side = use_sides(c) ? c->side_rec : nullptr;
     a.polls = c->wait_polls;
+    return a;
+}
+
+static int run_face(tg_ctx *c, const double *q)
+{
+    const FaceLaunch a = face_args(c, q);
     bool ns = c->viscous == TG_VISCOUS_CENTRAL;
     bool fold = fold_psi(c);
     Launch l(c, TG_PROF_FACE);
@@ -1667,7 +1682,7 @@ static void launch_cell_s(tg_ctx *c, double alpha, int last, double *q, double *
     launch_next(k_cell<MODE, NS, GT, SRC, false>, dim3((s.hi - s.lo + CELL_BLOCK - 1) / CELL_BLOCK), dim3(CELL_BLOCK),
                 c->stream,
         s, c->slot_face, c->slot_cnt, cd, (const GT *)c->G, c->U0, q, Rout, c->seg, c->st, alpha, last,
-        props_of(c), c->dtc, src, 0);
+        props_of(c), c->dtc, src, 0, mask_of(c));
 }
 
 template <int MODE, bool NS, typename GT>
@@ -1681,34 +1696,40 @@ static void launch_cell_t(tg_ctx *c, double alpha, int last, double *q, double *
     }
 }
 
+static CellLaunch cell_args(tg_ctx *c, int mode, double alpha, int last, double *q, double *Rout)
+{
+    CellLaunch a;
+    a.mode = mode;
+    a.ns = is_ns(c);
+    a.source = c->source;
+    a.two = (is_exact(c) && c->viscous == TG_VISCOUS_CENTRAL && c->order == 2) ? 1 : 0;
+    a.s = cell_sizes(c);
+    a.slot_face = c->slot_face;
+    a.slot_cnt = c->slot_cnt;
+    a.cd = CellData{c->volume, c->proj, c->eps2};
+    a.G = (const double *)c->G;
+    a.U0 = c->U0;
+    a.q = q;
+    a.Rout = Rout;
+    a.seg = c->seg;
+    a.st = c->st;
+    a.alpha = alpha;
+    a.last = last;
+    a.prop = props_of(c);
+    a.dtc = c->dtc;
+    a.src = Source{{c->src_par[0], c->src_par[1], c->src_par[2], c->src_par[3]},
+                   c->source == TG_SOURCE_DEVICE ? c->S : c->src_avg};
+    a.mask = mask_of(c);
+    return a;
+}
+
 template <int MODE>
 static int launch_cell(tg_ctx *c, double alpha, int last, double *q, double *Rout)
 {
     Launch l(c, TG_PROF_CELL);
     bool ns = is_ns(c);
     if (is_exact(c)) {
-        CellLaunch a;
-        a.mode = MODE;
-        a.ns = ns;
-        a.source = c->source;
-        a.two = (c->viscous == TG_VISCOUS_CENTRAL && c->order == 2) ? 1 : 0;
-        a.s = cell_sizes(c);
-        a.slot_face = c->slot_face;
-        a.slot_cnt = c->slot_cnt;
-        a.cd = CellData{c->volume, c->proj, c->eps2};
-        a.G = (const double *)c->G;
-        a.U0 = c->U0;
-        a.q = q;
-        a.Rout = Rout;
-        a.seg = c->seg;
-        a.st = c->st;
-        a.alpha = alpha;
-        a.last = last;
-        a.prop = props_of(c);
-        a.dtc = c->dtc;
-        a.src = Source{{c->src_par[0], c->src_par[1], c->src_par[2], c->src_par[3]},
-                       c->source == TG_SOURCE_DEVICE ? c->S : c->src_avg};
-        CU(launch_cell_exact(a, c->stream));
+        CU(launch_cell_exact(cell_args(c, MODE, alpha, last, q, Rout), c->stream));
         return TG_OK;
     }
     if (c->precision == TG_PRECISION_FP64) {
@@ -1770,6 +1791,14 @@ static int run_fluxes(tg_ctx *c, double *q, bool masked = false)
     return TG_OK;
 }
 
+// the whole residual of q: mode 0 R into Rout, mode 1 one RK stage
+template <int MODE>
+static int run_residual(tg_ctx *c, double *q, double *Rout, bool masked, double alpha = 0.0, int last = 0)
+{
+    TRY(run_fluxes(c, q, masked));
+    return launch_cell<MODE>(c, alpha, last, q, Rout);
+}
+
 // per-piece reductions of the cell steps (and of V R^2 with `res`)
 static int run_pieces(tg_ctx *c, int res)
 {
@@ -1784,7 +1813,7 @@ static int run_pieces(tg_ctx *c, int res)
 static int run_step_end(tg_ctx *c, int advance, int begin, double courant, bool after_kernel = true)
 {
     Launch l(c, TG_PROF_REDUCE);
-    if (!after_kernel) {  // behind a conditional node
+    if (!after_kernel) {  // behind a conditional node: an ordinary launch
         k_step_end<<<c->npieces, BLOCK, 0, c->stream>>>(c->seg, c->s.C, c->dtc, c->R, c->volume, c->part_min,
                                                         c->part_sum, advance, begin, courant, c->st);
         CU(cudaGetLastError());
@@ -1881,8 +1910,7 @@ extern "C" int tg_derivative(tg_ctx *c, const double *prim, double *deriv, doubl
         q = c->qs;
         TRY(set_rows(c, 0, prim, q));
     }
-    TRY(run_fluxes(c, q));
-    TRY(launch_cell<0>(c, 0.0, 0, q, c->R));
+    TRY(run_residual<0>(c, q, c->R, false));
     k_soa5_to_aos<<<grid_of(c->s.C), BLOCK, 0, c->stream>>>(c->s.C, c->R, c->aos);
     CU(cudaGetLastError());
     TRY(read_steps_async(c));
@@ -1977,8 +2005,7 @@ static int enqueue_explicit_step(tg_ctx *c, int stages, const double *alpha, dou
     for (int i = 0; i < stages; i++) {
         // the residual of stage i at time + alpha_i step (advance.c:100)
         c->t_time = c->st.time, c->t_step = c->st.step, c->t_coef = alpha[i];
-        TRY(run_fluxes(c, c->q, true));
-        TRY(launch_cell<1>(c, alpha[i + 1], i == stages - 1, c->q, c->R));
+        TRY(run_residual<1>(c, c->q, c->R, true, alpha[i + 1], i == stages - 1));
     }
     TRY(run_step_end(c, 1, begin_next, courant));
     return TG_OK;
@@ -2173,8 +2200,7 @@ static int advance_chunked(tg_ctx *c, int stages, const double *alpha, double co
     int i = 0;
     for (; i < stages - 1; i++) {
         c->t_time = c->st.time, c->t_step = c->st.step, c->t_coef = alpha[i];
-        TRY(run_fluxes(c, c->q, true));
-        TRY(launch_cell<1>(c, alpha[i + 1], 0, c->q, c->R));
+        TRY(run_residual<1>(c, c->q, c->R, true, alpha[i + 1], 0));
     }
     // the last stage: sources, boundary ghosts, gradients and the boundary and periodic faces whole,
     // then the inner faces and the cell updates chunk by chunk
@@ -2469,15 +2495,18 @@ static int while_end(tg_ctx *c, WhileLoop &w)
 }
 
 // derivative of a primitive state q (boundary rows refreshed) into Rout, with the kernels of
-// `precision` (the context's own, or FP64 for the FP32-flux form's Newton residuals)
-static int gm_derivative(tg_ctx *c, double *q, double *Rout, int precision)
+// `precision` (the context's own, or FP64 for the FP32-flux form's Newton residuals), for the instances
+// whose flag `which` (GmresFlag) is set
+static int gm_derivative(tg_ctx *c, double *q, double *Rout, int precision, int which)
 {
     // implicit Euler evaluates every residual at the end of the step, time + step (advance.c:144)
     c->t_time = c->st.time, c->t_step = c->st.step, c->t_coef = 1.0;
     const int own = c->precision;
     c->precision = precision;
-    int rc = run_fluxes(c, q);
-    if (rc == TG_OK) rc = launch_cell<0>(c, 0.0, 0, q, Rout);
+    // one mesh is in its loops as long as they run
+    c->eval_on = c->ninst > 1 ? c->gm.flag + (size_t)which * c->ninst : nullptr;
+    const int rc = run_residual<0>(c, q, Rout, false);
+    c->eval_on = nullptr;
     c->precision = own;
     return rc;
 }
@@ -2504,7 +2533,7 @@ static int gm_solve(tg_ctx *c, const GmresBatch &gb)
     // matvec (gmres.c:12-50); it differences two residuals of the same precision (gmres.c:41-46)
     k_krylov_vector<<<cb, BLOCK, 0, c->stream>>>(C, c->s.N, g.U, g.r, g.w, gb, c->prop[0], g.V, g.q1);
     CU(cudaGetLastError());
-    TRY(gm_derivative(c, g.q1, g.R1, c->precision));
+    TRY(gm_derivative(c, g.q1, g.R1, c->precision, GF_ARNOLDI));
     CU(launch_next(k_arnoldi_dots, dim3(c->npieces), dim3(KRYLOV_BLOCK), c->stream, C, g.V, g.R1, g.Rm ? g.Rm : c->R, gb,
                    g.w));
     CU(launch_next(k_arnoldi_update, dim3(c->npieces), dim3(KRYLOV_BLOCK), c->stream, C, g.V, gb, g.w, arnoldi.h));
@@ -2550,8 +2579,8 @@ static int enqueue_implicit_step(tg_ctx *c, double courant, double newton_tol, d
 
     // derivative of the iterate, Newton residual, its norms, the loop test
     auto newton_residual = [&](cudaGraphConditionalHandle h, int first) -> int {
-        TRY(gm_derivative(c, c->q, c->R, newton_precision(c)));
-        if (g.Rm) TRY(gm_derivative(c, c->q, g.Rm, c->precision));
+        TRY(gm_derivative(c, c->q, c->R, newton_precision(c), GF_NEWTON));
+        if (g.Rm) TRY(gm_derivative(c, c->q, g.Rm, c->precision, GF_NEWTON));
         CU(launch_next(k_newton_residual, dim3(c->npieces), dim3(KRYLOV_BLOCK), c->stream, C, g.U, c->U0, c->R, gb, c->st,
                        fd_rel, newton_tol, krylov_tol, first, g.r, h));
         c->launches += 1;

@@ -78,10 +78,11 @@ struct Sizes {
 // straddle two instances, one block each, and then over the instance's pieces in order: deterministic,
 // and the same bits for an instance alone or in a batch. A piece is PIECE_CELLS cells (one a thread, so
 // that a small mesh still spreads over the SMs: 16 k cells took 4 blocks with pieces of 4096) up
-// to PIECE_COUNT pieces an instance (two blocks on each of 148 SMs); larger instances get larger
+// to PIECE_COUNT pieces an instance (four blocks on each of 148 SMs; with two the step end of TGV 128^3
+// took 46 us instead of 36 and a Newton step of 123 k cells 5 % more); larger instances get larger
 // pieces, so that the one block that finishes last can sum an instance's partials.
 constexpr int PIECE_CELLS = 256;
-constexpr int PIECE_COUNT = 296;
+constexpr int PIECE_COUNT = 592;
 inline int piece_cells(long cells)
 {
     const long per = (cells + PIECE_COUNT - 1) / PIECE_COUNT;
@@ -98,6 +99,14 @@ struct Segments {
     const int *inst_piece_off; // [ninst + 1]
     const double *sum_volume;  // [ninst]
     int *ticket;               // [ninst] pieces of an instance that have finished the current pass (0 between)
+};
+
+// Instances a residual is evaluated for (on: null for all): an arena's Newton iterations and Krylov columns
+// leave out the instances that are done with them. The flags do not change while the residual's kernels run.
+struct Mask {
+    const int *on;         // [ninst]
+    const int *cell_inst;  // [C]
+    __device__ __forceinline__ bool leaves_out(int c) const { return on && !on[__ldg(cell_inst + c)]; }
 };
 
 // Per-instance step bookkeeping in device memory, so whole steps replay from a CUDA graph and

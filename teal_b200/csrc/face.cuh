@@ -1,9 +1,23 @@
 // Face-flux kernel: reconstruction, viscous and convective flux of one face per thread.
 #pragma once
-#include "common.cuh"
-#include "tma.cuh"
+#include "kernels.cuh"
 
 namespace tg {
+
+// arguments of a face-flux launch
+struct FaceLaunch {
+    Sizes s;
+    const void *geom;  // Geometry<R>*
+    const double *q;
+    const void *rec;
+    double gamma, mu, prandtl;
+    void *G;
+    int *err;  // device error word (bounded waits that give up set ERR_TIMEOUT)
+    PressureRef pr_ref;  // FP32-flux form: reference pressure per instance
+    int polls;           // limit of the staged kernel's first wait (MBAR_POLLS unless a test lowers it)
+    Mask mask;
+    const void *side;    // side records (k_gradient SIDES), or null: gradient records only
+};
 
 // ---- face fluxes (src/equations/derivative.c:18-227) ------------------------------------------
 //
@@ -345,32 +359,19 @@ __device__ __forceinline__ void face_flux(const Geo &geo, int i, int f, const Si
     flux_rec_store(G, s.F, f, gf);
 }
 
-// Flux record of a face between two side records (k_gradient SIDES): the reconstructed states are read,
+// Flux record of face f between two side records (k_gradient SIDES): the reconstructed states are read,
 // not formed, so a face costs two records, its normal and its area, and no gather of states or gradients.
+// l, r: the face's Geometry::sides.
 template <typename R, int FK>
-__global__ void __launch_bounds__(SIDE_BLOCK, side_minb<R>()) k_face_sides(Sizes s, Geometry<R> g,
-                                                   const double *__restrict__ q, const R *__restrict__ side,
-                                                   const R *__restrict__ rec, R gamma, R *__restrict__ G,
-                                                   PressureRefOf<R> pr_ref)
+__device__ __forceinline__ void side_flux(const Sizes &s, const Geometry<R> &g, int f, int l, int r, V3<R> n, R area,
+                                          const double *__restrict__ q, const R *__restrict__ side,
+                                          const R *__restrict__ rec, R gamma, const PressureRefOf<R> &pr_ref,
+                                          R (&gf)[5])
 {
-    static_assert(sizeof(R) == 0 || !kExact, "the exact form has no side records");
-    let_next_start();
-    const int f = s.lo + blockIdx.x * SIDE_BLOCK + threadIdx.x;
-    const int fc_ = min(f, s.hi - 1);
-    const int2 e = __ldg(g.sides + fc_);
-    const V3<R> n = load_v3(g.basis, s.F, fc_);
-    const R area = __ldg(g.area + fc_);
-    wait_for_previous();
-    q = after_wait(q);
-    side = after_wait(side);
-    rec = after_wait(rec);
-    if (f >= s.hi) {
-        return;
-    }
     double pref = 0.0;
     R pl[5], pr[5];
     if constexpr (sizeof(R) == sizeof(float)) {
-        pref = pr_ref.of(side_cell(e.x >= 0 ? e.x : e.y));
+        pref = pr_ref.of(side_cell(l >= 0 ? l : r));
     }
     auto row_state = [&](int row) {
         if constexpr (sizeof(R) == sizeof(float)) {
@@ -380,21 +381,21 @@ __global__ void __launch_bounds__(SIDE_BLOCK, side_minb<R>()) k_face_sides(Sizes
             return load_prim<R>(q, s.N, row);
         }
     };
-    if (e.x >= 0) {
-        side_load(side, s.SL, e.x, pl);
+    if (l >= 0) {
+        side_load(side, s.SL, l, pl);
     }
     else {
-        reconstruct<R, true>(row_state(~e.x), rec, ~e.x, load_v3(g.offl, s.F, f), pl);
+        reconstruct<R, true>(row_state(~l), rec, ~l, load_v3(g.offl, s.F, f), pl);
     }
-    if (e.y >= 0) {
-        side_load(side, s.SL, e.y, pr);
+    if (r >= 0) {
+        side_load(side, s.SL, r, pr);
     }
     else if (f >= s.F_in && f < s.F_bd) {  // the ghost state enters unreconstructed (derivative.c:203-211)
-        const Prim<R> qr = row_state(~e.y);
+        const Prim<R> qr = row_state(~r);
         pr[0] = qr.rho, pr[1] = qr.u.x, pr[2] = qr.u.y, pr[3] = qr.u.z, pr[4] = qr.p;
     }
     else {
-        reconstruct<R, true>(row_state(~e.y), rec, ~e.y, load_v3(g.offr, s.F, f), pr);
+        reconstruct<R, true>(row_state(~r), rec, ~r, load_v3(g.offr, s.F, f), pr);
     }
     const Basis<R> b = frame_of(n);
     Cons<R> fc{R(0), v3(R(0), R(0), R(0)), R(0)};
@@ -403,17 +404,54 @@ __global__ void __launch_bounds__(SIDE_BLOCK, side_minb<R>()) k_face_sides(Sizes
                                        make_local(prim_from(pr), gamma, b, R(pref)), gamma);
         fc.m = to_global(b, fc.m);
     }
-    const R gf[5] = {fc.rho * area, fc.m.x * area, fc.m.y * area, fc.m.z * area, fc.e * area};
+    gf[0] = mul_rn(fc.rho, area);
+    gf[1] = mul_rn(fc.m.x, area);
+    gf[2] = mul_rn(fc.m.y, area);
+    gf[3] = mul_rn(fc.m.z, area);
+    gf[4] = mul_rn(fc.e, area);
+}
+
+template <typename R, int FK, bool M>
+__global__ void __launch_bounds__(SIDE_BLOCK, side_minb<R>()) k_face_sides(Sizes s, Geometry<R> g,
+                                                   const double *__restrict__ q, const R *__restrict__ side,
+                                                   const R *__restrict__ rec, R gamma, R *__restrict__ G,
+                                                   PressureRefOf<R> pr_ref, Mask mask)
+{
+    static_assert(sizeof(R) == 0 || !kExact, "the exact form has no side records");
+    let_next_start();
+    const int f = s.lo + blockIdx.x * SIDE_BLOCK + threadIdx.x;
+    const int fc = min(f, s.hi - 1);
+    const int2 e = __ldg(g.sides + fc);
+    const V3<R> n = load_v3(g.basis, s.F, fc);
+    const R area = __ldg(g.area + fc);
+    wait_for_previous();
+    q = after_wait(q);
+    side = after_wait(side);
+    rec = after_wait(rec);
+    if (f >= s.hi || (M && mask.leaves_out(side_cell(e.x >= 0 ? e.x : e.y)))) {
+        return;
+    }
+    R gf[5];
+    side_flux<R, FK>(s, g, f, e.x, e.y, n, area, q, side, rec, gamma, pr_ref, gf);
     flux_rec_store(G, s.F, f, gf);
+}
+
+// whether a residual leaves out face c: both cells lie in one instance, and a partition's faces may have
+// a halo row on their left
+__device__ __forceinline__ bool left_out(const Mask &mask, int2 c, int C)
+{
+    return mask.leaves_out(c.x < C ? c.x : c.y);
 }
 
 // One thread per face, geometry loaded by the threads. face_minb caps the registers so that
 // several blocks stay resident per SM.
-// X: this is the exact translation unit's instantiation (a distinct kernel name per arithmetic).
-template <typename R, int FK, bool NS, int ORDER, bool FOLD, bool X>
+// X: this is the exact translation unit's instantiation (a distinct kernel name per arithmetic). M: some
+// instances are left out (Mask; the test alone made the Navier-Stokes kernel 12 % slower, TGV 128^3
+// 0.417 -> 0.467 ms, so launches without a mask have a kernel without it).
+template <typename R, int FK, bool NS, int ORDER, bool FOLD, bool X, bool M>
 __global__ void __launch_bounds__(FACE_BLOCK, face_minb<R>(NS)) k_face(Sizes s, Geometry<R> g, const double *__restrict__ q,
                                                    const R *__restrict__ rec, R gamma, R mu, R prandtl,
-                                                   R *__restrict__ G, PressureRefOf<R> pr_ref)
+                                                   R *__restrict__ G, PressureRefOf<R> pr_ref, Mask mask)
 {
     static_assert(X == kExact, "exact kernels live in the exact translation units only");
     let_next_start();
@@ -423,6 +461,10 @@ __global__ void __launch_bounds__(FACE_BLOCK, face_minb<R>(NS)) k_face(Sizes s, 
         return;
     }
     DirectGeo<R> geo{g, s.F, f};
+    if (M && left_out(mask, geo.cells(0), s.C)) {
+        wait_for_previous();
+        return;
+    }
     if constexpr (NS && ORDER == 2) {
         __shared__ R aside[sizeof(R) == sizeof(float) ? 10 * FACE_BLOCK : 1];
         face_flux_ns<R, FK, FOLD>(geo, 0, f, s, q, rec, gamma, mu, prandtl, G, pr_ref,
@@ -442,7 +484,7 @@ __global__ void __launch_bounds__(FACE_BLOCK, face_minb<R>(false)) k_face_staged
                                                           const double *__restrict__ q,
                                                           const R *__restrict__ rec, R gamma,
                                                           R *__restrict__ G, int *err,
-                                                          PressureRefOf<R> pr_ref, int polls)
+                                                          PressureRefOf<R> pr_ref, int polls, Mask mask)
 {
     static_assert(X == kExact, "exact kernels live in the exact translation units only");
     __shared__ __align__(16) FaceTile<R, ORDER> t;
@@ -453,7 +495,7 @@ __global__ void __launch_bounds__(FACE_BLOCK, face_minb<R>(false)) k_face_staged
         wait_for_previous();
         return;
     }
-    if (threadIdx.x >= n) {
+    if (threadIdx.x >= n || (mask.on && left_out(mask, t.cells(threadIdx.x), s.C))) {
         wait_for_previous();
     }
     else {

@@ -78,7 +78,8 @@ __global__ void __launch_bounds__(GRAD_THREADS, SIDES ? GRAD_MINB_SIDES : GRAD_M
                                                            const double *__restrict__ eps2,
                                                            const double *__restrict__ q,
                                                            R *__restrict__ rec, int *err, int polls,
-                                                           PressureRefOf<R> pr_ref, SideOut<R> side)
+                                                           PressureRefOf<R> pr_ref, SideOut<R> side,
+                                                           Mask mask)
 {
     static_assert(X == kExact, "exact kernels live in the exact translation units only");
     __shared__ __align__(16) int s_nbr[MIXED ? MAX_SLOTS : 1][GRAD_CELLS];
@@ -95,6 +96,10 @@ __global__ void __launch_bounds__(GRAD_THREADS, SIDES ? GRAD_MINB_SIDES : GRAD_M
     const int l = threadIdx.x % GRAD_CELLS;
     const int c = base + min(l, ncell - 1);
     let_next_start();
+    if (mask.on && !__any_sync(0xffffffffu, !mask.leaves_out(c))) {  // the same cells in every warp
+        wait_for_previous();
+        return;
+    }
     int row[MIXED ? 1 : MAX_SLOTS];
     if constexpr (MIXED) {
         // the whole tile by bulk copies; its slot count is the tile's largest, so a warp of
@@ -332,15 +337,56 @@ __device__ __forceinline__ void add_source(const Source &src, const Prim<double>
     }
 }
 
+// what follows the sum of a cell's fluxes: R kept (mode 0, last stage), the stage update U = U0 + R * alpha *
+// step and q = prim(U) (mode 1), and on the last stage U0 and the cell's stable step of the new state
+__device__ __forceinline__ void finish_cell(int mode, bool ns, int C, int N, int c, const double (&r)[5], int act,
+                                            double alpha, double step, int last, const Props &prop,
+                                            const CellData &cd, double *__restrict__ U0, double *__restrict__ q,
+                                            double *__restrict__ Rout, double *__restrict__ dtc)
+{
+    if (mode == 0 || last) {
+#pragma unroll
+        for (int v = 0; v < 5; v++) {
+            Rout[v * C + c] = r[v];
+        }
+    }
+    if (mode == 0) {
+        return;
+    }
+    if (!act) {
+        if (last) {
+            dtc[c] = DBL_MAX;
+        }
+        return;
+    }
+    Cons<double> u;
+    u.rho = U0[c] + ((r[0] * alpha) * step);
+    u.m.x = U0[C + c] + ((r[1] * alpha) * step);
+    u.m.y = U0[2 * C + c] + ((r[2] * alpha) * step);
+    u.m.z = U0[3 * C + c] + ((r[3] * alpha) * step);
+    u.e = U0[4 * C + c] + ((r[4] * alpha) * step);
+    Prim<double> p = cons_to_prim(u, prop.v[0]);
+    store_prim(q, N, c, p);
+    if (last) {
+        Cons<double> u0 = prim_to_cons(p, prop.v[0]);
+        U0[c] = u0.rho;
+        U0[C + c] = u0.m.x;
+        U0[2 * C + c] = u0.m.y;
+        U0[3 * C + c] = u0.m.z;
+        U0[4 * C + c] = u0.e;
+        dtc[c] = ns ? cell_timestep<true>(p, prop.v, cd, C, c) : cell_timestep<false>(p, prop.v, cd, C, c);
+    }
+}
+
 // X (exact translation units): with `two` (a viscous flux), the viscous records (second set) are summed
 // before the convective ones, the order of teal's two face loops, and R = -sum / V is a quotient.
 template <int MODE, bool NS, typename GT, int SRC, bool X>
-__global__ void __launch_bounds__(CELL_BLOCK, CELL_MINB) k_cell(Sizes s, const int *__restrict__ slot_face,
+__global__ void __launch_bounds__(CELL_BLOCK, cell_minb<GT>()) k_cell(Sizes s, const int *__restrict__ slot_face,
                                                 const uint8_t *__restrict__ slot_cnt, CellData cd,
                                                 const GT *__restrict__ G, double *__restrict__ U0,
                                                 double *__restrict__ q, double *__restrict__ Rout,
                                                 Segments seg, Steps st, double alpha, int last, Props prop,
-                                                double *__restrict__ dtc, Source src, int two)
+                                                double *__restrict__ dtc, Source src, int two, Mask mask)
 {
     static_assert(X == kExact, "exact kernels live in the exact translation units only");
     // nothing is read ahead of the wait: the slot indices held across it cost registers (spills at 40)
@@ -349,7 +395,7 @@ __global__ void __launch_bounds__(CELL_BLOCK, CELL_MINB) k_cell(Sizes s, const i
     G = after_wait(G);
     const int C = s.C, N = s.N;
     int c = s.lo + blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= s.hi) {
+    if (c >= s.hi || (MODE == 0 && mask.leaves_out(c))) {
         return;
     }
     // the stage update's inputs do not depend on the face records: their loads are issued first so
@@ -442,38 +488,7 @@ __global__ void __launch_bounds__(CELL_BLOCK, CELL_MINB) k_cell(Sizes s, const i
         Prim<double> qc{q[c], v3(q[N + c], q[2 * N + c], q[3 * N + c]), q[4 * N + c]};
         add_source<SRC>(src, qc, __ldg(seg.cell_inst + c), r);
     }
-    if (MODE == 0 || last) {
-#pragma unroll
-        for (int v = 0; v < 5; v++) {
-            Rout[v * C + c] = r[v];
-        }
-    }
-    if (MODE == 0) {
-        return;
-    }
-    if (!act) {
-        if (last) {
-            dtc[c] = DBL_MAX;
-        }
-        return;
-    }
-    Cons<double> u;
-    u.rho = U0[c] + ((r[0] * alpha) * step);
-    u.m.x = U0[C + c] + ((r[1] * alpha) * step);
-    u.m.y = U0[2 * C + c] + ((r[2] * alpha) * step);
-    u.m.z = U0[3 * C + c] + ((r[3] * alpha) * step);
-    u.e = U0[4 * C + c] + ((r[4] * alpha) * step);
-    Prim<double> p = cons_to_prim(u, prop.v[0]);
-    store_prim(q, N, c, p);
-    if (last) {
-        Cons<double> u0 = prim_to_cons(p, prop.v[0]);
-        U0[c] = u0.rho;
-        U0[C + c] = u0.m.x;
-        U0[2 * C + c] = u0.m.y;
-        U0[3 * C + c] = u0.m.z;
-        U0[4 * C + c] = u0.e;
-        dtc[c] = cell_timestep<NS>(p, prop.v, cd, C, c);
-    }
+    finish_cell(MODE, NS, C, N, c, r, act, alpha, step, last, prop, cd, U0, q, Rout, dtc);
 }
 
 // U0 = cons(q) and the stable time step of every cell (start of a run / after the host changed
@@ -514,6 +529,7 @@ struct GradientLaunch {
     bool mixed;   // cells with fewer than MAX_SLOTS faces exist
     int *err;     // device error word (a staging wait that gives up sets ERR_TIMEOUT)
     int polls;    // limit of the staging wait (MBAR_POLLS unless a test lowers it)
+    Mask mask;
 };
 
 struct CellLaunch {
@@ -534,6 +550,7 @@ struct CellLaunch {
     Props prop;
     double *dtc;
     Source src;
+    Mask mask;
 };
 
 struct BoundaryLaunch {

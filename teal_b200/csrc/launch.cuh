@@ -9,7 +9,8 @@
 namespace tg {
 
 // Launch of a kernel that waits for the one before it itself (wait_for_previous): it may start while that
-// kernel drains
+// kernel drains. Steps of 513 k cells gain 0.7 % (ramp, 431 -> 428 us), of 111 k cells in 10 meshes 2 %,
+// of 16 k cells 4 %, a residual of 2.4 k cells 14 %, implicit steps of six meshes 4 %.
 template <typename... K, typename... A>
 inline cudaError_t launch_next(void (*kernel)(K...), dim3 grid, dim3 block, cudaStream_t st, const A &...args)
 {
@@ -24,19 +25,6 @@ inline cudaError_t launch_next(void (*kernel)(K...), dim3 grid, dim3 block, cuda
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, K(args)...);
 }
-
-struct FaceLaunch {
-    Sizes s;
-    const void *geom;  // Geometry<R>*
-    const double *q;
-    const void *rec;
-    double gamma, mu, prandtl;
-    void *G;
-    int *err;  // device error word (bounded waits that give up set ERR_TIMEOUT)
-    PressureRef pr_ref;  // FP32-flux form: reference pressure per instance
-    int polls;           // limit of the staged kernel's first wait (MBAR_POLLS unless a test lowers it)
-    const void *side;    // side records (k_gradient SIDES), or null: gradient records only
-};
 
 // The launchers below are local to each translation unit (unnamed namespace): the exact and the plain
 // face translation units instantiate them with the same template arguments, and one shared
@@ -59,11 +47,17 @@ inline void launch_face_v(bool staged, const FaceLaunch &a, const Geometry<R> &g
     if constexpr (!NS) {
         if (staged) {
             launch_next(k_face_staged<R, FK, ORDER, FOLD, X>, grid, dim3(FACE_BLOCK), st, a.s, g, a.q, rec, gm, G,
-                        a.err, pref, a.polls);
+                        a.err, pref, a.polls, a.mask);
             return;
         }
     }
-    launch_next(k_face<R, FK, NS, ORDER, FOLD, X>, grid, dim3(FACE_BLOCK), st, a.s, g, a.q, rec, gm, mu, pr, G, pref);
+    if (a.mask.on) {
+        launch_next(k_face<R, FK, NS, ORDER, FOLD, X, true>, grid, dim3(FACE_BLOCK), st, a.s, g, a.q, rec, gm, mu, pr, G,
+                    pref, a.mask);
+        return;
+    }
+    launch_next(k_face<R, FK, NS, ORDER, FOLD, X, false>, grid, dim3(FACE_BLOCK), st, a.s, g, a.q, rec, gm, mu, pr, G, pref,
+                a.mask);
 }
 
 // staged geometry (bulk copies into shared memory) or thread loads without a viscous flux (tuned.h)
@@ -82,9 +76,14 @@ inline cudaError_t launch_face_r(bool ns, int order, bool fold, const FaceLaunch
             if constexpr (sizeof(R) == sizeof(float)) {
                 pref = a.pr_ref;
             }
-            return launch_next(k_face_sides<R, FK>, dim3((a.s.hi - a.s.lo + SIDE_BLOCK - 1) / SIDE_BLOCK),
-                               dim3(SIDE_BLOCK), st, a.s, g, a.q, static_cast<const R *>(a.side), rec, R(a.gamma), G,
-                               pref);
+            const dim3 grid((a.s.hi - a.s.lo + SIDE_BLOCK - 1) / SIDE_BLOCK), block(SIDE_BLOCK);
+            const R *side = static_cast<const R *>(a.side);
+            if (a.mask.on) {
+                return launch_next(k_face_sides<R, FK, true>, grid, block, st, a.s, g, a.q, side, rec, R(a.gamma), G, pref,
+                                   a.mask);
+            }
+            return launch_next(k_face_sides<R, FK, false>, grid, block, st, a.s, g, a.q, side, rec, R(a.gamma), G, pref,
+                               a.mask);
         }
     }
     const bool staged = !ns && TG_FACE_STAGED_EULER != 0;

@@ -31,7 +31,7 @@ constexpr int NA_MAX_DEVICES = 64;
 
 }  // namespace
 
-// partial sums, [5][pieces]: at most PIECE_COUNT pieces (12 KiB) per device. Every slot the finishing kernel
+// partial sums, [5][pieces]: at most PIECE_COUNT pieces (24 KiB) per device. Every slot the finishing kernel
 // reads is written by the partial kernel of the same call, so nothing has to start at zero.
 static __device__ __align__(256) double g_noalloc_partials[5 * PIECE_COUNT];
 

@@ -144,8 +144,20 @@ __device__ __forceinline__ Prim<R> cons_to_prim(const Cons<R> &c, R gamma)
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 
-// primitive -> conserved (src/euler/create.c:34-44); several kernels form U0 with it (the step's
+// dot, contracted the same way in every kernel: U0 and the stable steps are formed by several (the step's
 // last stage, the preparation of a loaded state), which must agree bit for bit
+template <typename R>
+__device__ __forceinline__ R dot_same(V3<R> a, V3<R> b)
+{
+    if constexpr (kExact) {
+        return dot(a, b);
+    }
+    else {
+        return fma(a.z, b.z, fma(a.y, b.y, mul_rn(a.x, b.x)));
+    }
+}
+
+// primitive -> conserved (src/euler/create.c:34-44)
 template <typename R>
 __device__ __forceinline__ Cons<R> prim_to_cons(const Prim<R> &q, R gamma)
 {
@@ -156,20 +168,24 @@ __device__ __forceinline__ Cons<R> prim_to_cons(const Prim<R> &q, R gamma)
         c.e = (q.p / (gamma - R(1))) + (dot(c.m, q.u) / R(2));
     }
     else {
-        c.e = mul_rn(q.p, R(1) / (gamma - R(1))) + (dot(c.m, q.u) / R(2));
+        c.e = mul_rn(q.p, R(1) / (gamma - R(1))) + mul_rn(dot_same(c.m, q.u), R(1) / R(2));
     }
     return c;
+}
+
+// sum over the axes of (|u| + a) times the cell's projection
+template <typename R>
+__device__ __forceinline__ R convective_radius(const Prim<R> &q, R gamma, V3<R> proj)
+{
+    R a = sqrt(gamma * q.p / q.rho);
+    return dot_same(v3(fabs(q.u.x) + a, fabs(q.u.y) + a, fabs(q.u.z) + a), proj);
 }
 
 // maximum stable step of one cell (src/euler/create.c:6-19)
 template <typename R>
 __device__ __forceinline__ R euler_timestep(const Prim<R> &q, R gamma, R volume, V3<R> proj)
 {
-    R a = sqrt(gamma * q.p / q.rho);
-    R lx = (fabs(q.u.x) + a) * proj.x;
-    R ly = (fabs(q.u.y) + a) * proj.y;
-    R lz = (fabs(q.u.z) + a) * proj.z;
-    return volume / ((lx + ly) + lz);
+    return volume / convective_radius(q, gamma, proj);
 }
 
 // with the viscous term (src/navierstokes/create.c:7-26)
@@ -177,12 +193,9 @@ template <typename R>
 __device__ __forceinline__ R navierstokes_timestep(const Prim<R> &q, R gamma, R mu, R prandtl,
                                                    R volume, V3<R> proj)
 {
-    R a = sqrt(gamma * q.p / q.rho);
-    R lx = (fabs(q.u.x) + a) * proj.x;
-    R ly = (fabs(q.u.y) + a) * proj.y;
-    R lz = (fabs(q.u.z) + a) * proj.z;
+    R lc = convective_radius(q, gamma, proj);
     R lv = fmax(R(4) * mu / (R(3) * q.rho), gamma * mu / (q.rho * prandtl));
-    return volume / (((lx + ly) + lz) + (R(4) * lv * dot(proj, proj) / volume));
+    return volume / (lc + (R(4) * lv * dot_same(proj, proj) / volume));
 }
 
 // ---- convective fluxes (src/euler/convective.c) ------------------------------------------------

@@ -16,18 +16,18 @@ static void gradient_m(const GradientLaunch &a, cudaStream_t st)
     if (a.s.hi <= a.s.lo) return;
     dim3 grid((a.s.hi - a.s.lo + GRAD_CELLS - 1) / GRAD_CELLS);
     switch (a.limiter) {
-        case 0: k_gradient<double, 0, true, MIXED, true><<<grid, GRAD_THREADS, 0, st>>>(a.s, a.g, a.eps2, a.q, a.rec, a.err, a.polls, NoPressureRef{}, SideOut<double>{}); break;
+        case 0: k_gradient<double, 0, true, MIXED, true><<<grid, GRAD_THREADS, 0, st>>>(a.s, a.g, a.eps2, a.q, a.rec, a.err, a.polls, NoPressureRef{}, SideOut<double>{}, a.mask); break;
         case 1:
             if (a.fold)
-                k_gradient<double, 1, true, MIXED, true><<<grid, GRAD_THREADS, 0, st>>>(a.s, a.g, a.eps2, a.q, a.rec, a.err, a.polls, NoPressureRef{}, SideOut<double>{});
+                k_gradient<double, 1, true, MIXED, true><<<grid, GRAD_THREADS, 0, st>>>(a.s, a.g, a.eps2, a.q, a.rec, a.err, a.polls, NoPressureRef{}, SideOut<double>{}, a.mask);
             else
-                k_gradient<double, 1, false, MIXED, true><<<grid, GRAD_THREADS, 0, st>>>(a.s, a.g, a.eps2, a.q, a.rec, a.err, a.polls, NoPressureRef{}, SideOut<double>{});
+                k_gradient<double, 1, false, MIXED, true><<<grid, GRAD_THREADS, 0, st>>>(a.s, a.g, a.eps2, a.q, a.rec, a.err, a.polls, NoPressureRef{}, SideOut<double>{}, a.mask);
             break;
         default:
             if (a.fold)
-                k_gradient<double, 2, true, MIXED, true><<<grid, GRAD_THREADS, 0, st>>>(a.s, a.g, a.eps2, a.q, a.rec, a.err, a.polls, NoPressureRef{}, SideOut<double>{});
+                k_gradient<double, 2, true, MIXED, true><<<grid, GRAD_THREADS, 0, st>>>(a.s, a.g, a.eps2, a.q, a.rec, a.err, a.polls, NoPressureRef{}, SideOut<double>{}, a.mask);
             else
-                k_gradient<double, 2, false, MIXED, true><<<grid, GRAD_THREADS, 0, st>>>(a.s, a.g, a.eps2, a.q, a.rec, a.err, a.polls, NoPressureRef{}, SideOut<double>{});
+                k_gradient<double, 2, false, MIXED, true><<<grid, GRAD_THREADS, 0, st>>>(a.s, a.g, a.eps2, a.q, a.rec, a.err, a.polls, NoPressureRef{}, SideOut<double>{}, a.mask);
             break;
     }
 }
@@ -47,7 +47,7 @@ static void cell_s(const CellLaunch &a, cudaStream_t st)
     if (a.s.hi <= a.s.lo) return;
     k_cell<MODE, NS, double, SRC, true><<<(a.s.hi - a.s.lo + CELL_BLOCK - 1) / CELL_BLOCK, CELL_BLOCK, 0, st>>>(
         a.s, a.slot_face, a.slot_cnt, a.cd, a.G, a.U0, a.q, a.Rout, a.seg, a.st, a.alpha, a.last, a.prop, a.dtc,
-        a.src, a.two);
+        a.src, a.two, a.mask);
 }
 
 template <int MODE, bool NS>

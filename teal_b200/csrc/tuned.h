@@ -35,11 +35,14 @@
 #define TG_FACE_STAGED_EULER 1  // Euler face kernel: geometry staged by bulk copies (1) or loaded (0)
 #endif
 #ifndef TG_CELL_MINB
-#define TG_CELL_MINB 12  // cell-gather blocks kept resident per SM (caps registers per thread)
+#define TG_CELL_MINB 10  // cell-gather blocks kept resident per SM (caps registers per thread)
+#endif
+#ifndef TG_CELL_MINB_FP32
+#define TG_CELL_MINB_FP32 12  // the same in the FP32-flux form
 #endif
 #ifndef TG_GRAD_MINB
 #define TG_GRAD_MINB 12  // gradient blocks (160 threads) kept resident per SM (caps registers per thread)
 #endif
 #ifndef TG_GRAD_MINB_SIDES
-#define TG_GRAD_MINB_SIDES 10  // the same for the gradient kernel that writes side records
+#define TG_GRAD_MINB_SIDES 9  // the same for the gradient kernel that writes side records
 #endif
