@@ -1791,10 +1791,41 @@ static int run_fluxes(tg_ctx *c, double *q, bool masked = false)
     return TG_OK;
 }
 
+// Whether the face fluxes and the cell update of a residual run in one launch: on small arenas (see
+// k_cell_fluxes), where side records exist and no source is added
+static bool use_fused(const tg_ctx *c)
+{
+    return use_sides(c) && c->source == TG_SOURCE_NONE && c->s.C <= TG_FUSED_CELLS;
+}
+
+static int launch_fused(tg_ctx *c, int mode, double alpha, int last, double *q, double *Rout)
+{
+    const FaceLaunch a = face_args(c, q);
+    const CellLaunch b = cell_args(c, mode, alpha, last, q, Rout);
+    Launch l(c, TG_PROF_FACE);
+    switch (c->flux) {
+        case TG_FLUX_ROE: CU(launch_cell_fluxes<FK_ROE>(c->precision, a, b, c->stream)); break;
+        case TG_FLUX_HLL: CU(launch_cell_fluxes<FK_HLL>(c->precision, a, b, c->stream)); break;
+        case TG_FLUX_HLLC: CU(launch_cell_fluxes<FK_HLLC>(c->precision, a, b, c->stream)); break;
+        case TG_FLUX_HLLE: CU(launch_cell_fluxes<FK_HLLE>(c->precision, a, b, c->stream)); break;
+        case TG_FLUX_AUSMD: CU(launch_cell_fluxes<FK_AUSMD>(c->precision, a, b, c->stream)); break;
+        case TG_FLUX_AUSMDV: CU(launch_cell_fluxes<FK_AUSMDV>(c->precision, a, b, c->stream)); break;
+        case TG_FLUX_LXF: CU(launch_cell_fluxes<FK_LXF>(c->precision, a, b, c->stream)); break;
+        case TG_FLUX_CENTRAL: CU(launch_cell_fluxes<FK_CENTRAL>(c->precision, a, b, c->stream)); break;
+        default: CU(launch_cell_fluxes<FK_NONE>(c->precision, a, b, c->stream)); break;
+    }
+    return TG_OK;
+}
+
 // the whole residual of q: mode 0 R into Rout, mode 1 one RK stage
 template <int MODE>
 static int run_residual(tg_ctx *c, double *q, double *Rout, bool masked, double alpha = 0.0, int last = 0)
 {
+    if (use_fused(c)) {
+        TRY(run_fluxes_pre(c, q, masked));
+        TRY(run_gradient(c, q));
+        return launch_fused(c, MODE, alpha, last, q, Rout);
+    }
     TRY(run_fluxes(c, q, masked));
     return launch_cell<MODE>(c, alpha, last, q, Rout);
 }

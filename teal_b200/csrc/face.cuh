@@ -436,6 +436,82 @@ __global__ void __launch_bounds__(SIDE_BLOCK, side_minb<R>()) k_face_sides(Sizes
     flux_rec_store(G, s.F, f, gf);
 }
 
+// Face fluxes and cell update in one launch for small meshes: a block is a tile of 32 cells, warp j computes
+// the fluxes of the cells' slots j (the left-to-right flux of the face, as k_face_sides: each inner face
+// is computed by both of its cells, with the same bits), five warps sum them in slot order and one
+// finishes the cells as k_cell does. It saves a launch and the round trip of the flux records, and pays
+// with twice the flux arithmetic: worth it while a launch costs more than that arithmetic
+// (TG_FUSED_CELLS, launch rule in context.cu).
+template <typename R, int FK>
+__global__ void __launch_bounds__(SIDE_TILE, 4) k_cell_fluxes(FaceLaunch a, Geometry<R> g, CellLaunch b)
+{
+    static_assert(sizeof(R) == 0 || !kExact, "the exact form has no side records");
+    __shared__ R s_flux[5][SIDE_TILE];
+    __shared__ int s_face[SIDE_TILE];
+    __shared__ double s_sum[5][32];
+    let_next_start();
+    const Sizes &s = a.s;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int c = blockIdx.x * 32 + lane;
+    const int cnt = c < s.C ? int(b.slot_cnt[c]) : 0;
+    const bool in = warp < cnt;
+    const int sf = in ? __ldg(b.slot_face + (size_t)warp * s.SL + c) : 0;
+    const int f = sf >= 0 ? sf : ~sf;
+    const int2 e = __ldg(g.sides + f);
+    const V3<R> n = load_v3(g.basis, s.F, f);
+    const R area = __ldg(g.area + f);
+    PressureRefOf<R> pr_ref{};
+    if constexpr (sizeof(R) == sizeof(float)) {
+        pr_ref = a.pr_ref;
+    }
+    wait_for_previous();
+    const double *q = after_wait(a.q);
+    const R *side = after_wait(static_cast<const R *>(a.side));
+    const R *rec = after_wait(static_cast<const R *>(a.rec));
+    if (a.mask.on && !__any_sync(0xffffffffu, c < s.C && !a.mask.leaves_out(c))) {  // the same cells in every warp
+        return;
+    }
+    R gf[5] = {R(0), R(0), R(0), R(0), R(0)};
+    if (in) {
+        side_flux<R, FK>(s, g, f, e.x, e.y, n, area, q, side, rec, R(a.gamma), pr_ref, gf);
+    }
+#pragma unroll
+    for (int v = 0; v < 5; v++) {
+        s_flux[v][threadIdx.x] = gf[v];
+    }
+    s_face[threadIdx.x] = sf;
+    __syncthreads();
+    if (warp < 5) {
+        double acc = 0;
+#pragma unroll
+        for (int j = 0; j < MAX_SLOTS; j++) {
+            if (j < cnt) {
+                const double x = double(s_flux[warp][j * 32 + lane]);
+                acc = s_face[j * 32 + lane] >= 0 ? acc + x : acc - x;
+            }
+        }
+        s_sum[warp][lane] = acc;
+    }
+    __syncthreads();
+    if (warp != 0 || c >= s.C || (b.mode == 0 && a.mask.leaves_out(c))) {
+        return;
+    }
+    int act = 1;
+    double step = 0.0;
+    if (b.mode != 0) {
+        const int inst = __ldg(b.seg.cell_inst + c);
+        act = b.st.active[inst];
+        step = b.st.step[inst];
+    }
+    const double ivol = 1.0 / __ldg(b.cd.volume + c);
+    double r[5];
+#pragma unroll
+    for (int v = 0; v < 5; v++) {
+        r[v] = -s_sum[v][lane] * ivol;
+    }
+    finish_cell(b.mode, b.ns, s.C, s.N, c, r, act, b.alpha, step, b.last, b.prop, b.cd, b.U0, b.q, b.Rout, b.dtc);
+}
+
 // whether a residual leaves out face c: both cells lie in one instance, and a partition's faces may have
 // a halo row on their left
 __device__ __forceinline__ bool left_out(const Mask &mask, int2 c, int C)

@@ -114,6 +114,10 @@ template <int FK>
 cudaError_t launch_face(int precision, bool ns, int order, bool fold, const FaceLaunch &a,
                         cudaStream_t st);
 
+// face fluxes and cell updates in one launch (k_cell_fluxes); `a.side` must be set
+template <int FK>
+cudaError_t launch_cell_fluxes(int precision, const FaceLaunch &a, const CellLaunch &b, cudaStream_t st);
+
 // FP64 with teal's exact arithmetic (face_*_exact.cu); with a viscous flux, `a.G` holds 2 x 5 F
 // values (convective and viscous records)
 template <int FK>
@@ -128,6 +132,18 @@ cudaError_t launch_face_exact(bool ns, int order, bool fold, const FaceLaunch &a
             return launch_face_r<FK, double>(ns, order, fold, a, st);                           \
         }                                                                                       \
         return launch_face_r<FK, float>(ns, order, fold, a, st);                                \
+    }                                                                                           \
+    template <>                                                                                 \
+    cudaError_t launch_cell_fluxes<FK>(int precision, const FaceLaunch &a, const CellLaunch &b, \
+                                       cudaStream_t st)                                         \
+    {                                                                                           \
+        const dim3 grid((a.s.C + 31) / 32), block(SIDE_TILE);                                   \
+        if (precision == 0) {                                                                   \
+            return launch_next(k_cell_fluxes<double, FK>, grid, block, st, a,                   \
+                               *static_cast<const Geometry<double> *>(a.geom), b);              \
+        }                                                                                       \
+        return launch_next(k_cell_fluxes<float, FK>, grid, block, st, a,                        \
+                           *static_cast<const Geometry<float> *>(a.geom), b);                   \
     }
 
 #define TG_INSTANTIATE_FACE_EXACT(FK)                                                              \

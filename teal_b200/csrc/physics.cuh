@@ -445,19 +445,16 @@ __device__ __forceinline__ Cons<R> flux_hllc(const Local<R> &l, const Local<R> &
 {
     R sl, sr;
     einfeldt_speeds(l, r, gamma, sl, sr);
-    if (sl >= R(0)) {
-        return physical_flux(l);
-    }
-    if (sr <= R(0)) {
-        return physical_flux(r);
-    }
     R fl = l.rho * (sl - l.u.x);
     R fr = r.rho * (sr - r.u.x);
     R s = (((r.p - l.p) + (fl * l.u.x)) - (fr * r.u.x)) / (fl - fr);
-    if (sl <= R(0) && R(0) <= s) {
-        return contact_flux(l, sl, fl, s);
+    // the side is selected first, so that one flux is evaluated and not up to four by a divergent warp
+    const bool left = sl >= R(0) || (!(sr <= R(0)) && sl <= R(0) && R(0) <= s);
+    const Local<R> k = left ? l : r;
+    if (sl >= R(0) || sr <= R(0)) {
+        return physical_flux(k);
     }
-    return contact_flux(r, sr, fr, s);
+    return contact_flux(k, left ? sl : sr, left ? fl : fr, s);
 }
 
 // HLLE with Einfeldt's averaged sound speed (convective.c:348-389)
