@@ -1366,15 +1366,17 @@ static int d2h(tg_ctx *c, double *dst, const double *src, size_t n)
         CU(cudaMemcpyAsync(c->pinned + o, src + o, span(k) * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
         CU(cudaEventRecord(c->read_ev[k], c->stream));
     }
-    std::atomic<int> next(0), failed(0);
+    // the helpers make no CUDA calls: this thread tells them how many chunks have arrived (-1: none will)
+    std::atomic<int> next(0), arrived(0);
     auto copy = [&]() {
-        if (cudaSetDevice(c->device) != cudaSuccess) failed = 1;
-        for (int k; !failed && (k = next++) < chunks;) {
-            if (cudaEventSynchronize(c->read_ev[k]) != cudaSuccess) {
-                failed = 1;
-                break;
-            }
+        for (int k; (k = next++) < chunks;) {
             const size_t o = (size_t)k * READ_CHUNK;
+            // a fresh array's pages are faulted in while the device still computes
+            volatile char *page = reinterpret_cast<volatile char *>(dst + o);
+            for (size_t b = 0; b < span(k) * sizeof(double); b += 4096) page[b] = page[b];
+            int n;
+            while ((n = arrived) <= k && n >= 0) std::this_thread::yield();
+            if (n < 0) return;
             memcpy(dst + o, c->pinned + o, span(k) * sizeof(double));
         }
     };
@@ -1384,10 +1386,14 @@ static int d2h(tg_ctx *c, double *dst, const double *src, size_t n)
     }
     catch (const std::system_error &) {  // no more threads: fewer, or this one alone
     }
+    for (int k = 0; k < chunks && arrived >= 0; k++) {
+        const cudaError_t e = cudaEventSynchronize(c->read_ev[k]);
+        arrived = e == cudaSuccess ? k + 1 : -1;
+    }
     copy();
     for (std::thread &t : threads) t.join();
     CU(cudaStreamSynchronize(c->stream));
-    if (failed) return fail(TG_ERR_CUDA, "reading the device's rows back failed");
+    if (arrived < 0) return fail(TG_ERR_CUDA, "reading the device's rows back failed");
     return TG_OK;
 }
 
@@ -2160,6 +2166,13 @@ extern "C" int tg_advance(tg_ctx *c, int method, const void *context, double cou
 #define TG_IO_CHUNKS 8
 #endif
 constexpr int IO_CHUNKS = TG_IO_CHUNKS;
+// least cells of a chunk: its share of the last stage (launches, tails) must cost less than the copy it
+// hides, 40 bytes a cell at about 53 GB/s. Below two chunks the step is the replayed graph with the
+// copy behind it.
+#ifndef TG_IO_CHUNK_CELLS
+#define TG_IO_CHUNK_CELLS 131072
+#endif
+constexpr int IO_CHUNK_CELLS = TG_IO_CHUNK_CELLS;
 
 static uint64_t io_bit(int k) { return uint64_t(1) << k; }
 
@@ -2167,8 +2180,7 @@ static int build_io_plan(tg_ctx *c)
 {
     const int C = c->s.C, F = c->s.F, Fin = c->s.F_in;
     std::unique_ptr<IoPlan> p(new IoPlan);
-    // chunks of at least 64 gradient tiles
-    int K = std::max(1, std::min(IO_CHUNKS, C / (64 * GRAD_CELLS)));
+    int K = std::max(1, std::min(IO_CHUNKS, C / IO_CHUNK_CELLS));
     const int per = ((C + K - 1) / K + GRAD_CELLS - 1) / GRAD_CELLS * GRAD_CELLS;
     K = (C + per - 1) / per;
     std::vector<int2> lr(F);
@@ -2277,6 +2289,16 @@ static int advance_chunked(tg_ctx *c, int stages, const double *alpha, double co
     return TG_OK;
 }
 
+// the rows of a single mesh (ghosts too) into a pinned host array, on the context's stream
+static int copy_rows(tg_ctx *c, double *out)
+{
+    const int rows = c->inst_row_off[1];
+    k_rows_gather<<<grid_of(rows), BLOCK, 0, c->stream>>>(rows, c->rowmap, c->s.N, c->q, c->aos);
+    CU(cudaGetLastError());
+    CU(cudaMemcpyAsync(out, c->aos, sizeof(double) * 5 * (size_t)rows, cudaMemcpyDeviceToHost, c->stream));
+    return TG_OK;
+}
+
 extern "C" int tg_advance_host(tg_ctx *c, int method, const void *context, double courant, double *time,
                                double max_step, const double *prim_in, double *prim_out, double *residual,
                                double *step0)
@@ -2308,7 +2330,16 @@ extern "C" int tg_advance_host(tg_ctx *c, int method, const void *context, doubl
     hi_at(c, SI_ACTIVE, 0) = 1;
     hi_error(c) = 0;
     TRY(write_steps(c));
-    const int rc = advance_chunked(c, stages, alpha, courant, prim_out);
+    int rc;
+    if (c->io->K > 1) {
+        c->st.use_max_time = 0;  // clipped by max_step, whatever a run loop left
+        rc = advance_chunked(c, stages, alpha, courant, prim_out);
+    }
+    else {
+        rc = step_graph(c, method, stages, alpha, courant, 0);
+        if (rc == TG_OK) rc = launch_step(c, stages, alpha, courant);
+        if (rc == TG_OK) rc = copy_rows(c, prim_out);
+    }
     c->cell_lo = 0, c->cell_hi = -1, c->face_lo = 0, c->face_hi = -1;
     if (rc != TG_OK) {
         // nothing may still write into the caller's buffer once this returns
