@@ -226,8 +226,8 @@ __device__ __forceinline__ Cons<R> viscous_face(const Geo &geo, int i, bool boun
 // resident blocks).
 template <typename R, int FK, bool FOLD, typename Geo>
 __device__ __forceinline__ void face_flux_ns(const Geo &geo, int i, int f, const Sizes &s,
-                                             const double *__restrict__ q, const R *__restrict__ rec, R gamma, R mu,
-                                             R prandtl, R *__restrict__ G, const PressureRefOf<R> &pr_ref,
+                                             const double *__restrict__ q, const R *__restrict__ rec, R gamma, R ig,
+                                             R mu, R prandtl, R *__restrict__ G, const PressureRefOf<R> &pr_ref,
                                              R *column)
 {
     const bool boundary = (f >= s.F_in) && (f < s.F_bd);
@@ -250,20 +250,23 @@ __device__ __forceinline__ void face_flux_ns(const Geo &geo, int i, int f, const
     Cons<R> fc{R(0), v3(R(0), R(0), R(0)), R(0)};
     if (FK != FK_NONE) {
         Basis<R> b;
+        R factor = R(0);
         if constexpr (kExact) {
             b = geo.basis_again(i);
         }
         else {
-            b = frame_of(geo.normal_again(i));
+            const V3<R> n = geo.normal_again(i);
+            factor = frame_factor(n);
+            b = frame_of(n, factor);
         }
-        const Local<R> l = make_local(prim_from(pl), gamma, b, R(pref));
-        const Local<R> r = make_local(prim_from(pr), gamma, b, R(pref));
+        const Local<R> l = make_local(prim_from(pl), gamma, b, R(pref), ig);
+        const Local<R> r = make_local(prim_from(pr), gamma, b, R(pref), ig);
         fc = convective_flux_local<FK>(l, r, gamma);
         if constexpr (kExact) {
             fc.m = to_global(geo.basis_again(i), fc.m);
         }
         else {
-            fc.m = to_global(frame_of(geo.normal_again(i)), fc.m);
+            fc.m = to_global(frame_of(geo.normal_again(i), factor), fc.m);
         }
     }
     const R area = geo.area(i);
@@ -365,8 +368,8 @@ __device__ __forceinline__ void face_flux(const Geo &geo, int i, int f, const Si
 template <typename R, int FK>
 __device__ __forceinline__ void side_flux(const Sizes &s, const Geometry<R> &g, int f, int l, int r, V3<R> n, R area,
                                           const double *__restrict__ q, const R *__restrict__ side,
-                                          const R *__restrict__ rec, R gamma, const PressureRefOf<R> &pr_ref,
-                                          R (&gf)[5])
+                                          const R *__restrict__ rec, R gamma, R ig,
+                                          const PressureRefOf<R> &pr_ref, R (&gf)[5])
 {
     double pref = 0.0;
     R pl[5], pr[5];
@@ -400,8 +403,8 @@ __device__ __forceinline__ void side_flux(const Sizes &s, const Geometry<R> &g, 
     const Basis<R> b = frame_of(n);
     Cons<R> fc{R(0), v3(R(0), R(0), R(0)), R(0)};
     if (FK != FK_NONE) {
-        fc = convective_flux_local<FK>(make_local(prim_from(pl), gamma, b, R(pref)),
-                                       make_local(prim_from(pr), gamma, b, R(pref)), gamma);
+        fc = convective_flux_local<FK>(make_local(prim_from(pl), gamma, b, R(pref), ig),
+                                       make_local(prim_from(pr), gamma, b, R(pref), ig), gamma);
         fc.m = to_global(b, fc.m);
     }
     gf[0] = mul_rn(fc.rho, area);
@@ -414,7 +417,7 @@ __device__ __forceinline__ void side_flux(const Sizes &s, const Geometry<R> &g, 
 template <typename R, int FK, bool M>
 __global__ void __launch_bounds__(SIDE_BLOCK, side_minb<R>()) k_face_sides(Sizes s, Geometry<R> g,
                                                    const double *__restrict__ q, const R *__restrict__ side,
-                                                   const R *__restrict__ rec, R gamma, R *__restrict__ G,
+                                                   const R *__restrict__ rec, R gamma, R ig, R *__restrict__ G,
                                                    PressureRefOf<R> pr_ref, Mask mask)
 {
     static_assert(sizeof(R) == 0 || !kExact, "the exact form has no side records");
@@ -432,7 +435,7 @@ __global__ void __launch_bounds__(SIDE_BLOCK, side_minb<R>()) k_face_sides(Sizes
         return;
     }
     R gf[5];
-    side_flux<R, FK>(s, g, f, e.x, e.y, n, area, q, side, rec, gamma, pr_ref, gf);
+    side_flux<R, FK>(s, g, f, e.x, e.y, n, area, q, side, rec, gamma, ig, pr_ref, gf);
     flux_rec_store(G, s.F, f, gf);
 }
 
@@ -473,7 +476,7 @@ __global__ void __launch_bounds__(SIDE_TILE, 4) k_cell_fluxes(FaceLaunch a, Geom
     }
     R gf[5] = {R(0), R(0), R(0), R(0), R(0)};
     if (in) {
-        side_flux<R, FK>(s, g, f, e.x, e.y, n, area, q, side, rec, R(a.gamma), pr_ref, gf);
+        side_flux<R, FK>(s, g, f, e.x, e.y, n, area, q, side, rec, R(a.gamma), R(1) / (R(a.gamma) - R(1)), pr_ref, gf);
     }
 #pragma unroll
     for (int v = 0; v < 5; v++) {
@@ -526,7 +529,7 @@ __device__ __forceinline__ bool left_out(const Mask &mask, int2 c, int C)
 // 0.417 -> 0.467 ms, so launches without a mask have a kernel without it).
 template <typename R, int FK, bool NS, int ORDER, bool FOLD, bool X, bool M>
 __global__ void __launch_bounds__(FACE_BLOCK, face_minb<R>(NS)) k_face(Sizes s, Geometry<R> g, const double *__restrict__ q,
-                                                   const R *__restrict__ rec, R gamma, R mu, R prandtl,
+                                                   const R *__restrict__ rec, R gamma, R ig, R mu, R prandtl,
                                                    R *__restrict__ G, PressureRefOf<R> pr_ref, Mask mask)
 {
     static_assert(X == kExact, "exact kernels live in the exact translation units only");
@@ -543,7 +546,7 @@ __global__ void __launch_bounds__(FACE_BLOCK, face_minb<R>(NS)) k_face(Sizes s, 
     }
     if constexpr (NS && ORDER == 2) {
         __shared__ R aside[sizeof(R) == sizeof(float) ? 10 * FACE_BLOCK : 1];
-        face_flux_ns<R, FK, FOLD>(geo, 0, f, s, q, rec, gamma, mu, prandtl, G, pr_ref,
+        face_flux_ns<R, FK, FOLD>(geo, 0, f, s, q, rec, gamma, ig, mu, prandtl, G, pr_ref,
                                   aside + (sizeof(R) == sizeof(float) ? threadIdx.x : 0));
     }
     else {

@@ -179,7 +179,10 @@ __global__ void __launch_bounds__(GRAD_THREADS, SIDES ? GRAD_MINB_SIDES : GRAD_M
         }
     }
     R gx = R(0), gy = R(0), gz = R(0);
-    double mn = qc, mx = qc;
+    // The extrema of q - qc over the neighbours, not of q: the differences are at hand, rounding is monotone
+    // (the same values, bit for bit), and a comparison with a select is half the instructions of an fmin or
+    // fmax in FP64 (in the FP32-flux form they become FP32 minima).
+    R dmn = R(0), dmx = R(0);
 #pragma unroll
     for (int j = 0; j < MAX_SLOTS; j++) {
         if (j >= jmax) break;
@@ -188,8 +191,8 @@ __global__ void __launch_bounds__(GRAD_THREADS, SIDES ? GRAD_MINB_SIDES : GRAD_M
             gx += d * s_w[3 * j + 0][l];
             gy += d * s_w[3 * j + 1][l];
             gz += d * s_w[3 * j + 2][l];
-            mn = fmin(mn, qn[j]);
-            mx = fmax(mx, qn[j]);
+            dmn = d < dmn ? d : dmn;
+            dmx = d > dmx ? d : dmx;
         }
     }
 
@@ -213,7 +216,7 @@ __global__ void __launch_bounds__(GRAD_THREADS, SIDES ? GRAD_MINB_SIDES : GRAD_M
             if (j < cnt) {
                 R d2 = ((gx * s_off[3 * j + 0][l]) + (gy * s_off[3 * j + 1][l])) + (gz * s_off[3 * j + 2][l]);
                 if (!is_close_zero(d2)) {
-                    const R d1 = ((d2 > R(0)) ? R(mx) : R(mn)) - R(qc);
+                    const R d1 = (d2 > R(0)) ? dmx : dmn;
                     if (LIM == 1) {
                         psi = fmin(psi, fmin(R(1), d1 / d2));
                     }
@@ -228,7 +231,6 @@ __global__ void __launch_bounds__(GRAD_THREADS, SIDES ? GRAD_MINB_SIDES : GRAD_M
     }
     else if (LIM != 0) {
         const R e2 = (LIM == 2) ? R(__ldg(eps2 + c)) : R(0);
-        const R dmx = R(mx - qc), dmn = R(mn - qc);
         R best_n = R(1), best_d = R(1);
 #pragma unroll
         for (int j = 0; j < MAX_SLOTS; j++) {

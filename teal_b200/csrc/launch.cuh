@@ -39,7 +39,7 @@ inline void launch_face_v(bool staged, const FaceLaunch &a, const Geometry<R> &g
         return;
     }
     dim3 grid((a.s.hi - a.s.lo + FACE_BLOCK - 1) / FACE_BLOCK);
-    R gm = R(a.gamma), mu = R(a.mu), pr = R(a.prandtl);
+    const R gm = R(a.gamma), ig = R(1) / (gm - R(1)), mu = R(a.mu), pr = R(a.prandtl);
     PressureRefOf<R> pref{};
     if constexpr (sizeof(R) == sizeof(float)) {
         pref = a.pr_ref;
@@ -52,11 +52,11 @@ inline void launch_face_v(bool staged, const FaceLaunch &a, const Geometry<R> &g
         }
     }
     if (a.mask.on) {
-        launch_next(k_face<R, FK, NS, ORDER, FOLD, X, true>, grid, dim3(FACE_BLOCK), st, a.s, g, a.q, rec, gm, mu, pr, G,
+        launch_next(k_face<R, FK, NS, ORDER, FOLD, X, true>, grid, dim3(FACE_BLOCK), st, a.s, g, a.q, rec, gm, ig, mu, pr, G,
                     pref, a.mask);
         return;
     }
-    launch_next(k_face<R, FK, NS, ORDER, FOLD, X, false>, grid, dim3(FACE_BLOCK), st, a.s, g, a.q, rec, gm, mu, pr, G, pref,
+    launch_next(k_face<R, FK, NS, ORDER, FOLD, X, false>, grid, dim3(FACE_BLOCK), st, a.s, g, a.q, rec, gm, ig, mu, pr, G, pref,
                 a.mask);
 }
 
@@ -79,10 +79,10 @@ inline cudaError_t launch_face_r(bool ns, int order, bool fold, const FaceLaunch
             const dim3 grid((a.s.hi - a.s.lo + SIDE_BLOCK - 1) / SIDE_BLOCK), block(SIDE_BLOCK);
             const R *side = static_cast<const R *>(a.side);
             if (a.mask.on) {
-                return launch_next(k_face_sides<R, FK, true>, grid, block, st, a.s, g, a.q, side, rec, R(a.gamma), G, pref,
+                return launch_next(k_face_sides<R, FK, true>, grid, block, st, a.s, g, a.q, side, rec, R(a.gamma), R(1) / (R(a.gamma) - R(1)), G, pref,
                                    a.mask);
             }
-            return launch_next(k_face_sides<R, FK, false>, grid, block, st, a.s, g, a.q, side, rec, R(a.gamma), G, pref,
+            return launch_next(k_face_sides<R, FK, false>, grid, block, st, a.s, g, a.q, side, rec, R(a.gamma), R(1) / (R(a.gamma) - R(1)), G, pref,
                                a.mask);
         }
     }

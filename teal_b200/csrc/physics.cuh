@@ -97,16 +97,25 @@ __device__ __forceinline__ V3<R> to_global(const Basis<R> &b, V3<R> v)
 // of the frame about the normal: any such tangents serve in place of the mesh's stored ones, up to
 // rounding, and the plain kernels read only the normal row of the stored basis.
 template <typename R>
-__device__ __forceinline__ Basis<R> frame_of(V3<R> n)
+__device__ __forceinline__ R frame_factor(V3<R> n)  // the frame's only quotient, kept where the frame is built twice
+{
+    return R(-1) / (copysign(R(1), n.z) + n.z);
+}
+template <typename R>
+__device__ __forceinline__ Basis<R> frame_of(V3<R> n, R a)
 {
     const R sg = copysign(R(1), n.z);
-    const R a = R(-1) / (sg + n.z);
     const R b = (n.x * n.y) * a;
     Basis<R> f;
     f.x = n;
     f.y = v3(R(1) + ((sg * (n.x * n.x)) * a), sg * b, -sg * n.x);
     f.z = v3(b, sg + ((n.y * n.y) * a), -n.y);
     return f;
+}
+template <typename R>
+__device__ __forceinline__ Basis<R> frame_of(V3<R> n)
+{
+    return frame_of(n, frame_factor(n));
 }
 
 // primitive state: density, velocity, pressure (src/euler.h EulerPrimitive)
@@ -224,9 +233,10 @@ struct Local : LocalRel<R> {
     R e;
 };
 
-// g.p is the pressure relative to pref (FP32-flux form) or the pressure itself (pref = 0)
+// g.p is the pressure relative to pref (FP32-flux form) or the pressure itself (pref = 0); ig = 1 / (gamma - 1),
+// which the face kernels take as an argument
 template <typename R>
-__device__ __forceinline__ Local<R> make_local(const Prim<R> &g, R gamma, const Basis<R> &b, R pref = R(0))
+__device__ __forceinline__ Local<R> make_local(const Prim<R> &g, R gamma, const Basis<R> &b, R pref, R ig)
 {
     Local<R> s;
     s.rho = g.rho;
@@ -239,7 +249,7 @@ __device__ __forceinline__ Local<R> make_local(const Prim<R> &g, R gamma, const 
             s.e = (s.p / (gamma - R(1))) + (dot(s.m, s.u) / R(2));
         }
         else {
-            s.e = (s.p * (R(1) / (gamma - R(1)))) + (dot(s.m, s.u) / R(2));
+            s.e = (s.p * ig) + (dot(s.m, s.u) / R(2));
         }
     }
     else {
@@ -247,10 +257,15 @@ __device__ __forceinline__ Local<R> make_local(const Prim<R> &g, R gamma, const 
         s.p = g.p + pref;
         s.m = mul(s.rho, s.u);
         const R kinetic = dot(s.m, s.u) / R(2);
-        s.e = (s.p * (R(1) / (gamma - R(1)))) + kinetic;
-        s.de = (s.dp * (R(1) / (gamma - R(1)))) + kinetic;
+        s.e = (s.p * ig) + kinetic;
+        s.de = (s.dp * ig) + kinetic;
     }
     return s;
+}
+template <typename R>
+__device__ __forceinline__ Local<R> make_local(const Prim<R> &g, R gamma, const Basis<R> &b, R pref = R(0))
+{
+    return make_local(g, gamma, b, pref, R(1) / (gamma - R(1)));
 }
 
 // physical flux normal to the face (convective.c:32-41)
