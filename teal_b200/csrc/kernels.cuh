@@ -196,16 +196,17 @@ __global__ void __launch_bounds__(GRAD_THREADS, SIDES ? GRAD_MINB_SIDES : GRAD_M
         }
     }
 
-    // limiter factor: the minimum over the cell's faces of teal's candidate ratios. Each candidate
-    // is a fraction num / den with num >= 0 and den > 0 (delta1 has delta2's sign or is zero):
-    //   Barth-Jespersen  min(1, delta1 / delta2) = |delta1| / |delta2|, the 1 by psi's start value
-    //                    (limiter.c:54-58);
+    // limiter factor: the minimum of 1 and of teal's candidate ratios over the cell's faces. With delta1 the
+    // extremum of q - qc on the side of delta2 (of its sign or zero), each candidate is a fraction with a
+    // positive denominator:
+    //   Barth-Jespersen  delta1 / delta2 (limiter.c:54-58);
     //   Venkatakrishnan  top / bot / delta2 (limiter.c:100-106) with delta2 divided out of top:
-    //                    (d1 (d1 + 2 d2) + eps2) / (d1 (d1 + d2) + 2 d2^2 + eps2), every term >= 0.
-    // The running minimum stays a fraction compared by cross multiplication and is divided once:
-    // one division per thread instead of one or two per face, within a few ulps of teal's per-face
-    // quotients (FP32: a product underflows only for candidates below about 1e-30, where a fraction
-    // of 0 and its rounding do not change the minimum; FP32 ramp-batch gradient 0.626 -> 0.517 ms).
+    //                    (d1 (d1 + 2 d2) + eps2) / (d1 (d1 + d2) + 2 d2^2 + eps2).
+    // For a given delta1 both fall as |delta2| grows, wherever they are below 1 (Venkatakrishnan: below 1 from
+    // |d2| = |d1| / 2 on, where the derivative's sign is that of (d1^2 + eps2) (d1 - 4 d2) - 4 d1 d2^2 < 0). So only the
+    // largest positive and the most negative delta2 count: per face a product and two comparisons, and two
+    // candidates at the end, compared by cross multiplication and divided once, instead of a candidate
+    // and a comparison of fractions per face (the kernel is bound by instruction issue: 72 % active).
     R psi = R(1);
     if (X && LIM != 0) {
         // teal's own candidates, one quotient per face (limiter.c:54-58, :100-106)
@@ -231,30 +232,30 @@ __global__ void __launch_bounds__(GRAD_THREADS, SIDES ? GRAD_MINB_SIDES : GRAD_M
     }
     else if (LIM != 0) {
         const R e2 = (LIM == 2) ? R(__ldg(eps2 + c)) : R(0);
-        R best_n = R(1), best_d = R(1);
+        R hi = R(0), lo = R(0);  // extrema of delta2
 #pragma unroll
         for (int j = 0; j < MAX_SLOTS; j++) {
             if (j >= jmax) break;
             if (j < cnt) {
-                R d2 = ((gx * s_off[3 * j + 0][l]) + (gy * s_off[3 * j + 1][l])) + (gz * s_off[3 * j + 2][l]);
-                if (!is_close_zero(d2)) {
-                    const R d1 = (d2 > R(0)) ? dmx : dmn;
-                    R num, den;
-                    if (LIM == 1) {
-                        num = fabs(d1);
-                        den = fabs(d2);
-                    }
-                    else {
-                        num = fma(d1, fma(R(2), d2, d1), e2);
-                        den = fma(d1, d1 + d2, fma(d2 + d2, d2, e2));
-                    }
-                    if (num * best_d < best_n * den) {
-                        best_n = num;
-                        best_d = den;
-                    }
-                }
+                const R d2 = ((gx * s_off[3 * j + 0][l]) + (gy * s_off[3 * j + 1][l])) + (gz * s_off[3 * j + 2][l]);
+                lo = d2 < lo ? d2 : lo;
+                hi = d2 > hi ? d2 : hi;
             }
         }
+        R best_n = R(1), best_d = R(1);
+        auto candidate = [&](R d1, R d2) {  // |delta1|, |delta2|
+            if (is_close_zero(d2)) {
+                return;
+            }
+            const R num = (LIM == 1) ? d1 : fma(d1, fma(R(2), d2, d1), e2);
+            const R den = (LIM == 1) ? d2 : fma(d1, d1 + d2, fma(d2 + d2, d2, e2));
+            if (num * best_d < best_n * den) {
+                best_n = num;
+                best_d = den;
+            }
+        };
+        candidate(dmx, hi);
+        candidate(-dmn, -lo);
         psi = best_n / best_d;
     }
     if (FOLD && LIM != 0) {
