@@ -169,13 +169,15 @@ __global__ void __launch_bounds__(GRAD_THREADS, SIDES ? GRAD_MINB_SIDES : GRAD_M
     if (l >= ncell) {
         return;
     }
+    // Slots past a cell's own faces name the cell itself with zero weights and offsets: they add zeros, so only
+    // the exact form and the side records look at the cell's own count.
     const int cnt = MIXED ? s_cnt[l] : MAX_SLOTS;
     const int jmax = MIXED ? s_J : MAX_SLOTS;
     if constexpr (MIXED) {
 #pragma unroll
         for (int j = 0; j < MAX_SLOTS; j++) {
             if (j >= jmax) break;
-            qn[j] = __ldg(qv + ((j < cnt) ? s_nbr[j][l] : c));
+            qn[j] = __ldg(qv + s_nbr[j][l]);
         }
     }
     R gx = R(0), gy = R(0), gz = R(0);
@@ -186,7 +188,7 @@ __global__ void __launch_bounds__(GRAD_THREADS, SIDES ? GRAD_MINB_SIDES : GRAD_M
 #pragma unroll
     for (int j = 0; j < MAX_SLOTS; j++) {
         if (j >= jmax) break;
-        if (j < cnt) {
+        if (!X || j < cnt) {
             R d = R(qn[j] - qc);
             gx += d * s_w[3 * j + 0][l];
             gy += d * s_w[3 * j + 1][l];
@@ -236,11 +238,9 @@ __global__ void __launch_bounds__(GRAD_THREADS, SIDES ? GRAD_MINB_SIDES : GRAD_M
 #pragma unroll
         for (int j = 0; j < MAX_SLOTS; j++) {
             if (j >= jmax) break;
-            if (j < cnt) {
-                const R d2 = ((gx * s_off[3 * j + 0][l]) + (gy * s_off[3 * j + 1][l])) + (gz * s_off[3 * j + 2][l]);
-                lo = d2 < lo ? d2 : lo;
-                hi = d2 > hi ? d2 : hi;
-            }
+            const R d2 = ((gx * s_off[3 * j + 0][l]) + (gy * s_off[3 * j + 1][l])) + (gz * s_off[3 * j + 2][l]);
+            lo = d2 < lo ? d2 : lo;
+            hi = d2 > hi ? d2 : hi;
         }
         R best_n = R(1), best_d = R(1);
         auto candidate = [&](R d1, R d2) {  // |delta1|, |delta2|
