@@ -404,10 +404,14 @@ __global__ void k_redirect(int F, int F_bd, int off_periodic_ghost, const int *_
     lr[f] = make_int2(l, r);
 }
 
-// teal AoS rows [n][5] -> state rows [row0, row0 + n) of the SoA state
-__global__ void k_rows_aos_to_soa(int n, int row0, int N, const double *__restrict__ aos, double *__restrict__ q)
+// teal AoS rows [n][5] -> state rows [row0, row0 + n) of the SoA state; *ref = p0 unless ref is null
+__global__ void k_rows_aos_to_soa(int n, int row0, int N, const double *__restrict__ aos, double *__restrict__ q,
+                                  double *ref, double p0)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0 && ref) {
+        *ref = p0;
+    }
     if (i >= n) {
         return;
     }
@@ -432,19 +436,7 @@ __global__ void k_rows_gather(int n, const int *__restrict__ rowmap, int N, cons
     }
 }
 
-// SoA [5][C] -> AoS [C][5] (derivative) and back
-__global__ void k_soa5_to_aos(int C, const double *__restrict__ soa, double *__restrict__ aos)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= C) {
-        return;
-    }
-#pragma unroll
-    for (int v = 0; v < 5; v++) {
-        aos[(size_t)i * 5 + v] = soa[v * C + i];
-    }
-}
-
+// AoS [C][5] -> SoA [5][C] (a derivative given by the host)
 __global__ void k_aos5_to_soa(int C, const double *__restrict__ aos, double *__restrict__ soa)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;

@@ -262,6 +262,7 @@ struct tg_ctx {
     std::vector<cudaEvent_t> read_ev;  // chunks of a staged read-back
     bool prepared = false;     // U0, dtc and the piece minima valid for the resident state
 
+    int rows_out = 0;  // the next residual is written in teal's rows [C][5]
     // instances the next residuals are evaluated for ([ninst] device flags; null: all), see Mask
     const int *eval_on = nullptr;
 
@@ -285,7 +286,6 @@ struct tg_ctx {
     double *ccenter = nullptr;  // [C][3] cell centres (device source)
     double *S = nullptr;        // [5][C] device source values of the residual being evaluated
     double *pref = nullptr;     // [ninst] reference pressure of the FP32-flux form (Local::dp)
-    std::vector<double> h_pref; // its host copy (the source of each upload stays alive)
     double *dprop = nullptr;    // [3] properties
     const void *src_kernel = nullptr;
     int src_prepare = TG_PREPARE_NONE;
@@ -1027,7 +1027,6 @@ static int create_ctx(MeshInput &in, const tg_equations *e, int precision, tg_ct
         if (precision == TG_PRECISION_FP32_FLUX) {
             TRY(dalloc(&c->pref, c->ninst));
             CU(cudaMemsetAsync(c->pref, 0, sizeof(double) * c->ninst, st));
-            c->h_pref.assign(c->ninst, 0.0);
         }
         CU(cudaMemsetAsync(c->dtc, 0, sizeof(double) * s.C, st));
         TRY(dalloc(&c->part_min, c->npieces));
@@ -1403,15 +1402,12 @@ static int set_rows(tg_ctx *c, int inst, const double *prim, double *q)
     int row0 = c->h_inst_cell_off[inst];
     int n = c->h_inst_cell_off[inst + 1] - row0;
     TRY(h2d(c, c->aos, prim, 5 * (size_t)n));
-    k_rows_aos_to_soa<<<grid_of(n), BLOCK, 0, c->stream>>>(n, row0, c->s.N, c->aos, q);
+    // the FP32-flux form's reference pressure, set by the same launch: the instance's first cell (any
+    // constant cancels over closed cells; a representative one keeps the relative pressures small)
+    const bool ref = q == c->q && c->pref && n > 0;
+    const double p0 = ref && std::isfinite(prim[4]) ? prim[4] : 0.0;
+    k_rows_aos_to_soa<<<grid_of(n), BLOCK, 0, c->stream>>>(n, row0, c->s.N, c->aos, q, ref ? c->pref + inst : nullptr, p0);
     CU(cudaGetLastError());
-    if (q == c->q && c->pref && n > 0) {
-        // the FP32-flux form's reference pressure: the instance's first cell (any constant cancels
-        // over closed cells; a representative one keeps the relative pressures small)
-        double p0 = prim[4];
-        c->h_pref[inst] = std::isfinite(p0) ? p0 : 0.0;
-        CU(cudaMemcpyAsync(c->pref + inst, &c->h_pref[inst], sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    }
     return TG_OK;
 }
 
@@ -1688,7 +1684,7 @@ static void launch_cell_s(tg_ctx *c, double alpha, int last, double *q, double *
     launch_next(k_cell<MODE, NS, GT, SRC, false>, dim3((s.hi - s.lo + CELL_BLOCK - 1) / CELL_BLOCK), dim3(CELL_BLOCK),
                 c->stream,
         s, c->slot_face, c->slot_cnt, cd, (const GT *)c->G, c->U0, q, Rout, c->seg, c->st, alpha, last,
-        props_of(c), c->dtc, src, 0, mask_of(c));
+        props_of(c), c->dtc, src, 0, mask_of(c), c->rows_out);
 }
 
 template <int MODE, bool NS, typename GT>
@@ -1726,6 +1722,7 @@ static CellLaunch cell_args(tg_ctx *c, int mode, double alpha, int last, double 
     a.src = Source{{c->src_par[0], c->src_par[1], c->src_par[2], c->src_par[3]},
                    c->source == TG_SOURCE_DEVICE ? c->S : c->src_avg};
     a.mask = mask_of(c);
+    a.rows = c->rows_out;
     return a;
 }
 
@@ -1947,9 +1944,10 @@ extern "C" int tg_derivative(tg_ctx *c, const double *prim, double *deriv, doubl
         q = c->qs;
         TRY(set_rows(c, 0, prim, q));
     }
-    TRY(run_residual<0>(c, q, c->R, false));
-    k_soa5_to_aos<<<grid_of(c->s.C), BLOCK, 0, c->stream>>>(c->s.C, c->R, c->aos);
-    CU(cudaGetLastError());
+    c->rows_out = 1;  // straight into the rows that go to the host
+    const int rc = run_residual<0>(c, q, c->aos, false);
+    c->rows_out = 0;
+    TRY(rc);
     TRY(read_steps_async(c));
     TRY(d2h(c, deriv, c->aos, 5 * (size_t)c->s.C));
     TRY(check_error(c));

@@ -512,7 +512,7 @@ __global__ void __launch_bounds__(SIDE_TILE, 4) k_cell_fluxes(FaceLaunch a, Geom
     for (int v = 0; v < 5; v++) {
         r[v] = -s_sum[v][lane] * ivol;
     }
-    finish_cell(b.mode, b.ns, s.C, s.N, c, r, act, b.alpha, step, b.last, b.prop, b.cd, b.U0, b.q, b.Rout, b.dtc);
+    finish_cell(b.mode, b.ns, s.C, s.N, c, r, act, b.alpha, step, b.last, b.rows, b.prop, b.cd, b.U0, b.q, b.Rout, b.dtc);
 }
 
 // whether a residual leaves out face c: both cells lie in one instance, and a partition's faces may have

@@ -340,17 +340,17 @@ __device__ __forceinline__ void add_source(const Source &src, const Prim<double>
     }
 }
 
-// what follows the sum of a cell's fluxes: R kept (mode 0, last stage), the stage update U = U0 + R * alpha *
+// what follows the sum of a cell's fluxes: R kept (mode 0, with `rows` in teal's [C][5]; last stage), the stage update U = U0 + R * alpha *
 // step and q = prim(U) (mode 1), and on the last stage U0 and the cell's stable step of the new state
 __device__ __forceinline__ void finish_cell(int mode, bool ns, int C, int N, int c, const double (&r)[5], int act,
-                                            double alpha, double step, int last, const Props &prop,
+                                            double alpha, double step, int last, int rows, const Props &prop,
                                             const CellData &cd, double *__restrict__ U0, double *__restrict__ q,
                                             double *__restrict__ Rout, double *__restrict__ dtc)
 {
     if (mode == 0 || last) {
 #pragma unroll
         for (int v = 0; v < 5; v++) {
-            Rout[v * C + c] = r[v];
+            Rout[mode == 0 && rows ? (size_t)5 * c + v : (size_t)v * C + c] = r[v];
         }
     }
     if (mode == 0) {
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(CELL_BLOCK, cell_minb<GT>()) k_cell(Sizes s, c
                                                 const GT *__restrict__ G, double *__restrict__ U0,
                                                 double *__restrict__ q, double *__restrict__ Rout,
                                                 Segments seg, Steps st, double alpha, int last, Props prop,
-                                                double *__restrict__ dtc, Source src, int two, Mask mask)
+                                                double *__restrict__ dtc, Source src, int two, Mask mask, int rows)
 {
     static_assert(X == kExact, "exact kernels live in the exact translation units only");
     // nothing is read ahead of the wait: the slot indices held across it cost registers (spills at 40)
@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(CELL_BLOCK, cell_minb<GT>()) k_cell(Sizes s, c
         Prim<double> qc{q[c], v3(q[N + c], q[2 * N + c], q[3 * N + c]), q[4 * N + c]};
         add_source<SRC>(src, qc, __ldg(seg.cell_inst + c), r);
     }
-    finish_cell(MODE, NS, C, N, c, r, act, alpha, step, last, prop, cd, U0, q, Rout, dtc);
+    finish_cell(MODE, NS, C, N, c, r, act, alpha, step, last, rows, prop, cd, U0, q, Rout, dtc);
 }
 
 // U0 = cons(q) and the stable time step of every cell (start of a run / after the host changed
@@ -554,6 +554,7 @@ struct CellLaunch {
     double *dtc;
     Source src;
     Mask mask;
+    int rows;  // mode 0: R in teal's rows [C][5]
 };
 
 struct BoundaryLaunch {

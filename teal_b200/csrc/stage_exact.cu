@@ -47,7 +47,7 @@ static void cell_s(const CellLaunch &a, cudaStream_t st)
     if (a.s.hi <= a.s.lo) return;
     k_cell<MODE, NS, double, SRC, true><<<(a.s.hi - a.s.lo + CELL_BLOCK - 1) / CELL_BLOCK, CELL_BLOCK, 0, st>>>(
         a.s, a.slot_face, a.slot_cnt, a.cd, a.G, a.U0, a.q, a.Rout, a.seg, a.st, a.alpha, a.last, a.prop, a.dtc,
-        a.src, a.two, a.mask);
+        a.src, a.two, a.mask, a.rows);
 }
 
 template <int MODE, bool NS>
