@@ -54,11 +54,11 @@ __host__ __device__ constexpr int side_minb()
     return sizeof(R) == sizeof(float) ? TG_SIDE_MINB_FP32 : TG_SIDE_MINB;
 }
 constexpr int CELL_BLOCK = TG_CELL_BLOCK;
-// resident cell-gather blocks per SM, FP64 or FP32 flux records
+// resident cell-gather blocks per SM: a bare residual (mode 0), else FP64 or FP32 flux records
 template <typename GT>
-__host__ __device__ constexpr int cell_minb()
+__host__ __device__ constexpr int cell_minb(int mode)
 {
-    return sizeof(GT) == sizeof(float) ? TG_CELL_MINB_FP32 : TG_CELL_MINB;
+    return mode == 0 ? TG_CELL_MINB_RESIDUAL : sizeof(GT) == sizeof(float) ? TG_CELL_MINB_FP32 : TG_CELL_MINB;
 }
 constexpr int GRAD_MINB = TG_GRAD_MINB;
 constexpr int GRAD_MINB_SIDES = TG_GRAD_MINB_SIDES;

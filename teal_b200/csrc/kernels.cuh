@@ -384,7 +384,7 @@ __device__ __forceinline__ void finish_cell(int mode, bool ns, int C, int N, int
 // X (exact translation units): with `two` (a viscous flux), the viscous records (second set) are summed
 // before the convective ones, the order of teal's two face loops, and R = -sum / V is a quotient.
 template <int MODE, bool NS, typename GT, int SRC, bool X>
-__global__ void __launch_bounds__(CELL_BLOCK, cell_minb<GT>()) k_cell(Sizes s, const int *__restrict__ slot_face,
+__global__ void __launch_bounds__(CELL_BLOCK, cell_minb<GT>(MODE)) k_cell(Sizes s, const int *__restrict__ slot_face,
                                                 const uint8_t *__restrict__ slot_cnt, CellData cd,
                                                 const GT *__restrict__ G, double *__restrict__ U0,
                                                 double *__restrict__ q, double *__restrict__ Rout,

@@ -40,6 +40,9 @@
 #ifndef TG_CELL_MINB
 #define TG_CELL_MINB 10  // cell-gather blocks kept resident per SM (caps registers per thread)
 #endif
+#ifndef TG_CELL_MINB_RESIDUAL
+#define TG_CELL_MINB_RESIDUAL 8  // the same for a bare residual (derivative calls, implicit steps)
+#endif
 #ifndef TG_CELL_MINB_FP32
 #define TG_CELL_MINB_FP32 12  // the same in the FP32-flux form
 #endif
