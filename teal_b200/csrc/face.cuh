@@ -223,7 +223,8 @@ __device__ __forceinline__ Cons<R> viscous_face(const Geo &geo, int i, bool boun
 // convective flux follows. `column`: this thread's shared-memory column (FP32-flux form). Measured
 // against two passes at 96 / 64 registers, TGV 128^3: FP64 0.467 -> 0.421 ms (0.464 at 96 registers with
 // the states in shared memory, 0.438 at 80), FP32-flux 0.301 -> 0.267 ms (0.275-0.298 at fewer
-// resident blocks).
+// resident blocks). The exact form, whose viscous record is of its own, stores it before the convective flux:
+// kept across it, its face kernel took 0.593 ms, so 0.580.
 template <typename R, int FK, bool FOLD, typename Geo>
 __device__ __forceinline__ void face_flux_ns(const Geo &geo, int i, int f, const Sizes &s,
                                              const double *__restrict__ q, const R *__restrict__ rec, R gamma, R ig,
@@ -241,6 +242,11 @@ __device__ __forceinline__ void face_flux_ns(const Geo &geo, int i, int f, const
     }
     Sides<R> sides(column);
     const Cons<R> fv = viscous_face<R, FOLD>(geo, i, boundary, c, s.N, q, rec, pref, gamma, mu, prandtl, sides);
+    if constexpr (kExact) {
+        const R area = geo.area(i);
+        const R gv[5] = {fv.rho * area, fv.m.x * area, fv.m.y * area, fv.m.z * area, fv.e * area};
+        flux_rec_store(G + flux_rec2_offset(s.F), s.F, f, gv);
+    }
     R pl[5], pr[5];
 #pragma unroll
     for (int v = 0; v < 5; v++) {
@@ -271,11 +277,7 @@ __device__ __forceinline__ void face_flux_ns(const Geo &geo, int i, int f, const
     }
     const R area = geo.area(i);
     R gf[5] = {fc.rho * area, fc.m.x * area, fc.m.y * area, fc.m.z * area, fc.e * area};
-    if constexpr (kExact) {
-        const R gv[5] = {fv.rho * area, fv.m.x * area, fv.m.y * area, fv.m.z * area, fv.e * area};
-        flux_rec_store(G + flux_rec2_offset(s.F), s.F, f, gv);
-    }
-    else {
+    if constexpr (!kExact) {
         gf[0] -= fv.rho * area;
         gf[1] -= fv.m.x * area;
         gf[2] -= fv.m.y * area;
