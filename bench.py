@@ -85,13 +85,21 @@ def kernel_bytes(C, F, S, NB, ns=True, fold=False, g=8, basis=3):
     gradient / geometry / flux-record element size (8 in FP64, 4 in the FP32-flux form), basis the
     basis rows a face reads (3: the normal, the plain forms; 9 in the exact form)."""
     grad_state = (15 + (0 if fold else 5)) * g
-    return {
+    if not ns and basis == 3:
+        # side records (the plain forms without a viscous flux): 5 values written per slot, two slots'
+        # values read per face, no offsets and no cell gathers but the boundary ghosts
+        gradient = 40 * (C + NB) + (4 + 6 * g) * S + 9 * C + 5 * g * S
+        face = (8 + (1 + basis + 10 + 5) * g) * F + 40 * NB
+    else:
         # q of cells and boundary ghosts, per slot: neighbour 4 + weight 3 g + offset 3 g; counts,
         # eps^2; writes gradient (+ limiter factors)
-        "gradient": 40 * (C + NB) + (4 + 6 * g) * S + 9 * C + grad_state * C,
+        gradient = 40 * (C + NB) + (4 + 6 * g) * S + 9 * C + grad_state * C
         # per face: cells 8, area, basis rows, offsets (+ correction), G write 5 g; per cell: q,
         # gradient (+ psi); ghost rows
-        "face": (8 + (1 + basis + 6 + 5 + (4 if ns else 0)) * g) * F + (40 + grad_state) * C + 40 * NB,
+        face = (8 + (1 + basis + 6 + 5 + (4 if ns else 0)) * g) * F + (40 + grad_state) * C + 40 * NB
+    return {
+        "gradient": gradient,
+        "face": face,
         # slot face indices, G read once, U0, volume, q write (last stage adds R, U0, projection)
         "cell": 4 * S + 1 * C + 5 * g * F + (40 + 8 + 40) * C,
     }

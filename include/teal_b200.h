@@ -239,7 +239,8 @@ int tg_advance(tg_ctx *ctx, int method, const void *context, double courant, dou
  * cells and each chunk's rows are copied to the host as soon as they are final. The results are
  * the bits of the three calls in sequence. prim_in (its first num_inner rows of 5) or null (the
  * resident state), prim_out [num_cells][5] or null. Pageable prim_out, the implicit method and
- * partitions run the three calls in sequence. The first chunked call builds the context's chunk plan
+ * partitions run the three calls in sequence; a mesh below two chunks (262,144 cells) takes its step whole,
+ * the copy behind it. The first chunked call builds the context's chunk plan
  * (one host pass over the faces). This is the work of teal's Advance (src/simulation.h:6-7) on
  * eqns->primitive.data, which the drop-in methods (tg_teal_*) call. */
 int tg_advance_host(tg_ctx *ctx, int method, const void *context, double courant, double *time,

@@ -17,6 +17,7 @@ import concurrent.futures
 import itertools
 import json
 import os
+import re
 import subprocess
 import sys
 import tempfile
@@ -113,16 +114,13 @@ def write_header(path, best):
              "// fewer resident face blocks, i.e. more registers per thread). A value given with -D at build",
              "// time wins.",
              "#pragma once", ""]
-    notes = {"TG_FACE_BLOCK": "threads per face-flux block",
-             "TG_FACE_MINB": "Navier-Stokes face-flux blocks kept resident per SM (caps registers per thread)",
-             "TG_FACE_MINB_EULER": "Euler face-flux blocks kept resident per SM (caps registers per thread)",
-             "TG_FACE_MINB_FP32": "FP32-flux face-flux blocks kept resident per SM (caps registers per thread)",
-             "TG_CELL_BLOCK": "threads per cell-gather block",
-             "TG_CELL_MINB": "cell-gather blocks kept resident per SM (caps registers per thread)",
-             "TG_FACE_STAGED_EULER": "Euler face kernel: geometry staged by bulk copies (1) or loaded (0)",
-             "TG_GRAD_MINB": "gradient blocks (160 threads) kept resident per SM (caps registers per thread)"}
+    # shapes that no sweep covers keep their values and notes
+    with open(os.path.join(CSRC, "tuned.h")) as f:
+        entries = {k: [v, note] for k, v, note in re.findall(r"#define (TG_\w+) (\d+)  // (.*)", f.read())}
     for k, v in best.items():
-        lines += [f"#ifndef {k}", f"#define {k} {v}  // {notes[k]}", "#endif"]
+        entries.setdefault(k, [v, k])[0] = v
+    for k, (v, note) in entries.items():
+        lines += [f"#ifndef {k}", f"#define {k} {v}  // {note}", "#endif"]
     with open(path, "w") as f:
         f.write("\n".join(lines) + "\n")
 

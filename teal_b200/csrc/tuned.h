@@ -1,10 +1,10 @@
 // Launch shapes of the hot kernels, chosen by teal_b200/autotune.py on a B200 (fastest measured RK
 // step: TGV for the face, cell and gradient shapes, the ramp for the Euler staging switch and the
 // Euler face occupancy; times within 0.5 % of the fastest
-// count as ties, resolved to fewer resident face blocks, i.e. more registers per thread). From the
-// later sweeps: cell 0.113 vs 0.133 ms per TGV 128^3 launch, gradient 0.264 vs 0.280 ms, Euler face
-// 0.271 ms at 28 blocks against 0.290 at 24 and 0.318 at 20 (ramp 80^3), FP32-flux face 0.309 ms at
-// 32 blocks against 0.326 at 20 (TGV 128^3). A value given with -D at build time wins.
+// count as ties, resolved to fewer resident face blocks, i.e. more registers per thread), and by single
+// sweeps for the shapes it does not cover. Per launch at TGV 128^3: Navier-Stokes face 0.401 ms at 16
+// blocks, 0.414 at 20, 0.445 at 12, 0.453 at 24; FP32-flux face 0.309 ms at 32 blocks against 0.326 at 20;
+// gradient 0.264 against 0.280 ms at 9 (both before its tiles); a value given with -D at build time wins.
 #pragma once
 
 #ifndef TG_FACE_BLOCK

@@ -14,7 +14,7 @@ from tests.cases import taylor_green, vortex
 
 pytestmark = pytest.mark.gpu
 
-# Both paths sum the same products in the same order (pieces of 4096 cells, the same block shapes),
+# Both paths sum the same products in the same order (the same pieces, the same block shapes),
 # so the results are compared bit for bit.
 
 
@@ -58,7 +58,7 @@ def test_noalloc_residual_vortex_one_piece():
 
 
 def test_noalloc_residual_taylor_green_ragged_pieces():
-    # 30^3 = 27000 cells: six full pieces of 4096 cells and a ragged seventh
+    # 30^3 = 27000 cells: 105 full pieces of 256 cells and a ragged one
     m = tb.Mesh.create((0, 0, 0), (2 * np.pi,) * 3, (30, 30, 30), (1, 1, 1))
     e = tb.Equations.navierstokes(m)
     e.set_convective_flux("roe")
