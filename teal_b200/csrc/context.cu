@@ -2556,7 +2556,7 @@ static int while_end(tg_ctx *c, WhileLoop &w)
 
 // derivative of a primitive state q (boundary rows refreshed) into Rout, with the kernels of
 // `precision` (the context's own, or FP64 for the FP32-flux form's Newton residuals), for the instances
-// whose flag `which` (GmresFlag) is set
+// whose flag `which` (GmresFlag) is set; without Rout the fluxes alone
 static int gm_derivative(tg_ctx *c, double *q, double *Rout, int precision, int which)
 {
     // implicit Euler evaluates every residual at the end of the step, time + step (advance.c:144)
@@ -2565,7 +2565,7 @@ static int gm_derivative(tg_ctx *c, double *q, double *Rout, int precision, int 
     c->precision = precision;
     // one mesh is in its loops as long as they run
     c->eval_on = c->ninst > 1 ? c->gm.flag + (size_t)which * c->ninst : nullptr;
-    const int rc = run_residual<0>(c, q, Rout, false);
+    const int rc = Rout ? run_residual<0>(c, q, Rout, false) : run_fluxes(c, q);
     c->eval_on = nullptr;
     c->precision = own;
     return rc;
@@ -2593,9 +2593,12 @@ static int gm_solve(tg_ctx *c, const GmresBatch &gb)
     // matvec (gmres.c:12-50); it differences two residuals of the same precision (gmres.c:41-46)
     k_krylov_vector<<<cb, BLOCK, 0, c->stream>>>(C, c->s.N, g.U, g.r, g.w, gb, c->prop[0], g.V, g.q1);
     CU(cudaGetLastError());
-    TRY(gm_derivative(c, g.q1, g.R1, c->precision, GF_ARNOLDI));
-    CU(launch_next(k_arnoldi_dots, dim3(c->npieces), dim3(KRYLOV_BLOCK), c->stream, C, g.V, g.R1, g.Rm ? g.Rm : c->R, gb,
-                   g.w));
+    // the first pass sums FP32 fluxes itself (k_arnoldi_dots) where the cell kernel would do nothing else
+    const bool gather = !is_fp64(c) && c->source == TG_SOURCE_NONE && !use_fused(c);
+    TRY(gm_derivative(c, g.q1, gather ? nullptr : g.R1, c->precision, GF_ARNOLDI));
+    CU(launch_next(gather ? k_arnoldi_dots<true> : k_arnoldi_dots<false>, dim3(c->npieces), dim3(KRYLOV_BLOCK), c->stream,
+                   c->s, c->slot_face, c->slot_cnt, c->volume, gather ? (const float *)c->G : nullptr, g.V, g.R1,
+                   g.Rm ? g.Rm : c->R, gb, g.w));
     CU(launch_next(k_arnoldi_update, dim3(c->npieces), dim3(KRYLOV_BLOCK), c->stream, C, g.V, gb, g.w, arnoldi.h));
     c->launches += 3;
     TRY(while_end(c, arnoldi));

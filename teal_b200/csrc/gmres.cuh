@@ -338,7 +338,14 @@ __device__ __forceinline__ double warp_sum8(double (&a)[8], int lane)
 // KRYLOV_GROUP basis vectors are in flight together and their 2 x KRYLOV_GROUP products are
 // summed over the warp at once. Four blocks an SM (64 registers) hold all pieces of an instance at once:
 // two implicit steps of 123 k cells 6.55 ms, 6.89 with three.
-__global__ void __launch_bounds__(KRYLOV_BLOCK, 4) k_arnoldi_dots(int C, const double *__restrict__ V,
+// GATHER: R1 is not read but summed here from the FP32 flux records (k_cell's sum): a launch and the round trip of
+// R1 less per column; two implicit steps of six ramps 2.47 -> 2.39 ms. FP64 records (60 registers for a cell's
+// six) gain nothing: 37 k cells 1.970 ms either way with spills at four blocks, 123 k cells 6.28 -> 6.89 at three.
+template <bool GATHER>
+__global__ void __launch_bounds__(KRYLOV_BLOCK, 4) k_arnoldi_dots(Sizes sz, const int *__restrict__ slot_face,
+                                                                  const uint8_t *__restrict__ slot_cnt,
+                                                                  const double *__restrict__ volume,
+                                                                  const float *__restrict__ G, const double *__restrict__ V,
                                                                   const double *__restrict__ R1,
                                                                   const double *__restrict__ R, GmresBatch gb,
                                                                   double *__restrict__ w)
@@ -347,9 +354,11 @@ __global__ void __launch_bounds__(KRYLOV_BLOCK, 4) k_arnoldi_dots(int C, const d
     __shared__ double acc[WARPS][2 * KRYLOV_TILE];
     let_next_start();
     wait_for_previous();
+    G = after_wait(G);
     V = after_wait(V);
     R1 = after_wait(R1);
     R = after_wait(R);
+    const int C = sz.C;
     const int beg = gb.seg.piece_beg[blockIdx.x], end = gb.seg.piece_beg[blockIdx.x + 1];
     const int inst = gb.seg.cell_inst[beg];
     if (!gb.arnoldi(inst)) {
@@ -370,7 +379,16 @@ __global__ void __launch_bounds__(KRYLOV_BLOCK, 4) k_arnoldi_dots(int C, const d
         for (int c0 = beg + 32 * warp; c0 < end; c0 += KRYLOV_BLOCK) {
             const int c = c0 + lane;
             const bool in = c < end;
-            double x[5], vk[5];
+            double x[5], vk[5], r1[5];
+            if (GATHER && in && i0 == 0) {
+                double acc[5];
+                sum_fluxes(sz, slot_face, slot_cnt, G, c, acc);
+                const double ivol = 1.0 / __ldg(volume + c);
+#pragma unroll
+                for (int v = 0; v < 5; v++) {
+                    r1[v] = mul_rn(-acc[v], ivol);  // rounded as k_cell stores it
+                }
+            }
 #pragma unroll
             for (int v = 0; v < 5; v++) {
                 const size_t j = (size_t)v * C + c;
@@ -378,7 +396,7 @@ __global__ void __launch_bounds__(KRYLOV_BLOCK, 4) k_arnoldi_dots(int C, const d
                 if (in) {
                     vk[v] = V[(size_t)k * n + j];
                     if (i0 == 0) {
-                        x[v] = vk[v] - ((step * (R1[j] - R[j])) / eps);
+                        x[v] = vk[v] - ((step * ((GATHER ? r1[v] : R1[j]) - R[j])) / eps);
                         w[j] = x[v];
                     }
                     else {

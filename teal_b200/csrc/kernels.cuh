@@ -340,6 +340,37 @@ __device__ __forceinline__ void add_source(const Source &src, const Prim<double>
     }
 }
 
+// sum of a cell's flux records in slot order: all slot indices first, then every record in flight at once
+template <typename GT>
+__device__ __forceinline__ void sum_fluxes(const Sizes &s, const int *__restrict__ slot_face,
+                                           const uint8_t *__restrict__ slot_cnt, const GT *G, int c, double (&acc)[5])
+{
+    const int cnt = slot_cnt[c];
+    int sf[MAX_SLOTS];
+#pragma unroll
+    for (int j = 0; j < MAX_SLOTS; j++) {
+        sf[j] = (j < cnt) ? __ldg(slot_face + j * s.SL + c) : 0;
+    }
+    double gv[MAX_SLOTS][5];
+#pragma unroll
+    for (int j = 0; j < MAX_SLOTS; j++) {
+        flux_rec_load(G, s.F, (j < cnt) ? (sf[j] >= 0 ? sf[j] : ~sf[j]) : 0, gv[j]);
+    }
+#pragma unroll
+    for (int v = 0; v < 5; v++) {
+        acc[v] = 0;
+    }
+#pragma unroll
+    for (int j = 0; j < MAX_SLOTS; j++) {
+        if (j < cnt) {
+#pragma unroll
+            for (int v = 0; v < 5; v++) {
+                acc[v] = (sf[j] >= 0) ? (acc[v] + gv[j][v]) : (acc[v] - gv[j][v]);
+            }
+        }
+    }
+}
+
 // what follows the sum of a cell's fluxes: R kept (mode 0, with `rows` in teal's [C][5]; last stage), the stage update U = U0 + R * alpha *
 // step and q = prim(U) (mode 1), and on the last stage U0 and the cell's stable step of the new state
 __device__ __forceinline__ void finish_cell(int mode, bool ns, int C, int N, int c, const double (&r)[5], int act,
@@ -451,28 +482,8 @@ __global__ void __launch_bounds__(CELL_BLOCK, cell_minb<GT>(MODE)) k_cell(Sizes 
         }
     }
     else {
-        // all slot indices first, then every face record in flight at once; sums in slot order
-        double acc[5] = {0, 0, 0, 0, 0};
-        const int cnt = slot_cnt[c];
-        int sf[MAX_SLOTS];
-#pragma unroll
-        for (int j = 0; j < MAX_SLOTS; j++) {
-            sf[j] = (j < cnt) ? __ldg(slot_face + j * s.SL + c) : 0;
-        }
-        double gv[MAX_SLOTS][5];
-#pragma unroll
-        for (int j = 0; j < MAX_SLOTS; j++) {
-            flux_rec_load(G, s.F, (j < cnt) ? (sf[j] >= 0 ? sf[j] : ~sf[j]) : 0, gv[j]);
-        }
-#pragma unroll
-        for (int j = 0; j < MAX_SLOTS; j++) {
-            if (j < cnt) {
-#pragma unroll
-                for (int v = 0; v < 5; v++) {
-                    acc[v] = (sf[j] >= 0) ? (acc[v] + gv[j][v]) : (acc[v] - gv[j][v]);
-                }
-            }
-        }
+        double acc[5];
+        sum_fluxes(s, slot_face, slot_cnt, G, c, acc);
         const double ivol = 1.0 / __ldg(cd.volume + c);  // one reciprocal for the five components
 #pragma unroll
         for (int v = 0; v < 5; v++) {
