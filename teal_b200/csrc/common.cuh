@@ -20,8 +20,8 @@ constexpr int BLOCK = 256;
 // A kernel launched with launch_next (launch.cuh) may start while the kernel before it drains: its blocks
 // read what no kernel writes (connectivity, geometry) and then wait for that kernel to complete. The
 // pointers of everything else are passed through after_wait, so that no load of it, read-only ones
-// included, can be moved above the wait. Every thread of every block waits, so that completion carries
-// over from one kernel to the next.
+// included, can be moved above the wait. Flags that leave out instances (Mask, an active flag) are such
+// data too. Every thread of every block waits, so that completion carries over from one kernel to the next.
 __device__ __forceinline__ void let_next_start()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -108,6 +108,11 @@ struct PressureRef {
     const int *cell_inst;   // [C]
     __device__ __forceinline__ double of(int c) const { return pref ? __ldg(pref + __ldg(cell_inst + c)) : 0.0; }
 };
+__device__ __forceinline__ PressureRef after_wait(PressureRef r)
+{
+    r.pref = after_wait(r.pref);
+    return r;
+}
 
 // the reference-pressure argument of a face kernel in precision R
 template <typename R>

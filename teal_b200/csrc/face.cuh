@@ -238,7 +238,7 @@ __device__ __forceinline__ void face_flux_ns(const Geo &geo, int i, int f, const
     rec = after_wait(rec);
     double pref = 0.0;
     if constexpr (sizeof(R) == sizeof(float)) {
-        pref = pr_ref.of(c.x);
+        pref = after_wait(pr_ref).of(c.x);
     }
     Sides<R> sides(column);
     const Cons<R> fv = viscous_face<R, FOLD>(geo, i, boundary, c, s.N, q, rec, pref, gamma, mu, prandtl, sides);
@@ -307,7 +307,7 @@ __device__ __forceinline__ void face_flux(const Geo &geo, int i, int f, const Si
     // difference is taken in FP64, before the rounding to FP32
     double pref = 0.0;
     if constexpr (sizeof(R) == sizeof(float)) {
-        pref = pr_ref.of(c.x);
+        pref = after_wait(pr_ref).of(c.x);
     }
 
     // convective flux: the basis and the cell states are dead while the flux runs in the face frame
@@ -376,7 +376,7 @@ __device__ __forceinline__ void side_flux(const Sizes &s, const Geometry<R> &g, 
     double pref = 0.0;
     R pl[5], pr[5];
     if constexpr (sizeof(R) == sizeof(float)) {
-        pref = pr_ref.of(side_cell(l >= 0 ? l : r));
+        pref = after_wait(pr_ref).of(side_cell(l >= 0 ? l : r));
     }
     auto row_state = [&](int row) {
         if constexpr (sizeof(R) == sizeof(float)) {
@@ -542,9 +542,11 @@ __global__ void __launch_bounds__(FACE_BLOCK, face_minb<R>(NS)) k_face(Sizes s, 
         return;
     }
     DirectGeo<R> geo{g, s.F, f};
-    if (M && left_out(mask, geo.cells(0), s.C)) {
+    if (M) {
         wait_for_previous();
-        return;
+        if (left_out(mask, geo.cells(0), s.C)) {
+            return;
+        }
     }
     if constexpr (NS && ORDER == 2) {
         __shared__ R aside[sizeof(R) == sizeof(float) ? 10 * FACE_BLOCK : 1];
@@ -576,10 +578,8 @@ __global__ void __launch_bounds__(FACE_BLOCK, face_minb<R>(false)) k_face_staged
         wait_for_previous();
         return;
     }
-    if (threadIdx.x >= n || (mask.on && left_out(mask, t.cells(threadIdx.x), s.C))) {
-        wait_for_previous();
-    }
-    else {
+    wait_for_previous();
+    if (threadIdx.x < n && !(mask.on && left_out(mask, t.cells(threadIdx.x), s.C))) {
         face_flux<R, FK, ORDER, FOLD>(t, threadIdx.x, f0 + threadIdx.x, s, q, rec, gamma, G,
                                           pr_ref);
     }

@@ -26,6 +26,7 @@ __global__ void k_boundary(Sizes s, const int2 *__restrict__ lr, const double *_
     const int2 c = f < s.F_bd ? lr[f] : make_int2(0, 0);
     wait_for_previous();
     q = after_wait(q);
+    active = after_wait(active);
     if (f >= s.F_bd) {
         return;
     }
@@ -96,9 +97,11 @@ __global__ void __launch_bounds__(GRAD_THREADS, SIDES ? GRAD_MINB_SIDES : GRAD_M
     const int l = threadIdx.x % GRAD_CELLS;
     const int c = base + min(l, ncell - 1);
     let_next_start();
-    if (mask.on && !__any_sync(0xffffffffu, !mask.leaves_out(c))) {  // the same cells in every warp
+    if (mask.on) {  // flags of an earlier kernel: behind the wait, and before copies that a block would have to await
         wait_for_previous();
-        return;
+        if (!__any_sync(0xffffffffu, !mask.leaves_out(c))) {  // the same cells in every warp
+            return;
+        }
     }
     int row[MIXED ? 1 : MAX_SLOTS];
     if constexpr (MIXED) {
@@ -266,7 +269,7 @@ __global__ void __launch_bounds__(GRAD_THREADS, SIDES ? GRAD_MINB_SIDES : GRAD_M
     if constexpr (SIDES) {
         double p0 = 0.0;
         if constexpr (sizeof(R) == sizeof(float)) {
-            p0 = (v == 4) ? pr_ref.of(c) : 0.0;  // pressures relative to the reference (Local::dp)
+            p0 = (v == 4) ? after_wait(pr_ref).of(c) : 0.0;  // pressures relative to the reference (Local::dp)
         }
         const R q0 = R(qc - p0);
         R *row_out = side.rec + (size_t)v * side_elements(s.SL) + (size_t)tile * SIDE_TILE;
