@@ -366,7 +366,9 @@ __device__ __forceinline__ void face_flux(const Geo &geo, int i, int f, const Si
 
 // Flux record of face f between two side records (k_gradient SIDES): the reconstructed states are read,
 // not formed, so a face costs two records, its normal and its area, and no gather of states or gradients.
-// l, r: the face's Geometry::sides.
+// l, r: the face's Geometry::sides. The states of inner cells are not read: the cells of k_cell_fluxes are
+// updated in place while other blocks still form their fluxes. A periodic owner's side comes from its
+// record alone; state rows that are read (boundary ghosts, a partition's halo) no cell update writes.
 template <typename R, int FK>
 __device__ __forceinline__ void side_flux(const Sizes &s, const Geometry<R> &g, int f, int l, int r, V3<R> n, R area,
                                           const double *__restrict__ q, const R *__restrict__ side,
@@ -398,6 +400,15 @@ __device__ __forceinline__ void side_flux(const Sizes &s, const Geometry<R> &g, 
     else if (f >= s.F_in && f < s.F_bd) {  // the ghost state enters unreconstructed (derivative.c:203-211)
         const Prim<R> qr = row_state(~r);
         pr[0] = qr.rho, pr[1] = qr.u.x, pr[2] = qr.u.y, pr[3] = qr.u.z, pr[4] = qr.p;
+    }
+    else if (~r < s.C) {  // a periodic ghost's owner
+        const V3<R> off = load_v3(g.offr, s.F, f);
+#pragma unroll
+        for (int v = 0; v < 5; v++) {
+            R gx, gy, gz, qv;
+            grad_rec_load(rec, ~r, v, gx, gy, gz, qv);
+            pr[v] = at_face(qv, v3(gx, gy, gz), off);
+        }
     }
     else {
         reconstruct<R, true>(row_state(~r), rec, ~r, load_v3(g.offr, s.F, f), pr);

@@ -63,8 +63,9 @@ __global__ void k_boundary(Sizes s, const int2 *__restrict__ lr, const double *_
 // SIDES writes the reconstructed states of the cell's sides instead, q + psi g . offset per slot
 // (derivative.c:158-164; side_index), for the face kernel to read two states of 40 bytes in place of two
 // gradient records, two states and two offsets (448 bytes): the thread has all of it at hand. Cells
-// flagged in SideOut::records store their gradient records as well: periodic faces have no slot in their
-// right cell, whose state is reconstructed with the face's own offset, and a partition sends records.
+// flagged in SideOut::records store a gradient record as well, with the cell's own value in psi's place (psi is
+// multiplied in): periodic faces have no slot in their right cell, whose state is reconstructed from that
+// record and the face's own offset, and a partition sends records.
 template <typename R>
 struct SideOut {
     R *rec = nullptr;                   // side records
@@ -274,7 +275,7 @@ __global__ void __launch_bounds__(GRAD_THREADS, SIDES ? GRAD_MINB_SIDES : GRAD_M
         const R q0 = R(qc - p0);
         R *row_out = side.rec + (size_t)v * side_elements(s.SL) + (size_t)tile * SIDE_TILE;
         if (side.records && ((__ldg(side.records + tile) >> l) & 1u)) {
-            grad_rec_store(rec, c, v, gx, gy, gz, psi);
+            grad_rec_store(rec, c, v, gx, gy, gz, q0);
         }
 #pragma unroll
         for (int j = 0; j < MAX_SLOTS; j++) {

@@ -1,7 +1,8 @@
 """Face fluxes and cell update in one launch (arenas of at most TG_FUSED_CELLS cells) against the two
 launches of larger arenas: a mesh alone takes the first, packed beside a larger one the second, and its
 bits are the same. Sizes around a 32-cell tile, mixed cells, boundaries, both precisions, explicit and
-implicit steps, instances that stop early."""
+implicit steps, instances that stop early; fully periodic boxes of up to the most cells that one launch
+takes, whose tiles do not all start together, over many steps."""
 
 import numpy as np
 import pytest
@@ -53,3 +54,20 @@ def test_alone_equals_packed(large, shape, flux, method, precision):
     assert (t_b[0], it_b[0], it_b[1]) == (t, it, 1)
     assert np.array_equal(res_b[0], res)
     assert np.array_equal(b.get_primitive(0), ctx.get_primitive())
+
+
+@pytest.mark.parametrize("precision", [tb.TG_PRECISION_FP64, tb.TG_PRECISION_FP32_FLUX])
+@pytest.mark.parametrize("shape", [(5, 4, 3), (27, 23, 11), (64, 64, 4), (37, 32, 16), (33, 31, 18), (37, 16, 33)])
+def test_periodic_alone_equals_packed(large, shape, precision):
+    # up to 592 tiles (18,944 cells); 37 x 16 x 33 = 19,536 cells are past the limit
+    mesh = box(shape, (1, 1, 1))
+    small = problem(mesh, "hllc", 1)
+    ctx = small.context(precision)
+    b = tb.Batch([small, problem(large, "hllc", 2)], precision)
+    want = b.run(tb.TG_ADVANCE_LSERK, 0.5, [40, 1])
+    for _ in range(3):
+        ctx.set_primitive(small.primitive)
+        t, it, res = ctx.run(tb.TG_ADVANCE_LSERK, 0.5, 40)
+        assert (t, it) == (want[0][0], want[1][0])
+        assert np.array_equal(res, want[2][0])
+        assert np.array_equal(ctx.get_primitive(), b.get_primitive(0))

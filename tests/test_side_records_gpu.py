@@ -1,7 +1,7 @@
 """Residuals through the side records (second order without a viscous flux) where they can go wrong: cell
 counts that are no multiple of a 32-cell tile, periodic axes two and three cells thick (the periodic
 faces have no slot in their right cell), boundaries, mixed cells whose tiles hold fewer slots. Against the
-CPU restatement (oracle/port.py), and the gradient entry point beside them.
+CPU restatement (oracle/port.py), the gradient entry point beside them, and the states the fluxes may read.
 
 Bars: 1e-12 in FP64, the residual bar of the plain form. The FP32-flux residual rounds states of order one
 to 2^-24 at h of about 1/10, where a residual component is a sum of six face fluxes over h: about
@@ -13,6 +13,7 @@ import pytest
 import teal_b200 as tb
 from oracle import port
 from teal_b200 import meshes
+from teal_b200 import partition as pt
 from tests.cases import rel_l2
 
 pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not port.available(), reason="CPU restatement not built")]
@@ -64,3 +65,28 @@ def test_residual_matches_the_restatement(shape, limiter):
     f = e.context(tb.TG_PRECISION_FP32_FLUX)
     f.set_primitive(prim)
     assert np.linalg.norm(f.derivative() - want) <= 2e-5 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("precision", [tb.TG_PRECISION_FP64, tb.TG_PRECISION_FP32_FLUX])
+@pytest.mark.parametrize("n,periodic", [((7, 5, 3), (1, 1, 1)), ((8, 4, 2), (1, 0, 1)), ((33, 2, 3), (0, 1, 0))])
+def test_fluxes_read_no_inner_state(n, periodic, precision):
+    """The fluxes of a stage come from the records alone: the fused face and cell kernel writes the state
+    while other blocks form theirs. A partition's phases let the state change between the two."""
+    m, e, prim = problem((n, periodic))
+    part = pt.partition(m, np.zeros(m.num_inner_cells, int))[0]
+    other = prim * 1.5
+    other[0, 4] = prim[0, 4]  # the FP32-flux form's reference pressure
+    got = []
+    for change in (False, True):
+        r = pt.Rank(part, e, precision)
+        r.set_state(prim)
+        r.set_step(0.5 * r.step_begin(), 0.0)
+        r.phase(0)
+        r.phase(1)
+        if change:
+            r.set_state(other)
+        r.phase(2, 1.0, 1)
+        got.append(r.state().copy())
+        r.close()
+    assert np.array_equal(got[0], got[1])
+    assert not np.array_equal(got[0], prim[: m.num_inner_cells])
