@@ -297,6 +297,7 @@ struct tg_ctx {
     // step graph cache
     cudaGraphExec_t graph = nullptr;
     int graph_method = -1, graph_stages = 0;
+    const double *graph_alpha = nullptr;  // the coefficient table (one for each time order and stage count)
     double graph_courant = 0;
     int graph_use_max_time = -1;
 
@@ -2058,8 +2059,8 @@ static int launch_step(tg_ctx *c, int stages, const double *alpha, double couran
 static int step_graph(tg_ctx *c, int method, int stages, const double *alpha, double courant, int use_max_time)
 {
     c->st.use_max_time = use_max_time;
-    if (c->graph && c->graph_method == method && c->graph_stages == stages && c->graph_courant == courant &&
-        c->graph_use_max_time == use_max_time) {
+    if (c->graph && c->graph_method == method && c->graph_stages == stages && c->graph_alpha == alpha &&
+        c->graph_courant == courant && c->graph_use_max_time == use_max_time) {
         return TG_OK;
     }
     if (c->graph) {
@@ -2086,6 +2087,7 @@ static int step_graph(tg_ctx *c, int method, int stages, const double *alpha, do
     CU(e2);
     c->graph_method = method;
     c->graph_stages = stages;
+    c->graph_alpha = alpha;
     c->graph_courant = courant;
     c->graph_use_max_time = use_max_time;
     return TG_OK;

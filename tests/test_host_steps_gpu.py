@@ -1,6 +1,6 @@
 """Steps from host state to host state on both sides of the chunk rule (two chunks from 262,144 cells on, below
 that the replayed step with the copy behind it), against the three calls, and after a run loop that left
-an end time behind."""
+an end time behind; steps whose time order changes at the same number of stages."""
 
 import numpy as np
 import pytest
@@ -47,3 +47,29 @@ def test_host_step_after_a_run_with_an_end_time(cells):
     ctx.run(tb.TG_ADVANCE_LSERK, 0.8, 5, max_time=0.5 * step)
     t, again, _ = ctx.advance_host(tb.TG_ADVANCE_LSERK, 0.8, 0.0, e.primitive, out)
     assert (t, again) == (step, step)
+
+
+@pytest.mark.parametrize("how", ["advance", "advance_host", "run"])
+def test_time_order_changes_at_a_fixed_stage_count(how):
+    m = tb.Mesh.create((0, 0, 0), (10, 10, 10), (20, 18, 4), (1, 1, 1))
+    e = tb.Equations.euler(m)
+    e.set_initial_condition("domain", vortex)
+    out = pinned(m.num_cells)
+
+    def state(ctx, rk):
+        if how == "advance_host":
+            ctx.advance_host(tb.TG_ADVANCE_LSERK, 0.8, 0.0, e.primitive, out, context=rk)
+            return out.copy()
+        ctx.set_primitive(e.primitive)
+        if how == "advance":
+            ctx.advance(tb.TG_ADVANCE_LSERK, 0.8, 0.0, context=rk)
+        else:
+            ctx.run(tb.TG_ADVANCE_LSERK, 0.8, 2, context=rk)
+        return ctx.get_primitive()
+
+    orders = [(3, 3), (2, 3), (1, 3), (3, 3)]
+    want = [state(tb.Context(m, e), rk) for rk in orders]  # a context each
+    ctx = e.context()
+    for rk, w in zip(orders, want):
+        assert np.array_equal(state(ctx, rk), w), rk
+    assert not np.array_equal(want[0], want[1])
