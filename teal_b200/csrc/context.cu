@@ -231,7 +231,7 @@ struct tg_ctx {
     int2 *lr = nullptr;
     int2 *sides = nullptr;     // side records of each face (contexts that use them, use_sides)
     unsigned *side_records = nullptr;  // cells whose gradient records are read too, a bit each per gradient tile
-    void *side_rec = nullptr;        // the side records
+    void *side_rec = nullptr;  // the side records
     int *slot_nbr = nullptr, *slot_face = nullptr;
     uint8_t *slot_cnt = nullptr;
     bool full_slots = true;    // every inner cell has MAX_SLOTS faces
@@ -247,7 +247,7 @@ struct tg_ctx {
     // state
     double *q = nullptr, *U0 = nullptr, *R = nullptr;
     double *qs = nullptr;  // scratch state for derivatives of host-given states (allocated on use)
-    void *grad = nullptr, *G = nullptr;  // gradient records [C][5][4], face flux records [F][4] + [F]
+    void *grad = nullptr, *G = nullptr;  // gradient records [N][5][4] (grad_records), face flux records [F][4] + [F]
     double *dtc = nullptr;               // per-cell stable step
     double *part_min = nullptr, *part_sum = nullptr;
     double *sd = nullptr;  // device step doubles [SD_COUNT][ninst]
@@ -756,8 +756,8 @@ static int alloc_geom32(tg_ctx *c)
     const Sizes &s = c->s;
     TRY(dalloc(&c->gb.area32, s.F));
     TRY(dalloc(&c->gb.basis32, 9 * (size_t)s.F));
-    TRY(dalloc(&c->gb.offl32, 3 * (size_t)s.F));
-    TRY(dalloc(&c->gb.offr32, 3 * (size_t)s.F));
+    if (c->gb.offl) TRY(dalloc(&c->gb.offl32, 3 * (size_t)s.F));
+    if (c->gb.offr) TRY(dalloc(&c->gb.offr32, 3 * (size_t)s.F));
     if (c->gb.corr) TRY(dalloc(&c->gb.corr32, 4 * (size_t)s.F));
     return TG_OK;
 }
@@ -935,25 +935,25 @@ static int create_ctx(MeshInput &in, const tg_equations *e, int precision, tg_ct
                 }
                 k_face_rows<<<grid_of(s.F), BLOCK, 0, st>>>(s.F, s.F_in, s.F_bd, s.C, c->lr, c->sides, c->side_records);
                 CU(cudaGetLastError());
-                // FP64 size in every form, as the gradient records
-                double *rec = nullptr;
-                TRY(dalloc(&rec, 5 * side_elements(s.SL)));
-                c->side_rec = rec;
             }
 
             // face geometry, structure of arrays
             TRY(upload(&c->gb.area, m->face_area, s.F, st));
             TRY(dalloc(&d_tmp, 9 * (size_t)s.F > 3 * (size_t)s.C ? 9 * (size_t)s.F : 3 * (size_t)s.C));
             TRY(upload_soa(&c->gb.basis, m->face_basis, s.F, 9, d_tmp, st));
-            std::vector<double> ol(3 * (size_t)s.F), orr(3 * (size_t)s.F);
-            for (int f = 0; f < s.F; f++) {
-                for (int d = 0; d < 3; d++) {
-                    ol[(size_t)f * 3 + d] = m->face_offset[(size_t)f * 6 + d];
-                    orr[(size_t)f * 3 + d] = m->face_offset[(size_t)f * 6 + 3 + d];
+            // With side records only the far sides of periodic faces and a partition's halo are reconstructed at
+            // the face: the other contexts hold no offsets and no gradient records (tg_gradient's go to
+            // the side records' place, grad_records), which makes up for the side records' memory.
+            const bool part = in.halo > 0 || !in.send_rows.empty();
+            auto offsets = [&](double **dst, int side) -> int {
+                std::vector<double> off(3 * (size_t)s.F);
+                for (int f = 0; f < s.F; f++) {
+                    for (int d = 0; d < 3; d++) off[(size_t)f * 3 + d] = m->face_offset[(size_t)f * 6 + 3 * side + d];
                 }
-            }
-            TRY(upload_soa(&c->gb.offl, ol.data(), s.F, 3, d_tmp, st));
-            TRY(upload_soa(&c->gb.offr, orr.data(), s.F, 3, d_tmp, st));
+                return upload_soa(dst, off.data(), s.F, 3, d_tmp, st);
+            };
+            if (!c->sides || part) TRY(offsets(&c->gb.offl, 0));
+            if (!c->sides || c->side_records) TRY(offsets(&c->gb.offr, 1));
             if (e->viscous == TG_VISCOUS_CENTRAL) {
                 TRY(upload_soa(&c->gb.corr, m->face_correction, s.F, 4, d_tmp, st));
             }
@@ -1003,7 +1003,12 @@ static int create_ctx(MeshInput &in, const tg_equations *e, int precision, tg_ct
         TRY(dalloc(&c->U0, 5 * (size_t)s.C));
         TRY(dalloc(&c->R, 5 * (size_t)s.C));
         CU(cudaMemsetAsync(c->R, 0, 5 * sizeof(double) * s.C, st));
-        if (c->order == 2) {
+        if (c->sides) {
+            double *rec = nullptr;
+            TRY(dalloc(&rec, 5 * side_elements(s.SL)));
+            c->side_rec = rec;
+        }
+        if (c->order == 2 && (!c->sides || c->side_records)) {
             // records for every state row: a partition's halo rows receive their owners' records
             CU(cudaMalloc(&c->grad, 20 * rsz * s.N));
         }
@@ -1054,7 +1059,7 @@ static int create_ctx(MeshInput &in, const tg_equations *e, int precision, tg_ct
                       c->si + SI_MAX_ITER * n, c->si + SI_ACTIVE * n,    c->si + SI_FAIL * n, c->si + SI_COUNT * n,
                       c->si + SI_COUNT * n + 1, 0};
         // the residual block is [ninst][5] inside the doubles: SD_RESIDUAL * n .. + 5 n
-        c->aos_len = (size_t)15 * ((size_t)m->num_cells > (size_t)s.F ? (size_t)m->num_cells : (size_t)s.F);
+        c->aos_len = std::max((size_t)15 * s.C, (size_t)5 * m->num_cells);  // gradients, or the rows of a state
         TRY(dalloc(&c->aos, c->aos_len));
         CU(cudaStreamSynchronize(st));
         return TG_OK;
@@ -1539,6 +1544,13 @@ static bool use_sides(const tg_ctx *c)
     return c->order == 2 && c->viscous != TG_VISCOUS_CENTRAL && !is_exact(c) && c->sides;
 }
 
+// the gradient records: their own array, or in contexts whose residuals read none the side records' (five
+// values for each of six slots, more than a cell's twenty)
+static void *grad_records(const tg_ctx *c)
+{
+    return c->grad ? c->grad : c->side_rec;
+}
+
 static PressureRef pressure_ref(const tg_ctx *c)
 {
     return PressureRef{c->precision == TG_PRECISION_FP32_FLUX ? c->pref : nullptr, c->cell_inst};
@@ -1550,7 +1562,7 @@ static void launch_gradient_s(tg_ctx *c, const Geometry<R> &g, bool fold, bool s
     const Sizes s = cell_sizes(c);
     if (s.hi <= s.lo) return;
     dim3 grid((s.hi - s.lo + GRAD_CELLS - 1) / GRAD_CELLS);
-    R *rec = (R *)c->grad;
+    R *rec = (R *)(sides ? c->grad : grad_records(c));
     PressureRefOf<R> pref{};
     if constexpr (sizeof(R) == sizeof(float)) pref = pressure_ref(c);
     auto launch = [&](auto kernel) {
@@ -1968,10 +1980,10 @@ extern "C" int tg_gradient(tg_ctx *c, double time, int limited, double *gradient
     const bool folded = lim == TG_LIMITER_NONE || c->viscous != TG_VISCOUS_CENTRAL;
     int limit = (limited && lim != TG_LIMITER_NONE && !folded) ? 1 : 0;
     if (is_fp64(c))
-        k_grad_to_aos<double><<<grid_of(c->s.C), BLOCK, 0, c->stream>>>(c->s.C, (const double *)c->grad, limit,
+        k_grad_to_aos<double><<<grid_of(c->s.C), BLOCK, 0, c->stream>>>(c->s.C, (const double *)grad_records(c), limit,
                                                                         c->aos);
     else
-        k_grad_to_aos<float><<<grid_of(c->s.C), BLOCK, 0, c->stream>>>(c->s.C, (const float *)c->grad, limit,
+        k_grad_to_aos<float><<<grid_of(c->s.C), BLOCK, 0, c->stream>>>(c->s.C, (const float *)grad_records(c), limit,
                                                                        c->aos);
     CU(cudaGetLastError());
     TRY(d2h(c, gradient, c->aos, 15 * (size_t)c->s.C));

@@ -80,8 +80,7 @@ def memory_estimate(req):
     else:
         nx, ny, nz = req.cells
         faces = 3 * cells + nx * ny + ny * nz + nz * nx
-    # Navier-Stokes: corrections and unlimited gradients; Euler: side records of up to 6 slots
-    per_cell = 700 + (80 if req.physics == _lib.TG_NAVIERSTOKES else 270)
+    per_cell = 700 + (80 if req.physics == _lib.TG_NAVIERSTOKES else 0)
     if req.method == "implicit euler":
         per_cell += 40 * (31 + 8)  # Krylov basis (dimension 30) and the Newton vectors
     return int(per_cell * cells + 450 * faces + (8 << 20))

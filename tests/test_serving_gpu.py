@@ -5,7 +5,7 @@ in shared launches; requests that arrive while others run join the arena between
 re-packed with every running request's exact state and clock), finished ones leave. Every result
 must be the same bits as the request solved alone, whether it ran alone, joined a running batch or
 saw others join and leave around it. `StreamServer` (a context and stream per request) is checked
-the same way.
+the same way. What a context holds on the device stays within the estimate that admits it.
 """
 
 import dataclasses
@@ -119,3 +119,35 @@ def test_cancelled_request_leaves_its_lane():
     assert done[0].error == "cancelled" and done[0].iterations < 200000
     assert not done[1].error and done[1].iterations == 20
     assert server.used == 0
+
+
+@pytest.mark.parametrize("precision", [_lib.TG_PRECISION_FP64, _lib.TG_PRECISION_FP32_FLUX])
+@pytest.mark.parametrize("mesh,cells", [("ramp", (20, 20, 20)), ("channel", (60, 40, 33))])
+@pytest.mark.parametrize("physics", [_lib.TG_EULER, _lib.TG_NAVIERSTOKES])
+def test_contexts_stay_within_the_memory_estimate(physics, mesh, cells, precision):
+    """The estimate counts FP64 contexts; an FP32-flux one holds FP32 copies of the geometry besides, at most
+    4 (17 values a face, 42 a cell). Euler contexts, whose residuals read side records and no gradient
+    records, are admitted with less memory than Navier-Stokes ones."""
+    import torch
+
+    import teal_b200 as tb
+
+    r = serving.Request(id=0, cells=cells, mesh=mesh, physics=physics, precision=precision)
+    eqns = serving.build_problem(r)
+    torch.zeros(1, device="cuda")
+    before = torch.cuda.mem_get_info()[0]
+    ctx = tb.Context(eqns.mesh, eqns, precision)
+    used = before - torch.cuda.mem_get_info()[0]
+    s = eqns.mesh.struct
+    extra = 4 * (17 * s.num_faces + 42 * s.num_inner_cells) if precision == _lib.TG_PRECISION_FP32_FLUX else 0
+    assert used <= serving.memory_estimate(r) + extra
+    euler = dataclasses.replace(r, physics=_lib.TG_EULER)
+    assert serving.memory_estimate(euler) <= serving.memory_estimate(r)
+    assert serving.memory_estimate(dataclasses.replace(r, physics=_lib.TG_NAVIERSTOKES)) > serving.memory_estimate(euler)
+    # gradients share the side records' memory: residuals around them keep their bits
+    ctx.set_primitive(eqns.primitive)
+    d = ctx.derivative()
+    g = ctx.gradient(limited=True)
+    assert np.array_equal(ctx.derivative(), d)
+    assert np.array_equal(ctx.gradient(limited=True), g)
+    ctx.close()
