@@ -1,6 +1,9 @@
 """Steps from host state to host state on both sides of the chunk rule (two chunks from 262,144 cells on, below
 that the replayed step with the copy behind it), against the three calls, and after a run loop that left
-an end time behind; steps whose time order changes at the same number of stages."""
+an end time behind; steps whose time order changes at the same number of stages; read-backs into
+pageable memory."""
+
+import time
 
 import numpy as np
 import pytest
@@ -73,3 +76,32 @@ def test_time_order_changes_at_a_fixed_stage_count(how):
     for rk, w in zip(orders, want):
         assert np.array_equal(state(ctx, rk), w), rk
     assert not np.array_equal(want[0], want[1])
+
+
+# one chunk and a little, several, and more than 64 chunks of 1 MiB (which then grow)
+@pytest.mark.parametrize("cells", [(31, 29, 30), (64, 64, 65), (120, 121, 122)])
+def test_pageable_read_back(cells):
+    m = tb.Mesh.create((0, 0, 0), (10, 10, 10), cells, (1, 1, 1))
+    e = tb.Equations.euler(m)
+    rng = np.random.default_rng(1)
+    e.primitive[:] = 1 + rng.random((m.num_cells, 5))
+    ctx = tb.Context(m, e)
+    ctx.set_primitive(e.primitive)
+    want = pinned(m.num_cells)
+    ctx.get_primitive(want)
+    stream = torch.cuda.Stream()
+    ctx.set_stream(stream.cuda_stream)
+    got = np.empty((m.num_cells, 5))
+    ctx.get_primitive(got)
+    assert np.array_equal(got, want)
+    # while the device still computes, the threads that will copy sleep
+    got[:] = 0
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(600_000_000)  # about 0.3 s
+    wall, cpu = time.perf_counter(), time.process_time()
+    ctx.get_primitive(got)
+    wall, cpu = time.perf_counter() - wall, time.process_time() - cpu
+    assert np.array_equal(got, want)
+    assert wall > 0.1
+    assert cpu < 1.8 * wall  # this thread and the copies; three spinning threads more would be near four
+    ctx.close()
