@@ -1,7 +1,8 @@
 """The Krylov vector passes of the implicit step at the sizes where they can go wrong: cell counts around
-a chunk (KRYLOV_BLOCK = 256 cells), chunks of several cells a thread (above 256 x 296 cells), bases
-that are no multiple of the four vectors loaded together, that fill the Krylov dimension, and that are
-longer than one accumulator tile (64). Against the CPU restatement (oracle/port.py).
+a piece (PIECE_CELLS = 256 cells, one a thread), pieces of several cells a thread (above PIECE_COUNT = 592 of
+them, 151,552 cells), bases that are no multiple of the four vectors loaded together, that fill the
+Krylov dimension, and that are longer than one accumulator tile (64), with one cell a thread and with
+two. Against the CPU restatement (oracle/port.py).
 
 Bar: the implicit bar without a limiter. The restatement's own step moves by 3e-9..9e-9 when its input
 is perturbed by 1e-16 (test_parity_gpu.py states the measurement); 1e-7 is about ten times that."""
@@ -20,12 +21,15 @@ FREE = (1.0, 0.6, 0.1, 0.0, 1.0 / 1.4)
 
 @pytest.mark.skipif(not port.available(), reason="CPU restatement not built")
 @pytest.mark.parametrize("cells,krylov_tol,dim", [
-    ((16, 16, 1), 0.3, 30),      # one full chunk
-    ((33, 8, 1), 0.3, 30),       # a chunk and 8 cells
-    ((7, 5, 3), 1e-3, 5),        # less than a chunk, the Krylov dimension filled
+    ((16, 16, 1), 0.3, 30),      # one full piece
+    ((33, 8, 1), 0.3, 30),       # a piece and 8 cells
+    ((7, 5, 3), 1e-3, 5),        # less than a piece, the Krylov dimension filled
     ((10, 9, 4), 1e-10, 100),    # more columns than an accumulator tile holds
-    ((44, 42, 41), 0.05, 30),    # 75,768 cells: 296 chunks of one cell a thread
-    ((44, 42, 43), 0.05, 30),    # 79,464 cells: two cells a thread
+    ((44, 42, 41), 0.05, 30),    # 75,768 cells: 296 pieces, the last one short
+    ((44, 42, 43), 0.05, 30),    # 79,464 cells: 311 pieces
+    ((37, 64, 64), 0.1, 30),     # 151,552 cells: 592 full pieces, the most of one cell a thread
+    ((53, 52, 55), 0.05, 30),    # 151,580 cells: two cells a thread, 297 pieces, 28 cells in the last
+    ((53, 52, 55), 1e-10, 70),   # the same with more columns than an accumulator tile holds
 ])
 def test_implicit_step_matches_the_restatement(cells, krylov_tol, dim):
     n = np.array(cells)

@@ -1,6 +1,7 @@
 """Step ends (one launch: pieces, instances, stop tests, the next step's start) at the edges of a reduction
-piece: one full piece of 256 cells, a piece and a remainder, less than one, several cells a thread (above
-256 x 296 cells); instances of a batch that stop at different steps."""
+piece: one full piece of 256 cells, a piece and a remainder, less than one, hundreds of pieces, the most
+(592, 151,552 cells), several cells a thread (above that); instances of a batch that stop at different
+steps."""
 
 import numpy as np
 import pytest
@@ -19,7 +20,8 @@ def problem(n):
     return e
 
 
-@pytest.mark.parametrize("n", [(16, 16, 2), (13, 11, 3), (5, 5, 3), (16, 8, 2), (150, 127, 4)])
+@pytest.mark.parametrize("n", [(16, 16, 2), (13, 11, 3), (5, 5, 3), (16, 8, 2), (150, 127, 4), (37, 64, 64), (53, 52, 55),
+                               (90, 83, 61)])
 def test_residual_norm_and_resident_steps(n):
     e = problem(n)
     ctx = e.context()
@@ -27,7 +29,7 @@ def test_residual_norm_and_resident_steps(n):
     vol = e.mesh.cell_volume[:C]
     rng = np.random.default_rng(1)
     d = rng.standard_normal((C, 5)) * 10.0 ** rng.integers(-3, 3, (C, 5))
-    # sums of C non-negative terms in trees: (log2 C + C / (256 pieces x 256 threads)) ulps at most
+    # sums of C non-negative terms in trees: (log2 C + cells a thread) ulps at most
     want = np.sqrt((vol[:, None] * d**2).sum(axis=0) / e.mesh.sum_volume)
     assert np.allclose(ctx.residual(d), want, rtol=1e-14 * np.log2(C))
     # run(k) starts each next step in the launch that ends the last one; k Advance calls start their own
