@@ -5,7 +5,8 @@ cell-gather block size) into a scratch directory,
 times a fixed number of RK steps of a workload on the current GPU with each build (a fresh process
 per build, selected with TEAL_B200_LIBRARY), and writes the fastest shape to
 teal_b200/csrc/tuned.h (and to --out when given). Shapes are tuned on the Taylor-Green vortex, the
-Euler staging switch (face geometry staged by bulk copies or loaded) on the unstructured ramp.
+face kernel between side records on the unstructured ramp, and the face kernel of first-order fluxes
+(staging by bulk copies or not, occupancy) on the ramp at space order 1.
 
     python -m teal_b200.autotune [--n 96] [--ramp-n 64] [--steps 10] [--precision fp64] [--out tuned_candidate.h]
 
@@ -28,18 +29,21 @@ ROOT = os.path.dirname(HERE)
 
 # face-flux block size x resident face threads per SM (65536 registers / threads = the cap per
 # thread: 384 -> 168, 512 -> 128, 640 -> 102, 768 -> 85) x cell-gather block size. The Navier-Stokes
-# workload tunes the shapes; the Euler staging switch (face geometry staged in shared memory by bulk
-# copies or loaded by the threads) is then tuned on the unstructured ramp with the chosen shapes.
+# workload tunes the shapes.
 FACE_BLOCKS = [32, 64, 128]
 FACE_THREADS = [384, 512, 640, 768]
-STAGED = [0, 1]
 CELL_BLOCKS = [256]
 # then cell-gather block size x blocks resident per SM (1536 threads -> 42 registers per thread)
 CELL_SHAPES = [(256, 1), (128, 8), (128, 12), (64, 24)]
 # then gradient blocks (160 threads) resident per SM: 9 leaves the registers free, 12 caps them at 32
 GRAD_MINB = [9, 12]
-# last, on the ramp: resident face threads per SM of the Euler face kernel (fewer registers than the
-# Navier-Stokes one needs)
+# on the ramp: resident blocks (TG_SIDE_BLOCK threads, the same for both precisions) per SM of the face
+# kernel between side records (second order without a viscous flux)
+SIDE_MINB = [5, 6, 7, 8]
+# last, on the ramp at space order 1, whose faces read states: geometry staged in shared memory by bulk
+# copies or loaded by the threads, and resident threads per SM (fewer registers than Navier-Stokes
+# needs). The exact form's second-order Euler faces take the same kernel.
+STAGED = [0, 1]
 EULER_FACE_THREADS = [640, 768, 896, 1024]
 
 TIMER = r"""
@@ -68,6 +72,8 @@ else:
     m = tb.Mesh.from_cells(meshes.ramp_mesh(n=(n, n, n)))
     e = tb.Equations.euler(m)
     e.set_convective_flux("ausmd"); e.set_limiter("minmod", 0.0)
+    if workload == "ramp1":
+        e.set_space_order(1)
     free = (1.0, 2.5, 0.0, 0.0, 1.0 / 1.4)
     e.set_boundary_condition("left", "supersonic inflow", free)
     e.set_boundary_condition("right", "supersonic outflow")
@@ -109,10 +115,10 @@ def time_variant(lib, n, steps, precision, workload="tgv"):
 
 def write_header(path, best):
     lines = ["// Launch shapes of the hot kernels, chosen by teal_b200/autotune.py on a B200 (fastest measured",
-             "// RK step: TGV for the face, cell and gradient shapes, the ramp for the Euler staging switch",
-             "// and the Euler face occupancy; times within 0.5 % of the fastest count as ties, resolved to",
-             "// fewer resident face blocks, i.e. more registers per thread). A value given with -D at build",
-             "// time wins.",
+             "// RK step: TGV for the face, cell and gradient shapes, the ramp for the side-record face kernel,",
+             "// the ramp at space order 1 for the Euler staging switch and the Euler face occupancy; times",
+             "// within 0.5 % of the fastest count as ties, resolved to fewer resident face blocks, i.e. more",
+             "// registers per thread). A value given with -D at build time wins.",
              "#pragma once", ""]
     # shapes that no sweep covers keep their values and notes
     with open(os.path.join(CSRC, "tuned.h")) as f:
@@ -128,7 +134,7 @@ def write_header(path, best):
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--n", type=int, default=96)
-    ap.add_argument("--ramp-n", type=int, default=64, help="grid of the unstructured ramp (Euler staging switch)")
+    ap.add_argument("--ramp-n", type=int, default=64, help="grid of the unstructured ramp (Euler face kernels)")
     ap.add_argument("--steps", type=int, default=10)
     ap.add_argument("--precision", default="fp64", choices=["fp64", "fp32"])
     ap.add_argument("--out", default=None, help="also write the chosen header here")
@@ -137,7 +143,7 @@ def main():
     variants = [{"TG_FACE_BLOCK": fb, "TG_FACE_MINB": ft // fb, "TG_CELL_BLOCK": cb}
                 for fb, ft, cb in itertools.product(FACE_BLOCKS, FACE_THREADS, CELL_BLOCKS)]
 
-    def sweep(variants, workload, n, work, per):
+    def sweep(variants, workload, n, work, per, resident="TG_FACE_MINB"):
         with concurrent.futures.ThreadPoolExecutor(max_workers=4) as pool:
             built = list(pool.map(lambda v: (v,) + build(v, work, per), variants))
         results = []
@@ -151,11 +157,11 @@ def main():
             print(json.dumps({"variant": v, "workload": workload, "ms_per_step": ms}), flush=True)
         if not results:
             raise SystemExit("no variant ran")
-        # times within 0.5 % of the fastest are ties: take the one with the fewest resident face
-        # threads per SM (most registers per thread, fewest spills)
+        # times within 0.5 % of the fastest are ties: take the one with the fewest resident threads per
+        # SM (most registers per thread, fewest spills)
         fastest = min(r[0] for r in results)
         ties = [r for r in results if r[0] <= 1.005 * fastest]
-        return min(ties, key=lambda r: (r[1]["TG_FACE_BLOCK"] * r[1]["TG_FACE_MINB"], r[0]))
+        return min(ties, key=lambda r: (r[1]["TG_FACE_BLOCK"] * r[1][resident], r[0]))
 
     with tempfile.TemporaryDirectory() as work:
         per = max(2, args.jobs // 4)
@@ -164,15 +170,18 @@ def main():
         ms, best = sweep(cells, "tgv", args.n, work, per)
         grads = [dict(best, TG_GRAD_MINB=gm) for gm in GRAD_MINB]
         ms, best = sweep(grads, "tgv", args.n, work, per)
+        side_minb = "TG_SIDE_MINB" if args.precision == "fp64" else "TG_SIDE_MINB_FP32"
+        sides = [dict(best, **{side_minb: sm}) for sm in SIDE_MINB]
+        ms_e, best = sweep(sides, "ramp", args.ramp_n, work, per, side_minb)
         euler = [dict(best, TG_FACE_STAGED_EULER=st) for st in STAGED]
-        ms_e, best = sweep(euler, "ramp", args.ramp_n, work, per)
+        ms_1, best = sweep(euler, "ramp1", args.ramp_n, work, per)
         occ = [dict(best, TG_FACE_MINB_EULER=t // best["TG_FACE_BLOCK"]) for t in EULER_FACE_THREADS]
-        ms_e, best = sweep(occ, "ramp", args.ramp_n, work, per)
+        ms_1, best = sweep(occ, "ramp1", args.ramp_n, work, per, "TG_FACE_MINB_EULER")
     write_header(os.path.join(CSRC, "tuned.h"), best)
     if args.out:
         write_header(args.out, best)
     print(json.dumps({"best": best, "ms_per_step": ms, "workload": f"tgv {args.n}^3 {args.precision}",
-                      "ramp_ms_per_step": ms_e}))
+                      "ramp_ms_per_step": ms_e, "ramp_first_order_ms_per_step": ms_1}))
 
 
 if __name__ == "__main__":

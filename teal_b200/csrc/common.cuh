@@ -62,7 +62,6 @@ __host__ __device__ constexpr int cell_minb(int mode)
 }
 constexpr int GRAD_MINB = TG_GRAD_MINB;
 constexpr int GRAD_MINB_SIDES = TG_GRAD_MINB_SIDES;
-constexpr int REDUCE_BLOCK = 1024;
 
 // ---- small helpers ---------------------------------------------------------------------------
 
@@ -135,12 +134,6 @@ __device__ __forceinline__ V3<R> load_v3(const R *__restrict__ a, int ld, int i)
 }
 
 template <typename R>
-__device__ __forceinline__ R prim_get(const Prim<R> &p, int v)
-{
-    return v == 0 ? p.rho : v == 1 ? p.u.x : v == 2 ? p.u.y : v == 3 ? p.u.z : p.p;
-}
-
-template <typename R>
 __device__ __forceinline__ Prim<R> prim_from(const R *a)
 {
     return Prim<R>{a[0], v3(a[1], a[2], a[3]), a[4]};
@@ -170,18 +163,6 @@ __device__ __forceinline__ Basis<R> reload_basis(const R *__restrict__ b, int ld
     m.y = v3(reload(b + 3 * ld + f), reload(b + 4 * ld + f), reload(b + 5 * ld + f));
     m.z = v3(reload(b + 6 * ld + f), reload(b + 7 * ld + f), reload(b + 8 * ld + f));
     return m;
-}
-
-template <typename R>
-__device__ __forceinline__ Prim<R> reload_prim(const double *__restrict__ q, int ld, int i)
-{
-    Prim<R> p;
-    p.rho = R(reload(q + i));
-    p.u.x = R(reload(q + ld + i));
-    p.u.y = R(reload(q + 2 * ld + i));
-    p.u.z = R(reload(q + 3 * ld + i));
-    p.p = R(reload(q + 4 * ld + i));
-    return p;
 }
 
 // Per-cell gradient record: (gx, gy, gz, psi) for each of the 5 variables, 20 values per cell;
@@ -342,30 +323,6 @@ __device__ __forceinline__ double block_sum(double v, double *sh)
         }
     }
     return r;  // valid in thread 0
-}
-
-template <int NT>
-__device__ __forceinline__ double block_min(double v, double *sh)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        v = fmin(v, __shfl_down_sync(0xffffffffu, v, o));
-    }
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) {
-        sh[warp] = v;
-    }
-    __syncthreads();
-    double r = DBL_MAX;
-    if (warp == 0) {
-        r = (lane < NT / 32) ? sh[lane] : DBL_MAX;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            r = fmin(r, __shfl_down_sync(0xffffffffu, r, o));
-        }
-    }
-    return r;
 }
 
 // Sums over the block (threads of BLOCK) of t[0..4] and the minimum of t[5], valid in threads 0-5 (thread k:
