@@ -171,7 +171,7 @@ struct Gmres {
     int dim = 0;
     double *U = nullptr;      // [5][C] Newton iterate (conserved)
     double *r = nullptr;      // [5][C] Newton residual
-    double *V = nullptr;      // [dim + 1][5][C] Krylov basis
+    double *V = nullptr;      // [dim][5][C] Krylov basis
     double *w = nullptr;      // [5][C]
     double *q1 = nullptr;     // [5][N] perturbed primitive state
     double *R1 = nullptr;     // [5][C] derivative of the perturbed state

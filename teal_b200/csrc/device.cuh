@@ -102,7 +102,8 @@ struct Segments {
 };
 
 // Instances a residual is evaluated for (on: null for all): an arena's Newton iterations and Krylov columns
-// leave out the instances that are done with them. The flags do not change while the residual's kernels run.
+// leave out the instances that are done with them. The flags do not change while the residual's kernels run, but
+// the kernel before the residual's first one may have written them: they are read behind the launch wait.
 struct Mask {
     const int *on;         // [ninst]
     const int *cell_inst;  // [C]

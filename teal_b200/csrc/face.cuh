@@ -456,8 +456,12 @@ __global__ void __launch_bounds__(SIDE_BLOCK, side_minb<R>()) k_face_sides(Sizes
 // the fluxes of the cells' slots j (the left-to-right flux of the face, as k_face_sides: each inner face
 // is computed by both of its cells, with the same bits), five warps sum them in slot order and one
 // finishes the cells as k_cell does. It saves a launch and the round trip of the flux records, and pays
-// with twice the flux arithmetic: worth it while a launch costs more than that arithmetic
-// (TG_FUSED_CELLS, launch rule in context.cu).
+// with twice the flux arithmetic: worth it while a launch costs more than that arithmetic. Steps of periodic hllc
+// boxes, two launches / one, us: 8 k cells 40.6 / 33.0, 16 k 46.6 / 39.5, 18.9 k 48.5 / 39.7, 20.5 k 51.4 / 47.8, 24.6 k
+// 51.7 / 51.9, 49 k 67.7 / 72.3 (FP32 fluxes 39.0 / 28.9, 43.5 / 34.4, 43.5 / 34.8, 44.3 / 36.2, 47.6 / 43.3, 57.6 /
+// 59.7); implicit steps of 37 k cells 2.06 / 2.17 ms. The line lies at one wave of 148 SMs x 128 cells
+// (TG_FUSED_CELLS). The blocks update the state in place while others form their fluxes, so side_flux reads no
+// inner cell's state.
 template <typename R, int FK>
 __global__ void __launch_bounds__(SIDE_TILE, 4) k_cell_fluxes(FaceLaunch a, Geometry<R> g, CellLaunch b)
 {

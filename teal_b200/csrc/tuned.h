@@ -32,7 +32,7 @@
 #define TG_SIDE_MINB_FP32 8  // its blocks kept resident per SM, FP32-flux form
 #endif
 #ifndef TG_FUSED_CELLS
-#define TG_FUSED_CELLS 18944  // most cells of an arena whose face fluxes and cell updates run in one launch
+#define TG_FUSED_CELLS 18944  // most cells of an arena whose face fluxes and cell updates run in one launch (148 x 128)
 #endif
 #ifndef TG_CELL_BLOCK
 #define TG_CELL_BLOCK 128  // threads per cell-gather block
