@@ -15,6 +15,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <thread>
 #include <vector>
@@ -164,7 +165,121 @@ struct GeomBuf {
     long long *toff64 = nullptr, *toff32 = nullptr;       // their byte offsets, [tiles + 1]
 };
 
-constexpr int READ_CHUNKS = 64;  // most chunks of a staged read-back (d2h)
+// Threads that copy a read-back's rows out of the pinned staging buffer beside the calling thread (d2h): a
+// context's own, started by its first large read-back into pageable memory and joined with it. They sleep
+// between calls and make no CUDA calls. A call takes whatever helpers are awake: it waits only for those at
+// work, not for one that wakes late (threads started and joined by each call made one call in ten wait 300
+// us for a thread that had nothing left to do).
+class ReadHelpers {
+public:
+    static constexpr int CHUNKS = 64;  // most chunks of a call
+
+    ReadHelpers()
+    {
+        try {
+            for (std::thread &t : threads_) t = std::thread([this] { serve(); });
+        }
+        catch (const std::exception &) {  // fewer threads, or none
+        }
+    }
+    ~ReadHelpers()
+    {
+        {
+            std::lock_guard<std::mutex> held(lock_);
+            quit_ = true;
+        }
+        start_.notify_all();
+        for (std::thread &t : threads_) {
+            if (t.joinable()) t.join();
+        }
+    }
+    // a call's n doubles, in chunks of `per`, that will arrive in `from` and go to `to`
+    void begin(double *to, const double *from, size_t n, size_t per)
+    {
+        {
+            std::lock_guard<std::mutex> held(lock_);
+            to_ = to, from_ = from, n_ = n, per_ = per;
+            chunks_ = (int)((n + per - 1) / per);
+            next_ = 0, arrived_ = 0;
+            call_++;
+            open_ = true;
+        }
+        start_.notify_all();
+    }
+    // the first `count` chunks have arrived (-1: no more will)
+    void arrived(int count)
+    {
+        {
+            std::lock_guard<std::mutex> held(lock_);
+            arrived_ = count;
+        }
+        told_.notify_all();
+    }
+    // takes part in the copying, and returns when every chunk that was taken has been copied
+    void finish()
+    {
+        copy();
+        {
+            std::lock_guard<std::mutex> held(lock_);
+            open_ = false;
+        }
+        wait(told_, [&] { return busy_ == 0; });
+    }
+
+private:
+    // spinning for as long as a chunk takes to arrive, since a woken thread comes later than that; then asleep
+    template <typename Over>
+    void wait(std::condition_variable &cv, Over over)
+    {
+        constexpr auto SPIN = std::chrono::microseconds(300);
+        for (const auto start = std::chrono::steady_clock::now(); !over();) {
+            if (std::chrono::steady_clock::now() - start < SPIN) {
+                std::this_thread::yield();
+            }
+            else {
+                std::unique_lock<std::mutex> held(lock_);
+                cv.wait(held, over);
+            }
+        }
+    }
+    void copy()
+    {
+        for (int k; (k = next_++) < chunks_;) {
+            const size_t o = (size_t)k * per_, bytes = std::min(per_, n_ - o) * sizeof(double);
+            // a fresh array's pages are faulted in while the device still computes
+            volatile char *page = reinterpret_cast<volatile char *>(to_ + o);
+            for (size_t b = 0; b < bytes; b += 4096) page[b] = page[b];
+            wait(told_, [&] { const int n = arrived_; return n > k || n < 0; });
+            if (arrived_ < 0) return;
+            memcpy(to_ + o, from_ + o, bytes);
+        }
+    }
+    void serve()
+    {
+        std::unique_lock<std::mutex> held(lock_);
+        for (long served = 0;;) {
+            start_.wait(held, [&] { return quit_ || (open_ && call_ != served); });
+            if (quit_) return;
+            served = call_;
+            busy_++;
+            held.unlock();
+            copy();
+            held.lock();
+            if (--busy_ == 0) told_.notify_all();
+        }
+    }
+
+    std::thread threads_[3];
+    std::mutex lock_;
+    std::condition_variable start_, told_;
+    double *to_ = nullptr;
+    const double *from_ = nullptr;
+    size_t n_ = 0, per_ = 1;
+    int chunks_ = 0;
+    long call_ = 0;
+    bool open_ = false, quit_ = false;
+    std::atomic<int> next_{0}, arrived_{0}, busy_{0};
+};
 
 // workspace of the Jacobian-free Newton-GMRES implicit step
 struct Gmres {
@@ -263,7 +378,8 @@ struct tg_ctx {
     size_t aos_len = 0;
     double *pinned = nullptr;  // pinned host staging buffer
     size_t pinned_len = 0;
-    cudaEvent_t read_ev[READ_CHUNKS] = {};  // chunks of a staged read-back
+    cudaEvent_t read_ev[ReadHelpers::CHUNKS] = {};  // chunks of a staged read-back
+    std::unique_ptr<ReadHelpers> read_helpers;      // started by the first one
     bool prepared = false;     // U0, dtc and the piece minima valid for the resident state
 
     int rows_out = 0;  // the next residual is written in teal's rows [C][5]
@@ -1355,14 +1471,17 @@ static int d2h(tg_ctx *c, double *dst, const double *src, size_t n)
     }
     TRY(ensure_pinned(c, n));
     // Large pageable arrays: the host's copy out of the staging buffer (and the page faults of a fresh
-    // array) takes several times the transfer, so it runs on READ_THREADS threads, each chunk as soon
-    // as it has arrived.
-    constexpr int READ_THREADS = 4;
+    // array) takes several times the transfer, so it runs on several threads, each chunk as soon as it has
+    // arrived. A residual of 152 k cells, us (and the slowest call in ten): 745 (770) without helpers, 383 (403) with
+    // them; with threads of each call's own 450 (970), asleep until each chunk is there 740. At 29 k cells, two
+    // chunks, 185 and 133 (155), with threads of its own 160 (460).
     constexpr size_t PAGE = 4096 / sizeof(double);
-    // 1 MiB a chunk, larger ones above READ_CHUNKS of them
-    const size_t per = std::max((size_t)256, (n + PAGE * READ_CHUNKS - 1) / (PAGE * READ_CHUNKS)) * PAGE;
+    constexpr int MOST = ReadHelpers::CHUNKS;
+    // 1 MiB a chunk, larger ones above MOST of them
+    const size_t per = std::max((size_t)256, (n + PAGE * MOST - 1) / (PAGE * MOST)) * PAGE;
     const int chunks = (int)((n + per - 1) / per);
-    if (chunks < 2) {
+    if (chunks >= 2 && !c->read_helpers) c->read_helpers.reset(new (std::nothrow) ReadHelpers);
+    if (chunks < 2 || !c->read_helpers) {
         CU(cudaMemcpyAsync(c->pinned, src, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
         CU(cudaStreamSynchronize(c->stream));
         memcpy(dst, c->pinned, n * sizeof(double));
@@ -1371,64 +1490,20 @@ static int d2h(tg_ctx *c, double *dst, const double *src, size_t n)
     for (int k = 0; k < chunks; k++) {
         if (!c->read_ev[k]) CU(cudaEventCreateWithFlags(&c->read_ev[k], cudaEventDisableTiming));
     }
-    auto span = [&](int k) { return std::min(per, n - (size_t)k * per); };
     for (int k = 0; k < chunks; k++) {
         const size_t o = (size_t)k * per;
-        CU(cudaMemcpyAsync(c->pinned + o, src + o, span(k) * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+        CU(cudaMemcpyAsync(c->pinned + o, src + o, std::min(per, n - o) * sizeof(double), cudaMemcpyDeviceToHost,
+                           c->stream));
         CU(cudaEventRecord(c->read_ev[k], c->stream));
     }
-    // The helpers make no CUDA calls: this thread tells them how many chunks have arrived (-1: none will).
-    // A chunk that is on its way they await spinning, since a woken thread comes later than the chunk (a residual
-    // of 152 k cells: 730-755 us sleeping, 440-690 spinning, 700-770 without helpers); while the device
-    // still computes they sleep. They are left out where threads cannot be started.
-    constexpr auto SPIN = std::chrono::microseconds(300);
-    std::atomic<int> next(0), arrived(0);
-    std::mutex lock;
-    std::condition_variable told;
-    auto await = [&](int k) {
-        const auto over = [&] { const int n = arrived; return n > k || n < 0; };
-        for (const auto start = std::chrono::steady_clock::now(); !over();) {
-            if (std::chrono::steady_clock::now() - start < SPIN) {
-                std::this_thread::yield();
-            }
-            else {
-                std::unique_lock<std::mutex> held(lock);
-                told.wait(held, over);
-            }
-        }
-        return arrived > k;
-    };
-    auto copy = [&]() {
-        for (int k; (k = next++) < chunks;) {
-            const size_t o = (size_t)k * per;
-            // a fresh array's pages are faulted in while the device still computes
-            volatile char *page = reinterpret_cast<volatile char *>(dst + o);
-            for (size_t b = 0; b < span(k) * sizeof(double); b += 4096) page[b] = page[b];
-            if (!await(k)) return;
-            memcpy(dst + o, c->pinned + o, span(k) * sizeof(double));
-        }
-    };
-    std::thread threads[READ_THREADS - 1];
-    try {
-        for (int t = 0; t < std::min(READ_THREADS, chunks) - 1; t++) threads[t] = std::thread(copy);
+    c->read_helpers->begin(dst, c->pinned, n, per);
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < chunks && e == cudaSuccess; k++) {
+        e = cudaEventSynchronize(c->read_ev[k]);
+        c->read_helpers->arrived(e == cudaSuccess ? k + 1 : -1);
     }
-    catch (const std::exception &) {
-    }
-    bool ok = true;
-    for (int k = 0; k < chunks && ok; k++) {
-        ok = cudaEventSynchronize(c->read_ev[k]) == cudaSuccess;
-        {
-            std::lock_guard<std::mutex> held(lock);
-            arrived = ok ? k + 1 : -1;
-        }
-        told.notify_all();
-    }
-    copy();
-    for (std::thread &t : threads) {
-        if (t.joinable()) t.join();
-    }
-    CU(cudaStreamSynchronize(c->stream));
-    if (!ok) return fail(TG_ERR_CUDA, "reading the device's rows back failed");
+    c->read_helpers->finish();
+    CU(e);
     return TG_OK;
 }
 

@@ -3,6 +3,7 @@ that the replayed step with the copy behind it), against the three calls, and af
 an end time behind; steps whose time order changes at the same number of stages; read-backs into
 pageable memory."""
 
+import threading
 import time
 
 import numpy as np
@@ -105,3 +106,31 @@ def test_pageable_read_back(cells):
     assert wall > 0.1
     assert cpu < 1.8 * wall  # this thread and the copies; three spinning threads more would be near four
     ctx.close()
+
+
+def test_pageable_read_backs_of_several_threads():
+    """Each context's helpers serve its own calls: contexts read back by two threads at once, many times, into
+    arrays that change, one of them destroyed and made anew in between."""
+    wrong = []
+
+    def work(seed, cells):
+        m = tb.Mesh.create((0, 0, 0), (10, 10, 10), cells, (1, 1, 1))
+        e = tb.Equations.euler(m)
+        rng = np.random.default_rng(seed)
+        for _ in range(3):
+            ctx = tb.Context(m, e)
+            for _ in range(20):
+                e.primitive[: m.num_inner_cells] = 1 + rng.random((m.num_inner_cells, 5))
+                ctx.set_primitive(e.primitive)
+                got = np.zeros((m.num_cells, 5))
+                ctx.get_primitive(got)
+                if not np.array_equal(got[: m.num_inner_cells], e.primitive[: m.num_inner_cells]):
+                    wrong.append(seed)
+            ctx.close()
+
+    threads = [threading.Thread(target=work, args=a) for a in ((1, (31, 29, 31)), (2, (50, 40, 41)))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
