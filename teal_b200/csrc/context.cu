@@ -420,6 +420,10 @@ struct tg_ctx {
     const double *graph_alpha = nullptr;  // the coefficient table (one for each time order and stage count)
     double graph_courant = 0;
     int graph_use_max_time = -1;
+    // the last step from host state to host state below two chunks (host_step)
+    int host_method = -1;
+    const double *host_alpha = nullptr;
+    double host_courant = 0;
 
     // polls of the staged face kernel's first bounded wait (lowered only by tg_set_wait_limit)
     int wait_polls = MBAR_POLLS;
@@ -2416,6 +2420,23 @@ static int copy_rows(tg_ctx *c, double *out)
     return TG_OK;
 }
 
+// A step below two chunks: replayed from its graph from the second one of its kind on. Capturing a graph costs
+// more than the launches of one step (20^3 cells: 527 us for a context's first step, 475 launched plainly), and
+// steps whose Courant number changes each time would do it each time.
+static int host_step(tg_ctx *c, int method, int stages, const double *alpha, double courant)
+{
+    const bool again = c->host_method == method && c->host_alpha == alpha && c->host_courant == courant;
+    if (again) {
+        TRY(step_graph(c, method, stages, alpha, courant, 0));
+        return launch_step(c, stages, alpha, courant);
+    }
+    c->host_method = method;
+    c->host_alpha = alpha;
+    c->host_courant = courant;
+    c->st.use_max_time = 0;  // clipped by max_step, whatever a run loop left
+    return enqueue_explicit_step(c, stages, alpha, courant);
+}
+
 extern "C" int tg_advance_host(tg_ctx *c, int method, const void *context, double courant, double *time,
                                double max_step, const double *prim_in, double *prim_out, double *residual,
                                double *step0)
@@ -2453,8 +2474,7 @@ extern "C" int tg_advance_host(tg_ctx *c, int method, const void *context, doubl
         rc = advance_chunked(c, stages, alpha, courant, prim_out);
     }
     else {
-        rc = step_graph(c, method, stages, alpha, courant, 0);
-        if (rc == TG_OK) rc = launch_step(c, stages, alpha, courant);
+        rc = host_step(c, method, stages, alpha, courant);
         if (rc == TG_OK) rc = copy_rows(c, prim_out);
     }
     c->cell_lo = 0, c->cell_hi = -1, c->face_lo = 0, c->face_hi = -1;

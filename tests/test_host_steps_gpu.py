@@ -53,6 +53,25 @@ def test_host_step_after_a_run_with_an_end_time(cells):
     assert (t, again) == (step, step)
 
 
+def test_host_steps_of_changing_courant_numbers():
+    """A kind of step is launched plainly the first time and replayed after that: the same bits either way,
+    and as the three calls."""
+    m = tb.Mesh.create((0, 0, 0), (10, 10, 10), (20, 18, 4), (1, 1, 1))
+    e = tb.Equations.euler(m)
+    e.set_initial_condition("domain", vortex)
+    ctx, three = tb.Context(m, e), tb.Context(m, e)
+    out, state = pinned(m.num_cells), e.primitive.copy()
+    t = 0.0
+    for courant in (0.4, 0.4, 0.4, 0.6, 0.4, 0.4, 0.8, 0.8, 0.6):
+        three.set_primitive(state)
+        want = three.advance(tb.TG_ADVANCE_LSERK, courant, t)
+        got = ctx.advance_host(tb.TG_ADVANCE_LSERK, courant, t, state, out)
+        assert got[:2] == want[:2]
+        assert np.array_equal(got[2], want[2])
+        assert np.array_equal(out, three.get_primitive())
+        state, t = out.copy(), got[0]
+
+
 @pytest.mark.parametrize("how", ["advance", "advance_host", "run"])
 def test_time_order_changes_at_a_fixed_stage_count(how):
     m = tb.Mesh.create((0, 0, 0), (10, 10, 10), (20, 18, 4), (1, 1, 1))
