@@ -165,14 +165,22 @@ struct GeomBuf {
     long long *toff64 = nullptr, *toff32 = nullptr;       // their byte offsets, [tiles + 1]
 };
 
+// Least doubles of a read-back that takes helpers, 16 MiB. What they copy lies in other cores' caches when the
+// caller goes on with it, and what the caller has just written lies in its own when they start: below that
+// the calls lose more than the copies gain. Steps from and to a pageable array, then scaled by the host, in us without
+// and with helpers: 1.3 MiB 320 / 600, 6 MiB 1280 / 1900, 10.9 MiB 2250 / 2600, 16.7 MiB 3420 / 3420, 18.1 MiB 3860 / 3620, 40
+// MiB 11000 / 7800.
+constexpr size_t READ_HELPED = (size_t)1 << 21;
+
 // Threads that copy a read-back's rows out of the pinned staging buffer beside the calling thread (d2h): a
 // context's own, started by its first large read-back into pageable memory and joined with it. They sleep
-// between calls and make no CUDA calls. A call takes whatever helpers are awake: it waits only for those at
-// work, not for one that wakes late (threads started and joined by each call made one call in ten wait 300
-// us for a thread that had nothing left to do).
+// between calls and make no CUDA calls. A call takes whatever helpers are awake, in small pieces: it waits only
+// for those at work, not for one that wakes late (threads started and joined by each call made one call in ten
+// wait 300 us for a thread that had nothing left to do).
 class ReadHelpers {
 public:
     static constexpr int CHUNKS = 64;  // most chunks of a call
+    static constexpr size_t PIECE = 16384;  // doubles a thread takes at once; a chunk holds whole pieces
 
     ReadHelpers()
     {
@@ -193,13 +201,18 @@ public:
             if (t.joinable()) t.join();
         }
     }
+    // a fresh array's pages are faulted in while the device still computes
+    static void touch(double *to, size_t bytes)
+    {
+        volatile char *page = reinterpret_cast<volatile char *>(to);
+        for (size_t b = 0; b < bytes; b += 4096) page[b] = page[b];
+    }
     // a call's n doubles, in chunks of `per`, that will arrive in `from` and go to `to`
     void begin(double *to, const double *from, size_t n, size_t per)
     {
         {
             std::lock_guard<std::mutex> held(lock_);
             to_ = to, from_ = from, n_ = n, per_ = per;
-            chunks_ = (int)((n + per - 1) / per);
             next_ = 0, arrived_ = 0;
             call_++;
             open_ = true;
@@ -244,11 +257,10 @@ private:
     }
     void copy()
     {
-        for (int k; (k = next_++) < chunks_;) {
-            const size_t o = (size_t)k * per_, bytes = std::min(per_, n_ - o) * sizeof(double);
-            // a fresh array's pages are faulted in while the device still computes
-            volatile char *page = reinterpret_cast<volatile char *>(to_ + o);
-            for (size_t b = 0; b < bytes; b += 4096) page[b] = page[b];
+        for (size_t o; (o = next_.fetch_add(PIECE)) < n_;) {
+            const int k = (int)(o / per_);
+            const size_t bytes = std::min(PIECE, n_ - o) * sizeof(double);
+            touch(to_ + o, bytes);
             wait(told_, [&] { const int n = arrived_; return n > k || n < 0; });
             if (arrived_ < 0) return;
             memcpy(to_ + o, from_ + o, bytes);
@@ -275,10 +287,10 @@ private:
     double *to_ = nullptr;
     const double *from_ = nullptr;
     size_t n_ = 0, per_ = 1;
-    int chunks_ = 0;
     long call_ = 0;
     bool open_ = false, quit_ = false;
-    std::atomic<int> next_{0}, arrived_{0}, busy_{0};
+    std::atomic<size_t> next_{0};
+    std::atomic<int> arrived_{0}, busy_{0};
 };
 
 // workspace of the Jacobian-free Newton-GMRES implicit step
@@ -379,7 +391,7 @@ struct tg_ctx {
     double *pinned = nullptr;  // pinned host staging buffer
     size_t pinned_len = 0;
     cudaEvent_t read_ev[ReadHelpers::CHUNKS] = {};  // chunks of a staged read-back
-    std::unique_ptr<ReadHelpers> read_helpers;      // started by the first one
+    std::unique_ptr<ReadHelpers> read_helpers;      // started by the first large one
     bool prepared = false;     // U0, dtc and the piece minima valid for the resident state
 
     int rows_out = 0;  // the next residual is written in teal's rows [C][5]
@@ -1474,18 +1486,12 @@ static int d2h(tg_ctx *c, double *dst, const double *src, size_t n)
         return TG_OK;
     }
     TRY(ensure_pinned(c, n));
-    // Large pageable arrays: the host's copy out of the staging buffer (and the page faults of a fresh
-    // array) takes several times the transfer, so it runs on several threads, each chunk as soon as it has
-    // arrived. A residual of 152 k cells, us (and the slowest call in ten): 745 (770) without helpers, 383 (403) with
-    // them; with threads of each call's own 450 (970), asleep until each chunk is there 740. At 29 k cells, two
-    // chunks, 185 and 133 (155), with threads of its own 160 (460).
-    constexpr size_t PAGE = 4096 / sizeof(double);
-    constexpr int MOST = ReadHelpers::CHUNKS;
-    // 1 MiB a chunk, larger ones above MOST of them
-    const size_t per = std::max((size_t)256, (n + PAGE * MOST - 1) / (PAGE * MOST)) * PAGE;
+    // Pageable arrays: the host's copy out of the staging buffer (and the page faults of a fresh array) takes several
+    // times the transfer. Above 1 MiB it goes chunk by chunk, each as soon as it has arrived.
+    constexpr size_t MIB = (size_t)1 << 17;  // doubles
+    const size_t per = std::max((size_t)1, (n + MIB * ReadHelpers::CHUNKS - 1) / (MIB * ReadHelpers::CHUNKS)) * MIB;
     const int chunks = (int)((n + per - 1) / per);
-    if (chunks >= 2 && !c->read_helpers) c->read_helpers.reset(new (std::nothrow) ReadHelpers);
-    if (chunks < 2 || !c->read_helpers) {
+    if (chunks < 2) {
         CU(cudaMemcpyAsync(c->pinned, src, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
         CU(cudaStreamSynchronize(c->stream));
         memcpy(dst, c->pinned, n * sizeof(double));
@@ -1499,6 +1505,16 @@ static int d2h(tg_ctx *c, double *dst, const double *src, size_t n)
         CU(cudaMemcpyAsync(c->pinned + o, src + o, std::min(per, n - o) * sizeof(double), cudaMemcpyDeviceToHost,
                            c->stream));
         CU(cudaEventRecord(c->read_ev[k], c->stream));
+    }
+    if (n >= READ_HELPED && !c->read_helpers) c->read_helpers.reset(new (std::nothrow) ReadHelpers);
+    if (n < READ_HELPED || !c->read_helpers) {
+        for (int k = 0; k < chunks; k++) {
+            const size_t o = (size_t)k * per, bytes = std::min(per, n - o) * sizeof(double);
+            ReadHelpers::touch(dst + o, bytes);
+            CU(cudaEventSynchronize(c->read_ev[k]));
+            memcpy(dst + o, c->pinned + o, bytes);
+        }
+        return TG_OK;
     }
     c->read_helpers->begin(dst, c->pinned, n, per);
     cudaError_t e = cudaSuccess;

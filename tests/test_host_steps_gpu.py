@@ -98,8 +98,8 @@ def test_time_order_changes_at_a_fixed_stage_count(how):
     assert not np.array_equal(want[0], want[1])
 
 
-# one chunk and a little, several, and more than 64 chunks of 1 MiB (which then grow)
-@pytest.mark.parametrize("cells", [(31, 29, 30), (64, 64, 65), (120, 121, 122)])
+# one chunk of 1 MiB and a little, several, with helpers (16 MiB), and more than 64 chunks (which then grow)
+@pytest.mark.parametrize("cells", [(31, 29, 30), (64, 64, 65), (76, 75, 78), (120, 121, 122)])
 def test_pageable_read_back(cells):
     m = tb.Mesh.create((0, 0, 0), (10, 10, 10), cells, (1, 1, 1))
     e = tb.Equations.euler(m)
@@ -128,7 +128,7 @@ def test_pageable_read_back(cells):
 
 
 def test_pageable_read_backs_of_several_threads():
-    """Each context's helpers serve its own calls: contexts read back by two threads at once, many times, into
+    """Each context's helpers serve its own calls: contexts read back by several threads at once, many times, into
     arrays that change, one of them destroyed and made anew in between."""
     wrong = []
 
@@ -147,7 +147,7 @@ def test_pageable_read_backs_of_several_threads():
                     wrong.append(seed)
             ctx.close()
 
-    threads = [threading.Thread(target=work, args=a) for a in ((1, (31, 29, 31)), (2, (50, 40, 41)))]
+    threads = [threading.Thread(target=work, args=a) for a in ((1, (31, 29, 31)), (2, (76, 75, 78)), (3, (77, 74, 79)))]
     for t in threads:
         t.start()
     for t in threads:
